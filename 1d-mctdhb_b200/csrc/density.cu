@@ -20,6 +20,7 @@
 #include "gram.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "wide.h"
 
 namespace mctdhb {
 
@@ -185,6 +186,8 @@ size_t gram_partial_elems(const SpaceView& sp) {
 
 size_t dens_partial_elems(const SpaceView& sp) {
     const size_t per_row = (size_t)dens_slices(sp) * dens_ep(sp.M);
+    if (wide_eligible(sp.N, sp.M))
+        return std::max(per_row, wide_gram_elems(sp.M, annihilated_dim(sp, 2)));
     return dens_templated(sp.M) ? std::max(per_row, gram_partial_elems(sp)) : per_row;
 }
 
@@ -255,7 +258,7 @@ int dens_prepare(const SpaceView& sp, const double2* C, double2* partial, cudaSt
         case 7: return gram_prepare_tmpl<7>();
         case 8: return gram_prepare_tmpl<8>();
     }
-    return 0;
+    return wide_eligible(sp.N, sp.M) ? wide_prepare() : 0;
 }
 
 // Set-up of the per-row kernels (dens_tmpl.cuh): launch attributes and the
@@ -272,12 +275,14 @@ int dens_prepare_rows(const SpaceView& sp, const double2* C, double2* partial, c
 int dens_apply(const SpaceView& sp, const double2* C, double2* partial, double2* rho1,
                double2* rho2, const int* d_desc, cudaStream_t st) {
     if (dens_templated(sp.M)) return gram_apply(sp, C, partial, rho1, rho2, st);
+    if (wide_eligible(sp.N, sp.M))
+        return wide_dens(sp, annihilated_dim(sp, 2), C, partial, rho1, rho2, st);
     return dens_apply_rows(sp, C, partial, rho1, rho2, d_desc, st);
 }
 
 // The per-row pass: every row's contributions to every unique element,
-// reduced across the warp (dens_tmpl.cuh for M <= 8, the generic kernel
-// beyond).
+// reduced across the warp (dens_tmpl.cuh for M <= 8, the generic kernel for
+// one boson or one orbital beyond).
 int dens_apply_rows(const SpaceView& sp, const double2* C, double2* partial, double2* rho1,
                     double2* rho2, const int* d_desc, cudaStream_t st) {
     const int grid = dens_grid(sp);

@@ -27,6 +27,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "wide.h"
 
 namespace mctdhb {
 
@@ -158,7 +159,7 @@ __global__ void hcp_w_kernel(int N, int M, const double2* __restrict__ hob,
 bool hcp_eligible(int N, int M) { return N >= 2 && M >= 2 && M <= kMaxTemplOrb; }
 
 size_t hcp_scratch_bytes(int N, int M) {
-    if (!hcp_eligible(N, M)) return 0;
+    if (!hcp_eligible(N, M) && !wide_eligible(N, M)) return 0;
     return (size_t)fock_dimension(N - 2, M) * (size_t)(M * (M + 1) / 2) * sizeof(double2);
 }
 
@@ -178,11 +179,11 @@ int hcp_prepare(int M) {
 int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, double2* d_tab,
             cudaStream_t st) {
     hc_prep_kernel<<<1, 32, 0, st>>>(sp.M, d_hob, d_hint, d_tab);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
     if (sp.pair_y != nullptr) {
+        if (sp.M > kMaxTemplOrb) return wide_prep(sp, d_hob, d_hint, st);
         hcp_w_kernel<<<1, 256, 0, st>>>(sp.N, sp.M, d_hob, d_hint, sp.pair_w);
-        MCTDHB_CUDA_TRY(cudaGetLastError());
     }
+    MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
@@ -271,7 +272,8 @@ int hc_tune_launch(void* p, int v, cudaStream_t st) {
 
 int hc_variant(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,
                const HcEpilogue& ep, cudaStream_t st) {
-    if (sp.pair_y != nullptr) return pair_variant(sp, C, HC, ep, st);
+    if (sp.pair_y != nullptr)
+        return sp.M > kMaxTemplOrb ? 0 : pair_variant(sp, C, HC, ep, st);
     if (!hc_templated(sp.M) || sp.dim < 4096) return 0;
     HcTuneCtx ctx{&sp, C, HC, tab, &ep};
     return tune_pick("hc", sp.N, sp.M, kHcVariants, st, hc_tune_launch, &ctx);
@@ -279,7 +281,8 @@ int hc_variant(const SpaceView& sp, const double2* C, double2* HC, const double2
 
 int hc_apply(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,
              const HcEpilogue& ep, cudaStream_t st) {
-    if (sp.pair_y != nullptr) return hcp_apply(sp, C, HC, ep, st);
+    if (sp.pair_y != nullptr)
+        return sp.M > kMaxTemplOrb ? wide_hc(sp, C, HC, ep, st) : hcp_apply(sp, C, HC, ep, st);
     const int v = hc_variant(sp, C, HC, tab, ep, st);
     return hc_launch_v(sp, C, HC, tab, ep, v, st);
 }

@@ -15,6 +15,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "wide.h"
 
 namespace mctdhb {
 
@@ -78,7 +79,16 @@ int space_init(SpaceCtx& s, int N, int M) {
     if (dens_prepare(s.view, nullptr, nullptr, nullptr)) return -1;
     // pair-space H.C: the pair matrix and its D(N-2, M) x P scratch; when the
     // scratch cannot be had the space keeps the per-row kernel
-    if (hcp_eligible(N, M)) {
+    // More than 8 orbitals: taken only where the room left still holds every
+    // Lanczos workspace a caller may ask for (64 vectors and the callers' own),
+    // so no call that ran beside the per-row kernel runs out of memory now.
+    bool pair = hcp_eligible(N, M);
+    if (wide_eligible(N, M)) {
+        size_t free_b = 0, total_b = 0;
+        MCTDHB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+        pair = hcp_scratch_bytes(N, M) + (size_t)72 * dim * sizeof(double2) <= free_b;
+    }
+    if (pair) {
         const size_t P = (size_t)M * (M + 1) / 2;
         double2 *w = nullptr, *y = nullptr;
         if (cudaMalloc(&w, (P * P + 1) * sizeof(double2)) == cudaSuccess &&
