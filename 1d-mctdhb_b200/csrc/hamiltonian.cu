@@ -178,11 +178,15 @@ int hcp_prepare(int M) {
 
 int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, double2* d_tab,
             cudaStream_t st) {
-    hc_prep_kernel<<<1, 32, 0, st>>>(sp.M, d_hob, d_hint, d_tab);
-    if (sp.pair_y != nullptr) {
-        if (sp.M > kMaxTemplOrb) return wide_prep(sp, d_hob, d_hint, st);
+    // the packed table is read by the per-row kernels alone: a space with pair
+    // scratch forms the pair matrix only (the table took one thread 52 us at
+    // four orbitals, 105 us at six)
+    if (sp.pair_y == nullptr)
+        hc_prep_kernel<<<1, 32, 0, st>>>(sp.M, d_hob, d_hint, d_tab);
+    else if (sp.M > kMaxTemplOrb)
+        return wide_prep(sp, d_hob, d_hint, st);
+    else
         hcp_w_kernel<<<1, 256, 0, st>>>(sp.N, sp.M, d_hob, d_hint, sp.pair_w);
-    }
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
