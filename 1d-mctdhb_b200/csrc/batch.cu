@@ -38,6 +38,7 @@
 #include "kernels.h"
 #include "moves.cuh"
 #include "orbital.h"
+#include "orbstep.cuh"
 
 using namespace mctdhb;
 
@@ -383,9 +384,7 @@ int enqueue_step(mctdhb_batch_s* b, unsigned mask) {
     const int vgrid = num_sms() * 8, sgrid = b->max_slots;
     const int lz = b->lz;
     int* mon = batch_mon(b->d_cnt);
-    bt_orbital_kernel<<<sgrid, kBatchOrbThreads, kBatchMaxGrid * sizeof(double), st>>>(S, sl, nL, 0,
-                                                                                       mon);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
+    if (orb_step_launch(S, sl, nL, sgrid, kOrbStep, mon, st)) return -1;
     auto hc = [&](int iter) {
         return per_group(b, mask, [&](int M, cudaStream_t s) {
             return hc_group(M, S, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt, iter, s, 3,
@@ -818,9 +817,8 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
         set_error("mctdhb_batch_admit: upload failed");
         return undo();
     }
-    bt_orbital_kernel<<<1, kBatchOrbThreads, kBatchMaxGrid * sizeof(double), st>>>(
-        b->d_slots, pl + 1, pl, 1, nullptr);
-    if (prepare_group(M) ||
+    if (prepare_group(M) || orb_step_prepare() ||
+        orb_step_launch(b->d_slots, pl + 1, pl, 1, kOrbMatrices, nullptr, st) ||
         dens_group(M, b->d_slots, b->d_pro_g, dpc, pl + 1, pl, 1, st))
         return undo();
     bt_tail_kernel<<<1, kBatchVecThreads, 0, st>>>(b->d_slots, pl + 1, pl, 1, nullptr);

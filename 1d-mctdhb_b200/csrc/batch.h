@@ -26,7 +26,6 @@ constexpr int kBatchMaxLz = 16;        // Lanczos vectors per step
 constexpr int kBatchMinOrb = 2, kBatchMaxOrb = 8;
 constexpr int kBatchMaxGrid = 4096;
 constexpr int kBatchMonIter = -1;  // H.C launch of the monitor (eigen residual)
-constexpr int kBatchOrbThreads = 512;
 
 // per-slot device scalars (double2 units)
 constexpr int BS_DIAG = 0;
@@ -77,6 +76,7 @@ struct BatchSlot {
     SpaceView sp; // with the pair matrix sp.pair_w and its scratch sp.pair_y
     const double* g;     // contact interaction (device scalar)
     double2 *orb, *stage, *H, *Q, *hob, *hint, *rho1, *rho2, *rinv, *work;
+    double2* orb_next;   // a copy of the orbitals after the Runge-Kutta step (null: none)
     double2 *V;          // lz x nc Krylov vectors; V[0] holds the coefficients
     // split step (split: 1): the half-step operator (orbital.h,
     // split_half_operator; dense: column-major G x G, else the circulant

@@ -1,10 +1,11 @@
 // batch_kernels.cu -- the slot-level and vector kernels of the batched engine
 // (batch.h).  Per slot, one step is the full step of the single-system
 // solver (driver.c:159-201):
-//   bt_orbital_kernel   one block per slot: Runge-Kutta step of the orbital
-//                       equation with the slot's rho1^{-1} and rho2,
-//                       Gram-Schmidt in imaginary time, h_kl and g_ksql of the
-//                       new orbitals, the pair matrix of H.C, Lanczos set-up
+//   orb_step_launch     (orbstep.cu) one cluster of blocks per slot:
+//                       Runge-Kutta step of the orbital equation with the
+//                       slot's rho1^{-1} and rho2, Gram-Schmidt in imaginary
+//                       time, h_kl and g_ksql of the new orbitals, the pair
+//                       matrix of H.C, Lanczos set-up
 //   Lanczos             the pair-space H.C (per M, batch_tmpl.cuh) and the
 //                       vector kernels below, multiconfig_lanczos.c:12-90
 //                       operation for operation
@@ -34,397 +35,7 @@ __device__ __forceinline__ bool slot_running(const BatchSlot& S) {
     return S.flags[BF_STATE] == SLOT_RUNNING;
 }
 
-// ---------------------------------------------------------------------------
-// orbital side, one block per slot
-// ---------------------------------------------------------------------------
-
-// <y_s|y_l> (Simpson) for every s, l into out[s * M + l], one warp per entry
-__device__ void bt_overlaps(const BatchSlot& S, const double2* __restrict__ y, double2* out) {
-    const OrbView& o = S.ov;
-    const int M = o.M, G = o.G;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int p = warp; p < M * M; p += nw) {
-        const int a = p / M, b = p % M;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int x = lane; x < G; x += 32) {
-            const double2 t = cfma_conj(y[(size_t)a * G + x], y[(size_t)b * G + x],
-                                        make_double2(0.0, 0.0));
-            acc.x += o.w[x] * t.x;
-            acc.y += o.w[x] * t.y;
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) out[p] = acc;
-    }
-    __syncthreads();
-}
-
-// robust projector (orbital_integration.c:22-92): P <- S^{-1} P with the
-// full overlap matrix S_sl = <y_s|y_l> of the stage orbitals, as the
-// single-system solver does; a singular S keeps the simple projector's P
-// and flags the slot (BF_ROBFAIL)
-__device__ void bt_robust(const BatchSlot& S, const double2* __restrict__ y, double2* sP) {
-    __shared__ double2 sS[kBatchMaxOrb * kBatchMaxOrb], sI[kBatchMaxOrb * kBatchMaxOrb];
-    const int M = S.ov.M;
-    bt_overlaps(S, y, sS);
-    if (threadIdx.x == 0) {
-        if (herm_inverse(M, sS, sI)) {
-            S.flags[BF_ROBFAIL] = 1;
-        } else {
-            double2 t[kBatchMaxOrb * kBatchMaxOrb];
-            for (int a = 0; a < M; a++)
-                for (int k = 0; k < M; k++) {
-                    double2 z = make_double2(0.0, 0.0);
-                    for (int l = 0; l < M; l++) z = cfma(sI[a * M + l], sP[l * M + k], z);
-                    t[a * M + k] = z;
-                }
-            for (int i = 0; i < M * M; i++) sP[i] = t[i];
-        }
-    }
-    __syncthreads();
-}
-
-// overlap residual sum_{k<l} |<f_k|f_l>| / M of the slot's orbitals
-// (integrator_monitor.c:31-42) into scal[BS_MISC + 5], summed in the
-// reference's (k, l) order
-__device__ void bt_overlap_residual(const BatchSlot& S) {
-    __shared__ double2 sS[kBatchMaxOrb * kBatchMaxOrb];
-    const int M = S.ov.M;
-    bt_overlaps(S, S.orb, sS);
-    if (threadIdx.x == 0) {
-        double sum = 0.0;
-        for (int k = 0; k < M; k++)
-            for (int l = k + 1; l < M; l++) sum += hypot(sS[k * M + l].x, sS[k * M + l].y);
-        S.scal[BS_MISC + 5] = make_double2(sum / M, 0.0);
-    }
-    __syncthreads();
-}
-
-// dy/dt of the orbital equation (orbital_integration.c:179-240) for all
-// orbitals y (M x G): H = linear part + interacting part, overlaps
-// P[s][k] = <y_s|H_k> (simple projector, :95-131), out = -i tf (H - sum_s y_s P[s][k]).
-__device__ void bt_rhs(const BatchSlot& S, const double2* __restrict__ y, double2* __restrict__ out,
-                       double2* sP) {
-    const OrbView& o = S.ov;
-    const int M = o.M, G = o.G, n = M * G;
-    double2* H = S.H;
-    const double2* Q = S.Q;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = t / G, x = t % G;
-        const double2 lin = o.lin_t ? toeplitz_at(o, y + (size_t)k * G, x)
-                                    : linear_at(o, y + (size_t)k * G, x);
-        double2 fx[kBatchMaxOrb];
-        for (int a = 0; a < M; a++) fx[a] = y[(size_t)a * G + x];
-        const double2* Qk = Q + (size_t)k * M * M * M;
-        double2 red = make_double2(0.0, 0.0);
-        for (int s = 0; s < M; s++) {
-            double2 ts = make_double2(0.0, 0.0);
-            for (int l = 0; l < M; l++) {
-                double2 tl = make_double2(0.0, 0.0);
-                for (int q = 0; q < M; q++) tl = cfma(Qk[s + q * M + l * M * M], fx[q], tl);
-                ts = cfma(tl, fx[l], ts);
-            }
-            red = cfma(make_double2(fx[s].x, -fx[s].y), ts, red);
-        }
-        H[t] = cadd(red, lin);
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int p = warp; p < M * M; p += nw) {
-        const int s = p / M, k = p % M;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int x = lane; x < G; x += 32) {
-            const double2 t = cfma_conj(y[(size_t)s * G + x], H[(size_t)k * G + x],
-                                        make_double2(0.0, 0.0));
-            acc.x += o.w[x] * t.x;
-            acc.y += o.w[x] * t.y;
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) sP[p] = acc;
-    }
-    __syncthreads();
-    if (S.flags[BF_ROBUST]) bt_robust(S, y, sP);
-    const double2 mi_tf = make_double2(o.tf.y, -o.tf.x);
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = t / G, x = t % G;
-        double2 proj = make_double2(0.0, 0.0);
-        for (int s = 0; s < M; s++) proj = cfma(y[(size_t)s * G + x], sP[s * M + k], proj);
-        const double2 d = make_double2(H[t].x - proj.x, H[t].y - proj.y);
-        out[t] = cmul(mi_tf, d);
-    }
-    __syncthreads();
-}
-
-// the split step's nonlinear right-hand side (orbital_integration.c:
-// 243-281), as orb_split_rhs_kernel: -i tf (interacting - sum_j (h[j][k] +
-// B[k][j]) f_j + V f_k), h of the half-stepped orbitals
-__device__ void bt_split_rhs(const BatchSlot& S, const double2* __restrict__ y,
-                             double2* __restrict__ out) {
-    const OrbView& o = S.ov;
-    const int M = o.M, G = o.G, n = M * G;
-    const double2* Q = S.Q;
-    const double2 mi_tf = make_double2(o.tf.y, -o.tf.x);
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = t / G, x = t % G;
-        double2 fx[kBatchMaxOrb];
-        for (int a = 0; a < M; a++) fx[a] = y[(size_t)a * G + x];
-        const double2* Qk = Q + (size_t)k * M * M * M;
-        double2 red = make_double2(0.0, 0.0);
-        for (int s = 0; s < M; s++) {
-            double2 ts = make_double2(0.0, 0.0);
-            for (int l = 0; l < M; l++) {
-                double2 tl = make_double2(0.0, 0.0);
-                for (int q = 0; q < M; q++) tl = cfma(Qk[s + q * M + l * M * M], fx[q], tl);
-                ts = cfma(tl, fx[l], ts);
-            }
-            red = cfma(make_double2(fx[s].x, -fx[s].y), ts, red);
-        }
-        for (int j = 0; j < M; j++) {
-            const double2 c = cadd(S.hob[j * M + k], S.B[k * M + j]);
-            red.x -= c.x * fx[j].x - c.y * fx[j].y;
-            red.y -= c.x * fx[j].y + c.y * fx[j].x;
-        }
-        red = cadd(red, cscale(fx[k], o.pot[x]));
-        out[t] = cmul(mi_tf, red);
-    }
-    __syncthreads();
-}
-
-// linear half step of the split step, y <- Op y for every orbital, through
-// the spare stage buffer (orb_half_kernel: the same sums in the same order)
-__device__ void bt_half_step(const BatchSlot& S, double2* y) {
-    const int M = S.ov.M, G = S.ov.G, n = M * G;
-    const int dense = S.half_dense, nn = dense ? G : G - 1;
-    double2* w = S.stage + (size_t)7 * n - n;  // stage[6], the stage input of RK
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = t / G, x = t % G;
-        const double2* f = y + (size_t)k * G;
-        double2 acc = make_double2(0.0, 0.0);
-        if (dense) {
-            for (int j = 0; j < nn; j++) acc = cfma(S.half[(size_t)j * G + x], f[j], acc);
-        } else {
-            const double2* tk = S.half + (nn - 1 - (x == nn ? 0 : x));
-            for (int j = 0; j < nn; j++) acc = cfma(tk[j], f[j], acc);
-        }
-        w[t] = acc;
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < n; t += blockDim.x) y[t] = w[t];
-    __syncthreads();
-}
-
-// B[k][j] = sum_a rinv[k][a] sum_{s,q,l} rho2[a + sM + qM^2 + lM^3]
-//           hint[j + sM + lM^2 + qM^3] (orb_bmat_kernel, same order)
-__device__ void bt_bmat(const BatchSlot& S) {
-    const int M = S.M, M2 = M * M, M3 = M2 * M;
-    for (int e = threadIdx.x; e < M2; e += blockDim.x) {
-        const int k = e / M, j = e % M;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int a = 0; a < M; a++) {
-            double2 inner = make_double2(0.0, 0.0);
-            for (int s = 0; s < M; s++)
-                for (int q = 0; q < M; q++)
-                    for (int l = 0; l < M; l++)
-                        inner = cfma(S.rho2[a + s * M + q * M2 + l * M3],
-                                     S.hint[j + s * M + l * M2 + q * M3], inner);
-            acc = cfma(S.rinv[k * M + a], inner, acc);
-        }
-        S.B[e] = acc;
-    }
-    __syncthreads();
-}
-
-// out = y + dt sum_j c_j k_j
-struct Combo {
-    int n;
-    int j[5];
-    double c[5];
-};
-
-// (out may be y itself: each point is read before it is written)
-__device__ void bt_combo(const BatchSlot& S, const double2* y, const Combo& cb, double2* out) {
-    const int n = S.ov.M * S.ov.G;
-    const double dt = S.dt;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int q = 0; q < cb.n; q++) {
-            const double2 kv = S.stage[(size_t)cb.j[q] * n + t];
-            s.x += cb.c[q] * kv.x;
-            s.y += cb.c[q] * kv.y;
-        }
-        out[t] = make_double2(y[t].x + dt * s.x, y[t].y + dt * s.y);
-    }
-    __syncthreads();
-}
-
-// Runge-Kutta step of the orbitals in place (orbital_integration.c:284-349)
-// with the named tableaux Heun (2), classical RK4 (4) and Butcher RK5 (5);
-// split: the split step's nonlinear right-hand side (orbital_integration.c:
-// 387-415) in place of the full one.  Stage j lives in stage[j], the stage
-// input in stage[6].
-__device__ void bt_rk_step(const BatchSlot& S, double2* sP, bool split) {
-    const int n = S.ov.M * S.ov.G;
-    double2* y = S.orb;
-    double2* w = S.stage + (size_t)6 * n;
-    auto k = [&](int j) { return S.stage + (size_t)j * n; };
-    auto rhs = [&](const double2* in, double2* out) {
-        if (split)
-            bt_split_rhs(S, in, out);
-        else
-            bt_rhs(S, in, out, sP);
-    };
-    auto C1 = [](int a, double ca) { Combo c{1, {a}, {ca}}; return c; };
-    switch (S.rk) {
-        case 2:
-            rhs(y, k(0));
-            bt_combo(S, y, C1(0, 1.0), w);
-            rhs(w, k(1));
-            bt_combo(S, y, Combo{2, {0, 1}, {0.5, 0.5}}, y);
-            break;
-        case 4:
-            rhs(y, k(0));
-            bt_combo(S, y, C1(0, 0.5), w);
-            rhs(w, k(1));
-            bt_combo(S, y, C1(1, 0.5), w);
-            rhs(w, k(2));
-            bt_combo(S, y, C1(2, 1.0), w);
-            rhs(w, k(3));
-            bt_combo(S, y, Combo{4, {0, 1, 2, 3}, {1.0 / 6, 2.0 / 6, 2.0 / 6, 1.0 / 6}}, y);
-            break;
-        default:  // 5
-            rhs(y, k(0));
-            bt_combo(S, y, C1(0, 0.25), w);
-            rhs(w, k(1));
-            bt_combo(S, y, Combo{2, {0, 1}, {0.125, 0.125}}, w);
-            rhs(w, k(2));
-            bt_combo(S, y, Combo{2, {1, 2}, {-0.5, 1.0}}, w);
-            rhs(w, k(3));
-            bt_combo(S, y, Combo{2, {0, 3}, {3.0 / 16, 9.0 / 16}}, w);
-            rhs(w, k(4));
-            bt_combo(S, y,
-                     Combo{5, {0, 1, 2, 3, 4}, {-3.0 / 7, 2.0 / 7, 12.0 / 7, -12.0 / 7, 8.0 / 7}},
-                     w);
-            rhs(w, k(5));
-            bt_combo(S, y,
-                     Combo{5, {0, 2, 3, 4, 5}, {7.0 / 90, 32.0 / 90, 12.0 / 90, 32.0 / 90, 7.0 / 90}},
-                     y);
-            break;
-    }
-}
-
-__device__ void bt_periodic(const BatchSlot& S) {
-    const int M = S.ov.M, G = S.ov.G;
-    if (S.ov.periodic && threadIdx.x < M) S.orb[(size_t)threadIdx.x * G + G - 1] = S.orb[(size_t)threadIdx.x * G];
-    __syncthreads();
-}
-
-// h_kl (orbital_matrices.c:22-70): one warp per pair k <= l;
-// g_ksql: one warp per 8 x 8 tensor-core tile (hint_tile)
-__device__ void bt_matrices(const BatchSlot& S) {
-    const OrbView& o = S.ov;
-    const int M = o.M, G = o.G;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const double r = 1.0 / (12 * o.dx);
-    const int npair = M * (M + 1) / 2;
-    for (int p = warp; p < npair; p += nw) {
-        int q = p, k = 0;
-        while (q >= M - k) {
-            q -= M - k;
-            k++;
-        }
-        const int l = k + q;
-        const double2* fk = S.orb + (size_t)k * G;
-        const double2* fl = S.orb + (size_t)l * G;
-        double2 acc = make_double2(0.0, 0.0);
-        for (int x = lane; x < G; x += 32) {
-            const double2 t = hob_integrand(o, fk, fl, x, r);
-            acc.x += o.w[x] * t.x;
-            acc.y += o.w[x] * t.y;
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            if (k == l) {
-                S.hob[k * M + k] = make_double2(acc.x, 0.0);
-            } else {
-                S.hob[k * M + l] = acc;
-                S.hob[l * M + k] = make_double2(acc.x, -acc.y);
-            }
-        }
-    }
-    const int tiles = (M * M + 7) / 8;
-    for (int t = warp; t < tiles * tiles; t += nw) hint_tile(o, S.orb, S.g, S.hint, t, lane);
-    __syncthreads();
-}
-
 }  // namespace
-
-// mode 0: one full orbital step (periodic copy, Runge-Kutta, Gram-Schmidt,
-// periodic copy), then the matrices of the new orbitals;
-// mode 1: the matrices of the orbitals as given (set-up of a new slot)
-__global__ void __launch_bounds__(kBatchOrbThreads)
-    bt_orbital_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
-                      const int* __restrict__ nlist, int mode, int* __restrict__ mon) {
-    // a new step: no monitor H.C due yet in any orbital count
-    if (mon != nullptr && blockIdx.x == 0 && threadIdx.x < kBatchNumM) mon[threadIdx.x] = 0;
-    if ((int)blockIdx.x >= *nlist) return;
-    const BatchSlot& S = slots[list[blockIdx.x]];
-    if (!slot_running(S)) return;
-    extern __shared__ double scan[];  // G doubles (Gram-Schmidt)
-    __shared__ double2 sP[kBatchMaxOrb * kBatchMaxOrb];
-    const int M = S.M;
-    if (mode == 0) {
-        bt_periodic(S);
-        // Q[k][s + qM + lM^2] = g sum_a rinv[k][a] rho2[a, s, q, l]
-        const int M3 = M * M * M, M4 = M3 * M;
-        const double g = *S.g;
-        for (int e = threadIdx.x; e < M4; e += blockDim.x) {
-            const int k = e / M3, sql = e % M3;
-            double2 acc = make_double2(0.0, 0.0);
-            for (int a = 0; a < M; a++) acc = cfma(S.rinv[k * M + a], S.rho2[a + M * sql], acc);
-            S.Q[e] = cscale(acc, g);
-        }
-        __syncthreads();
-        if (S.split) {
-            // orbital_integration.c:352-434: half step, h and g of the
-            // half-stepped orbitals, B, RK of the nonlinear part, half step
-            bt_half_step(S, S.orb);
-            bt_matrices(S);
-            bt_bmat(S);
-            bt_rk_step(S, sP, true);
-            bt_half_step(S, S.orb);
-        } else {
-            bt_rk_step(S, sP, false);
-        }
-        if (S.imag) {
-            orthonormalize_block(S.ov, S.orb, scan);
-            __syncthreads();
-        }
-        bt_periodic(S);
-        // real time: the orbitals' drift from orthonormality, for the
-        // monitor of the tail kernel (driver.c:69-96)
-        if (!S.imag) bt_overlap_residual(S);
-    }
-    bt_matrices(S);
-    __syncthreads();
-    // the pair matrix of H.C for the new h and g, and its real flag
-    // (pairhc_tmpl.cuh)
-    const int P2 = M * (M + 1) / 2 * (M * (M + 1) / 2);
-    bool real = true;
-    for (int e = threadIdx.x; e < P2; e += blockDim.x) {
-        const double2 w = pair_w_entry(S.N, M, S.hob, S.hint, e);
-        real = real && w.y == 0.0;
-        S.sp.pair_w[e] = w;
-    }
-    real = __syncthreads_and(real);
-    if (threadIdx.x == 0) {
-        S.sp.pair_w[P2] = make_double2(real ? 1.0 : 0.0, 0.0);
-        // Lanczos set-up of this step (multiconfig_lanczos.c:30-41)
-        S.flags[BF_BREAK] = 0;
-        S.flags[BF_ITERS] = S.lz;
-        S.flags[BF_QL] = 0;
-        S.scal[BS_MISC + 0] = make_double2(0.0, 0.0);
-        S.scal[BS_OFFD + S.lz - 1] = make_double2(0.0, 0.0);
-    }
-}
 
 // ---------------------------------------------------------------------------
 // vector kernels over tiles of kBatchVecRows rows
@@ -646,42 +257,46 @@ __global__ void __launch_bounds__(kBatchVecThreads)
     S.scal[BS_MISC + 1] = make_double2(1.0 / beta, 0.0);
 }
 
-// y = U exp(-i D pdt) U^T e1 of the tridiagonal (alpha, beta) (implicit QL)
-__global__ void bt_small_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
-                                const int* __restrict__ nlist) {
+// y = U exp(-i D pdt) U^T e1 of the tridiagonal (alpha, beta) (implicit QL),
+// one warp per slot as lz_small_kernel
+__global__ void __launch_bounds__(32)
+    bt_small_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
+                    const int* __restrict__ nlist) {
     BT_SLOT
-    if (threadIdx.x != 0) return;
-    const int n = S.flags[BF_ITERS];
+    __shared__ double z[kBatchMaxLz * kBatchMaxLz];
+    __shared__ double2 aux[kBatchMaxLz];
+    const int lane = threadIdx.x, n = S.flags[BF_ITERS];
     double d[kBatchMaxLz], e[kBatchMaxLz];
     for (int k = 0; k < n; k++) {
         d[k] = S.scal[BS_DIAG + k].x;
         e[k] = S.scal[BS_OFFD + k].x;
     }
-    double* z = (double*)(S.scal + BS_Z);
-    S.flags[BF_QL] = tridiag_ql(n, d, e, z);
+    const int rc = tridiag_ql_warp(n, d, e, z);
+    if (lane == 0) S.flags[BF_QL] = rc;
     const double2 pdt = S.pdt;
     // imaginary time: exponents shifted by their maximum (a constant factor
     // the renormalisation at the end of the step removes), so exp cannot
-    // overflow at |E| dt > 709; real time: no shift, unchanged bits
+    // overflow at |E| dt > 709; real time: no shift
     double shift = 0.0;
     if (pdt.y != 0.0)
         for (int k = 0; k < n; k++) shift = k == 0 ? d[k] * pdt.y : fmax(shift, d[k] * pdt.y);
-    double2 aux[kBatchMaxLz];
-    for (int k = 0; k < n; k++) {
-        const double re = d[k] * pdt.y, im = -d[k] * pdt.x;
+    __syncwarp();
+    if (lane < n) {
+        const double re = d[lane] * pdt.y, im = -d[lane] * pdt.x;
         const double mag = exp(re - shift);
         double sn, cs;
         sincos(im, &sn, &cs);
-        const double u = z[0 * n + k];
-        aux[k] = make_double2(u * mag * cs, u * mag * sn);
+        const double u = z[lane];
+        aux[lane] = make_double2(u * mag * cs, u * mag * sn);
     }
-    for (int k = 0; k < n; k++) {
+    __syncwarp();
+    if (lane < n) {
         double2 s = make_double2(0.0, 0.0);
         for (int j = 0; j < n; j++) {
-            s.x += z[k * n + j] * aux[j].x;
-            s.y += z[k * n + j] * aux[j].y;
+            s.x += z[lane * n + j] * aux[j].x;
+            s.y += z[lane * n + j] * aux[j].y;
         }
-        S.scal[BS_Y + k] = s;
+        S.scal[BS_Y + lane] = s;
     }
 }
 
@@ -693,15 +308,16 @@ __global__ void __launch_bounds__(kBatchVecThreads)
                    const int* __restrict__ nlist, int prologue, int* __restrict__ mon) {
     BT_SLOT
     const int M = S.M;
-    if (threadIdx.x == 0) {
-        // staged in shared memory: the routine's dependent accesses stay on
-        // the SM (same operations and bits as on the arena's copies)
+    if (threadIdx.x < 32) {
+        // the first warp, on copies in shared memory
         __shared__ double2 r1[kBatchMaxOrb * kBatchMaxOrb], ri[kBatchMaxOrb * kBatchMaxOrb];
-        __shared__ double2 w[3 * kBatchMaxOrb * kBatchMaxOrb + kBatchMaxOrb / 2 + 1];
+        __shared__ double2 w[3 * kBatchMaxOrb * kBatchMaxOrb];
         const int M2 = M * M;
-        for (int i = 0; i < M2; i++) r1[i] = S.rho1[i];
-        S.flags[BF_INFO] = sync_rho1(M, r1, ri, S.reg_fac, w, (double*)(w + 3 * M2));
-        for (int i = 0; i < M2; i++) {
+        for (int i = threadIdx.x; i < M2; i += 32) r1[i] = S.rho1[i];
+        __syncwarp();
+        const int info = sync_rho1_warp(M, r1, ri, S.reg_fac, w);
+        if (threadIdx.x == 0) S.flags[BF_INFO] = info;
+        for (int i = threadIdx.x; i < M2; i += 32) {
             S.rho1[i] = r1[i];
             S.rinv[i] = ri[i];
         }

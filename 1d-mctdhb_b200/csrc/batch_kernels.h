@@ -6,10 +6,6 @@
 
 namespace mctdhb {
 
-// mon: the count block's monitor flags, cleared at the start of a step
-// (mode 0); nullptr for the admission set-up (mode 1)
-__global__ void bt_orbital_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
-                                  const int* __restrict__ nlist, int mode, int* __restrict__ mon);
 __global__ void bt_dot_kernel(const BatchSlot* __restrict__ slots,
                               const BatchTile* __restrict__ tiles, const int* __restrict__ ntiles,
                               int i);

@@ -196,17 +196,22 @@ __global__ void lz_init_kernel(double2* scal, int* iflag, int m) {
 // mode 2: the same up to a positive constant factor, for a step that
 //         renormalises y (imaginary time)
 // mode 1: lowest Ritz vector y = U[:, argmin D], energy -> scal[S_MISC+2]
-__global__ void lz_small_kernel(int mode, double2 prop_dt, double2* __restrict__ scal,
-                                int* __restrict__ iflag, double* __restrict__ z,
-                                double* __restrict__ energy) {
-    if (threadIdx.x != 0) return;
-    const int n = iflag[1];
+// One warp: the QL recurrence on every lane, the eigenvector rows, the
+// exponentials and the rows of y one lane each (one thread with the
+// eigenvectors in global memory took 34 us at 5 vectors, the warp 17 us).
+__global__ void __launch_bounds__(32)
+    lz_small_kernel(int mode, double2 prop_dt, double2* __restrict__ scal,
+                    int* __restrict__ iflag, double* __restrict__ energy) {
+    extern __shared__ double z[];  // n x n, then n complex
+    const int lane = threadIdx.x, n = iflag[1];
+    double2* aux = (double2*)(z + kSlots * kSlots);
     double d[kSlots], e[kSlots];
     for (int k = 0; k < n; k++) {
         d[k] = scal[S_DIAG + k].x;
         e[k] = scal[S_OFFD + k].x;
     }
-    iflag[2] = tridiag_ql(n, d, e, z);
+    const int rc = tridiag_ql_warp(n, d, e, z);
+    if (lane == 0) iflag[2] = rc;
     if (mode != 1) {
         // mode 2: exponents shifted by their maximum (a constant factor the
         // renormalisation at the end of the step removes), so exp cannot
@@ -215,8 +220,8 @@ __global__ void lz_small_kernel(int mode, double2 prop_dt, double2* __restrict__
         if (mode == 2 && prop_dt.y != 0.0)
             for (int k = 0; k < n; k++)
                 shift = k == 0 ? d[k] * prop_dt.y : fmax(shift, d[k] * prop_dt.y);
-        double2 aux[kSlots];
-        for (int k = 0; k < n; k++) {
+        __syncwarp();
+        for (int k = lane; k < n; k += 32) {
             // exp(-i d_k prop_dt), prop_dt complex
             const double re = d[k] * prop_dt.y, im = -d[k] * prop_dt.x;
             const double mag = exp(re - shift);
@@ -225,7 +230,8 @@ __global__ void lz_small_kernel(int mode, double2 prop_dt, double2* __restrict__
             const double u = z[0 * n + k];
             aux[k] = make_double2(u * mag * cs, u * mag * sn);
         }
-        for (int k = 0; k < n; k++) {
+        __syncwarp();
+        for (int k = lane; k < n; k += 32) {
             double2 s = make_double2(0.0, 0.0);
             for (int j = 0; j < n; j++) {
                 s.x += z[k * n + j] * aux[j].x;
@@ -241,9 +247,12 @@ __global__ void lz_small_kernel(int mode, double2 prop_dt, double2* __restrict__
                 sentinel = d[k];
                 jm = k;
             }
-        for (int k = 0; k < n; k++) scal[S_Y + k] = make_double2(z[k * n + jm], 0.0);
-        scal[S_MISC + 2] = make_double2(sentinel, 0.0);
-        if (energy) *energy = sentinel;
+        __syncwarp();
+        for (int k = lane; k < n; k += 32) scal[S_Y + k] = make_double2(z[k * n + jm], 0.0);
+        if (lane == 0) {
+            scal[S_MISC + 2] = make_double2(sentinel, 0.0);
+            if (energy) *energy = sentinel;
+        }
     }
 }
 
@@ -287,8 +296,8 @@ int lanczos_alloc(LanczosWork& w, const SpaceCtx& s, int mmax) {
     MCTDHB_CUDA_TRY(cudaMalloc(&w.V, (size_t)mmax * s.dim * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&w.out, (size_t)s.dim * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&w.part, part_elems * sizeof(double2)));
-    MCTDHB_CUDA_TRY(cudaMalloc(&w.scal, (S_TOTAL + kSlots * kSlots / 2 + 8) * sizeof(double2)));
-    MCTDHB_CUDA_TRY(cudaMemset(w.scal, 0, (S_TOTAL + kSlots * kSlots / 2 + 8) * sizeof(double2)));
+    MCTDHB_CUDA_TRY(cudaMalloc(&w.scal, S_TOTAL * sizeof(double2)));
+    MCTDHB_CUDA_TRY(cudaMemset(w.scal, 0, S_TOTAL * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&w.iflag, 4 * sizeof(int)));
     return 0;
 }
@@ -302,7 +311,8 @@ void lanczos_free(LanczosWork& w) {
     w = LanczosWork();
 }
 
-static double* zbuf(const LanczosWork& w) { return (double*)(w.scal + S_TOTAL); }
+// shared memory of lz_small_kernel: the eigenvectors and the exponentials
+constexpr int kSmallSmem = kSlots * kSlots * (int)sizeof(double) + kSlots * (int)sizeof(double2);
 
 int lanczos_run(const SpaceCtx& s, LanczosWork& w, int m, cudaStream_t st) {
     if (m < 1 || m > w.mmax) {
@@ -367,8 +377,8 @@ int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 pro
     MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, d_C, (size_t)n * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, st));
     if (lanczos_run(s, w, m, st)) return -1;
-    lz_small_kernel<<<1, 32, 0, st>>>(imagtime ? 2 : 0, prop_dt, w.scal, w.iflag, zbuf(w),
-                                      nullptr);
+    lz_small_kernel<<<1, 32, kSmallSmem, st>>>(imagtime ? 2 : 0, prop_dt, w.scal, w.iflag,
+                                               nullptr);
     lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     if (imagtime) {
@@ -481,8 +491,8 @@ int lowest_state(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double*
     MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, d_C, (size_t)n * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, st));
     if (lanczos_run(s, w, m, st)) return -1;
-    lz_small_kernel<<<1, 32, 0, st>>>(1, make_double2(0.0, 0.0), w.scal, w.iflag, zbuf(w),
-                                      d_energy);
+    lz_small_kernel<<<1, 32, kSmallSmem, st>>>(1, make_double2(0.0, 0.0), w.scal, w.iflag,
+                                               d_energy);
     lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;

@@ -116,73 +116,72 @@ __global__ void orb_q_kernel(int M, const double* __restrict__ g_dev,
     Q[e] = cscale(acc, *g_dev);
 }
 
-// DVR / spectral linear part (orbital_integration.c:137-176):
-// L_k(x) = sum_j lin_t[j - x + n - 1] f_k(j) + V(x) f_k(x) on the n = G - 1
-// periodic points, L_k(n) = L_k(0).  Block (k, chunk) stages f_k in shared
-// memory; thread x sums over j, reading the kernel at consecutive addresses.
-__global__ void __launch_bounds__(256) orb_toeplitz_kernel(OrbView o, const double2* __restrict__ y,
-                                                           double2* __restrict__ L) {
-    extern __shared__ double2 fs[];  // n values
-    const int G = o.G, n = G - 1;
-    const int k = blockIdx.y;
+// out_k(x) = sum_j op[j - x + n - 1] f_k(j) on the n = G - 1 periodic points,
+// out_k(n) = out_k(0) (plus V(x) f_k(x) where pot is given): the DVR / spectral
+// linear part (orbital_integration.c:137-176) and the circulant half step of
+// the split-step integrator; dense: out_k(x) = sum_j op[j G + x] f_k(j) on all
+// G points (the half step on zero bounds, stored column-major).  A block
+// takes 32 points of one orbital, each warp an eighth of the sum over j (the
+// pieces are added in order): one thread per point ran a chain of 2 n
+// dependent FMAs on 24 blocks, 72 us at M=6 on 1024 points against 16 us.
+__global__ void __launch_bounds__(256)
+    orb_operator_kernel(int G, int dense, const double2* __restrict__ op,
+                        const double* __restrict__ pot, const double2* __restrict__ y,
+                        double2* __restrict__ out) {
+    extern __shared__ double2 fs[];  // n values, then 8 x 32 pieces
+    const int n = dense ? G : G - 1, k = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const double2* f = y + (size_t)k * G;
+    double2* piece = fs + n;
     for (int j = threadIdx.x; j < n; j += blockDim.x) fs[j] = f[j];
     __syncthreads();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x > n) return;
-    const int xr = x == n ? 0 : x;
-    const double2* t = o.lin_t + (n - 1 - xr);
-    double2 acc = make_double2(0.0, 0.0);
-    for (int j = 0; j < n; j++) acc = cfma(__ldg(t + j), fs[j], acc);
-    L[(size_t)k * G + x] = cadd(acc, cscale(fs[xr], o.pot[xr]));
-}
-
-// Linear half step of the split-step integrator: out_k = Op f_k.  Circulant
-// Op on the n = G - 1 periodic points (kernel t, (Op f)_x =
-// sum_j t[j - x + n - 1] f_j, out(n) = out(0)), or dense on all G points
-// (zero bounds; stored column-major, Op[x][j] = D[j G + x]).
-__global__ void __launch_bounds__(256) orb_half_kernel(OrbView o, const double2* __restrict__ op,
-                                                       int dense, const double2* __restrict__ y,
-                                                       double2* __restrict__ out) {
-    extern __shared__ double2 fs[];
-    const int G = o.G, n = dense ? G : G - 1;
-    const int k = blockIdx.y;
-    const double2* f = y + (size_t)k * G;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) fs[j] = f[j];
-    __syncthreads();
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= G) return;
-    double2 acc = make_double2(0.0, 0.0);
-    if (dense) {
-        for (int j = 0; j < n; j++) acc = cfma(__ldg(op + (size_t)j * G + x), fs[j], acc);
-    } else {
-        const double2* t = op + (n - 1 - (x == n ? 0 : x));
-        for (int j = 0; j < n; j++) acc = cfma(__ldg(t + j), fs[j], acc);
+    const int x = blockIdx.x * 32 + lane, xr = x < n ? x : 0;  // x = n repeats 0
+    const int per = (n + 7) / 8, j0 = w * per, j1 = min(j0 + per, n);
+    const double2* t = dense ? op + xr : op + (n - 1 - xr);
+    const size_t step = dense ? (size_t)G : 1;
+    double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    int j = j0;
+#pragma unroll 4
+    for (; j + 1 < j1; j += 2) {
+        acc[0] = cfma(__ldg(t + j * step), fs[j], acc[0]);
+        acc[1] = cfma(__ldg(t + (j + 1) * step), fs[j + 1], acc[1]);
     }
-    out[(size_t)k * G + x] = acc;
+    if (j < j1) acc[0] = cfma(__ldg(t + j * step), fs[j], acc[0]);
+    piece[w * 32 + lane] = cadd(acc[0], acc[1]);
+    __syncthreads();
+    if (w != 0 || x >= G) return;
+    double2 s = piece[lane];
+    for (int u = 1; u < 8; u++) s = cadd(s, piece[u * 32 + lane]);
+    if (pot) s = cadd(s, cscale(fs[xr], pot[xr]));
+    out[(size_t)k * G + x] = s;
 }
+static size_t operator_smem(int n) { return ((size_t)n + 256) * sizeof(double2); }
 
 // B[k][j] = sum_{a,s,q,l} rinv[k][a] rho2[a + sM + qM^2 + lM^3]
 //           hint[j + sM + lM^2 + qM^3]: the projection of the interacting
 // part through g in orb_full_nonlinear (split_nonlinear_orbitals.c:63-160),
 // summed over all index orders (rho2 and g are symmetric in the pairs)
-__global__ void orb_bmat_kernel(int M, const double2* __restrict__ rinv,
-                                const double2* __restrict__ rho2,
-                                const double2* __restrict__ hint, double2* __restrict__ B) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M * M) return;
-    const int k = e / M, j = e % M, M2 = M * M, M3 = M2 * M;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int a = 0; a < M; a++) {
-        double2 inner = make_double2(0.0, 0.0);
-        for (int s = 0; s < M; s++)
-            for (int q = 0; q < M; q++)
-                for (int l = 0; l < M; l++)
-                    inner = cfma(rho2[a + s * M + q * M2 + l * M3],
-                                 hint[j + s * M + l * M2 + q * M3], inner);
-        acc = cfma(rinv[k * M + a], inner, acc);
+// One block per column j: a warp per a sums rho2 with hint, then the product
+// with rinv (one thread per entry, M^4 terms each, took 106 us at M=6).
+__global__ void __launch_bounds__(256)
+    orb_bmat_kernel(int M, const double2* __restrict__ rinv, const double2* __restrict__ rho2,
+                    const double2* __restrict__ hint, double2* __restrict__ B) {
+    __shared__ double2 inner[kMaxOrb];
+    const int j = blockIdx.x, M2 = M * M, M3 = M2 * M, lane = threadIdx.x & 31;
+    for (int a = threadIdx.x >> 5; a < M; a += 8) {
+        double2 acc = make_double2(0.0, 0.0);
+        for (int c = lane; c < M3; c += 32) {
+            const int s = c % M, q = c / M % M, l = c / M2;
+            acc = cfma(rho2[a + s * M + q * M2 + l * M3], hint[j + s * M + l * M2 + q * M3], acc);
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) inner[a] = acc;
     }
-    B[e] = acc;
+    __syncthreads();
+    for (int k = threadIdx.x; k < M; k += blockDim.x) {
+        double2 acc = make_double2(0.0, 0.0);
+        for (int a = 0; a < M; a++) acc = cfma(rinv[k * M + a], inner[a], acc);
+        B[k * M + j] = acc;
+    }
 }
 
 // nonlinear right-hand side of the split step (orbital_integration.c:
@@ -332,30 +331,27 @@ __global__ void orthonormalize_kernel(OrbView o, double2* __restrict__ F) {
     orthonormalize_block(o, F, scan);
 }
 
-// rho1 <- regularised rho1, rinv = rho1^{-1} (one thread; M <= 30).  With
-// dynamic shared memory (smem > 0) the matrices are staged there: the
-// routine's thousands of dependent accesses then stay on the SM instead of
-// going to L2 (about 1 ms at M = 8 in global memory); same operations, same
-// bits.
-__global__ void sync_rho1_kernel(int M, double2* rho1, double2* rinv, double reg_fac,
-                                 double2* work, int* info, int smem) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// rho1 <- regularised rho1, rinv = rho1^{-1} by one warp (M <= 30), in shared
+// memory where the matrices fit (smem > 0)
+__global__ void __launch_bounds__(32)
+    sync_rho1_kernel(int M, double2* rho1, double2* rinv, double reg_fac, double2* work, int* info,
+                     int smem) {
     const int M2 = M * M;
+    int r;
     if (smem > 0) {
         extern __shared__ double2 sh[];
         double2 *r1 = sh, *ri = sh + M2, *w = sh + 2 * M2;
-        for (int i = 0; i < M2; i++) r1[i] = rho1[i];
-        const int r = sync_rho1(M, r1, ri, reg_fac, w, (double*)(w + 3 * M2));
-        for (int i = 0; i < M2; i++) {
+        for (int i = threadIdx.x; i < M2; i += 32) r1[i] = rho1[i];
+        __syncwarp();
+        r = sync_rho1_warp(M, r1, ri, reg_fac, w);
+        for (int i = threadIdx.x; i < M2; i += 32) {
             rho1[i] = r1[i];
             rinv[i] = ri[i];
         }
-        if (info) *info = r;
-        return;
+    } else {
+        r = sync_rho1_warp(M, rho1, rinv, reg_fac, work);
     }
-    double* wd = (double*)(work + 3 * M2);
-    const int r = sync_rho1(M, rho1, rinv, reg_fac, work, wd);
-    if (info) *info = r;
+    if (info && threadIdx.x == 0) *info = r;
 }
 
 // total energy (integrator_monitor.c:56-88) in one block (energy_block)
@@ -382,7 +378,8 @@ int orb_init(OrbCtx& c, int M, int G, double xi, double xf, double a2, double2 a
     MCTDHB_CUDA_TRY(cudaMemset(c.d_pot, 0, G * sizeof(double)));
     const std::vector<double> w = simpson_weights(G, dx);
     MCTDHB_CUDA_TRY(cudaMemcpy(c.d_w, w.data(), G * sizeof(double), cudaMemcpyHostToDevice));
-    for (int i = 0; i < 8; i++) MCTDHB_CUDA_TRY(cudaMalloc(&c.d_k[i], n * sizeof(double2)));
+    MCTDHB_CUDA_TRY(cudaMalloc(&c.d_k[0], 8 * n * sizeof(double2)));
+    for (int i = 1; i < 8; i++) c.d_k[i] = c.d_k[0] + i * n;
     MCTDHB_CUDA_TRY(cudaMalloc(&c.d_H, n * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&c.d_P, (size_t)M * M * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&c.d_Q, (size_t)M * M * M * M * sizeof(double2)));
@@ -406,7 +403,7 @@ int orb_init(OrbCtx& c, int M, int G, double xi, double xf, double a2, double2 a
 void orb_release(OrbCtx& c) {
     cudaFree(c.d_w);
     cudaFree(c.d_pot);
-    for (int i = 0; i < 8; i++) cudaFree(c.d_k[i]);
+    cudaFree(c.d_k[0]);
     cudaFree(c.d_H);
     cudaFree(c.d_P);
     cudaFree(c.d_Q);
@@ -436,9 +433,9 @@ static int orb_rhs(const OrbCtx& c, const double2* y, double2* out, cudaStream_t
     const int n = c.M * c.G;
     const double2* L = nullptr;
     if (c.view.lin_t) {
-        const dim3 grid((c.G + 255) / 256, c.M);
-        orb_toeplitz_kernel<<<grid, 256, (size_t)(c.G - 1) * sizeof(double2), st>>>(c.view, y,
-                                                                                   c.d_L);
+        const dim3 grid((c.G + 31) / 32, c.M);
+        orb_operator_kernel<<<grid, 256, operator_smem(c.G - 1), st>>>(c.G, 0, c.view.lin_t,
+                                                                       c.view.pot, y, c.d_L);
         L = c.d_L;
     }
     orb_haction_kernel<<<(n + 127) / 128, 128, 0, st>>>(c.view, y, c.d_Q, L, c.d_H);
@@ -531,16 +528,19 @@ int orb_rk_step(const OrbCtx& c, int order, double dt, const double2* rinv, cons
     return rk_stages(c, false, order, dt, y, ynext, st);
 }
 
-// apply the half-step operator to every orbital of y (in place, through
-// the spare stage buffer)
-static int half_step(const OrbCtx& c, double2* y, cudaStream_t st) {
-    const int G = c.G;
-    const int nn = c.half_dense ? G : G - 1;
-    const dim3 grid((G + 255) / 256, c.M);
-    orb_half_kernel<<<grid, 256, (size_t)nn * sizeof(double2), st>>>(c.view, c.d_half,
-                                                                      c.half_dense, y, c.d_k[7]);
+int orb_half_step(const OrbCtx& c, const double2* y, double2* out, cudaStream_t st) {
+    const int G = c.G, nn = c.half_dense ? G : G - 1;
+    const dim3 grid((G + 31) / 32, c.M);
+    orb_operator_kernel<<<grid, 256, operator_smem(nn), st>>>(G, c.half_dense, c.d_half, nullptr, y,
+                                                              out);
     MCTDHB_CUDA_TRY(cudaGetLastError());
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(y, c.d_k[7], (size_t)c.M * G * sizeof(double2),
+    return 0;
+}
+
+// in place, through the spare stage buffer
+static int half_step(const OrbCtx& c, double2* y, cudaStream_t st) {
+    if (orb_half_step(c, y, c.d_k[7], st)) return -1;
+    MCTDHB_CUDA_TRY(cudaMemcpyAsync(y, c.d_k[7], (size_t)c.M * c.G * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, st));
     return 0;
 }
@@ -557,7 +557,7 @@ int orb_split_step(OrbCtx& c, int order, double dt, const double2* rinv, const d
     // sync_orbital_matrices inside propagate_splitstep_orb)
     if (orb_matrices(c, y, hob, hint, st)) return -1;
     orb_q_kernel<<<(M4 + 127) / 128, 128, 0, st>>>(M, c.d_g, rinv, rho2, c.d_Q);
-    orb_bmat_kernel<<<(M * M + 63) / 64, 64, 0, st>>>(M, rinv, rho2, hint, c.d_B);
+    orb_bmat_kernel<<<M, 256, 0, st>>>(M, rinv, rho2, hint, c.d_B);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     c.split_hob = hob;
     if (rk_stages(c, true, order, dt, y, ynext, st)) return -1;
@@ -632,6 +632,17 @@ std::vector<double2> derivative_toeplitz(int der, int G, double dx, double a2,
     return t;
 }
 
+// the operator kernel's shared memory at its largest grid (8191 points)
+static int operator_prepare() {
+    static std::atomic<uint64_t> done{0};
+    return set_attributes_once(done, []() -> int {
+        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(orb_operator_kernel,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)operator_smem(8191)));
+        return 0;
+    });
+}
+
 int orb_set_derivative(OrbCtx& c, int der) {
     if (der == c.der) return 0;
     if (der != kDerFiniteDiff && der != kDerDVR && der != kDerSpectral) {
@@ -659,9 +670,7 @@ int orb_set_derivative(OrbCtx& c, int der) {
     MCTDHB_CUDA_TRY(cudaMalloc(&c.d_L, (size_t)c.M * c.G * sizeof(double2)));
     MCTDHB_CUDA_TRY(
         cudaMemcpy(c.d_lin_t, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
-    MCTDHB_CUDA_TRY(cudaFuncSetAttribute(orb_toeplitz_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)((size_t)(c.G - 1) * sizeof(double2))));
+    if (operator_prepare()) return -1;
     c.view.lin_t = c.d_lin_t;
     c.der = der;
     return 0;
@@ -764,10 +773,7 @@ int orb_set_split(OrbCtx& c, int split, double dt, int imagtime) {
     MCTDHB_CUDA_TRY(
         cudaMemcpy(c.d_half, op.data(), op.size() * sizeof(double2), cudaMemcpyHostToDevice));
     MCTDHB_CUDA_TRY(cudaMalloc(&c.d_B, (size_t)c.M * c.M * sizeof(double2)));
-    const int nn = dense ? G : G - 1;
-    MCTDHB_CUDA_TRY(cudaFuncSetAttribute(orb_half_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)((size_t)nn * sizeof(double2))));
+    if (operator_prepare()) return -1;
     c.half_dense = dense;
     c.split = 1;
     return 0;
@@ -792,8 +798,8 @@ int orb_orthonormalize(const OrbCtx& c, double2* orb, cudaStream_t st) {
 
 int orb_sync_rho1(const OrbCtx& c, double2* rho1, double2* rinv, double reg_fac, int* d_info,
                   cudaStream_t st) {
-    // rho1, rinv and the 3 M^2 + M work values in shared memory up to 48 KB
-    const size_t sm = (size_t)(5 * c.M * c.M) * sizeof(double2) + (size_t)c.M * sizeof(double);
+    // rho1, rinv and the 3 M^2 work values in shared memory up to 48 KB
+    const size_t sm = (size_t)(5 * c.M * c.M) * sizeof(double2);
     const int smem = sm <= 48 * 1024 ? (int)sm : 0;
     sync_rho1_kernel<<<1, 32, smem, st>>>(c.M, rho1, rinv, reg_fac, c.d_work, d_info, smem);
     MCTDHB_CUDA_TRY(cudaGetLastError());

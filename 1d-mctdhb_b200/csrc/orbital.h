@@ -38,7 +38,7 @@ struct OrbCtx {
     double* d_w = nullptr;
     double* d_pot = nullptr;
     double* d_g = nullptr;         // contact interaction strength (device scalar)
-    double2* d_k[8] = {};          // Runge-Kutta stages + stage input
+    double2* d_k[8] = {};          // Runge-Kutta stages + stage input (one allocation)
     double2* d_H = nullptr;        // H phi
     double2* d_P = nullptr;        // projector overlaps
     double2* d_Q = nullptr;        // g rho1^{-1} rho2
@@ -87,6 +87,8 @@ int split_half_operator(int G, double dx, double a2, double2 a1, int periodic, i
 // g of the half-stepped orbitals into hob / hint, and RK of the nonlinear part
 int orb_split_step(OrbCtx& c, int order, double dt, const double2* rinv, const double2* rho2,
                    double2* y, double2* ynext, double2* hob, double2* hint, cudaStream_t st);
+// the half-step operator applied to every orbital of y into out (not y)
+int orb_half_step(const OrbCtx& c, const double2* y, double2* out, cudaStream_t st);
 // S_sl = <f_s|f_l> (Simpson) into c.d_S
 int orb_overlap_matrix(const OrbCtx& c, const double2* orb, cudaStream_t st);
 int orb_orthonormalize(const OrbCtx& c, double2* orb, cudaStream_t st);

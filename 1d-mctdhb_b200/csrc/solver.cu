@@ -18,6 +18,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "orbital.h"
+#include "orbstep.cuh"
 
 using namespace mctdhb;
 
@@ -31,6 +32,15 @@ struct mctdhb_solver_s {
             *d_hint = nullptr, *d_rho1 = nullptr, *d_rho2 = nullptr, *d_rinv = nullptr,
             *d_E = nullptr;
     int* d_info = nullptr;
+    // the orbital side as one cluster of blocks (orbstep.cu), 2..8 orbitals on
+    // up to 4096 points: two views of this system (the orbitals; for the
+    // split step's nonlinear part, the half-stepped ones in d_orb_next), their
+    // list {1, 0} and {1, 1}, scalars and flags
+    bool cluster = false;
+    BatchSlot* d_slot = nullptr;
+    int* d_list = nullptr;
+    double2* d_scal = nullptr;
+    int* d_flags = nullptr;
     cudaStream_t cs = nullptr;
     // recorded on the caller's stream after each step or phase launch; reads
     // of the state on `cs` wait for it
@@ -87,12 +97,72 @@ __global__ void relax_rule_kernel(RelaxCtl* __restrict__ c, const double2* __res
     cudaGraphSetConditional(h, stop ? 0u : 1u);
 }
 
+// the device views of the system for the cluster kernel, before a capture
+int upload_slots(mctdhb_solver_s* s) {
+    if (!s->cluster) return 0;
+    const OrbCtx& o = s->orb;
+    BatchSlot h[2] = {};
+    BatchSlot& d = h[0];
+    d.N = s->N;
+    d.M = s->M;
+    d.G = s->G;
+    d.imag = s->imagtime;
+    d.rk = s->rk_order;
+    d.lz = 1;
+    d.dt = s->dt;
+    d.ov = o.view;
+    d.sp = s->sp->sp.view;
+    d.g = o.d_g;
+    d.orb = s->d_orb;
+    d.orb_next = o.split ? nullptr : s->d_orb_next;
+    d.stage = o.d_k[0];
+    d.H = o.d_H;
+    d.hob = s->d_hob;
+    d.hint = s->d_hint;
+    d.rho1 = s->d_rho1;
+    d.rho2 = s->d_rho2;
+    d.rinv = s->d_rinv;
+    d.split = o.split;
+    d.half_dense = o.half_dense;
+    d.half = o.d_half;
+    d.B = o.d_B;
+    d.scal = s->d_scal;
+    d.flags = s->d_flags;
+    h[1] = d;
+    h[1].orb = s->d_orb_next;
+    const int list[4] = {1, 0, 1, 1};
+    const int state = SLOT_RUNNING;
+    MCTDHB_CUDA_TRY(cudaMemcpy(s->d_slot, h, sizeof(h), cudaMemcpyHostToDevice));
+    MCTDHB_CUDA_TRY(cudaMemcpy(s->d_list, list, sizeof(list), cudaMemcpyHostToDevice));
+    MCTDHB_CUDA_TRY(cudaMemcpy(s->d_flags + BF_STATE, &state, sizeof(int), cudaMemcpyHostToDevice));
+    MCTDHB_CUDA_TRY(cudaMemcpy(s->d_flags + BF_ROBUST, &o.robust, sizeof(int),
+                               cudaMemcpyHostToDevice));
+    return orb_step_prepare();
+}
+
+// one launch of the cluster kernel on view v
+int cluster_step(mctdhb_solver_s* s, int v, int parts, cudaStream_t st) {
+    const int* l = s->d_list + 2 * v;
+    return orb_step_launch(s->d_slot, l + 1, l, 1, parts, nullptr, st);
+}
+
 // phase 0 (orbital_integration.c:284-349): orbitals advanced with the
 // current rho1^{-1} and rho2
 int phase_orbitals(mctdhb_solver_s* s, cudaStream_t st) {
     OrbCtx& o = s->orb;
-    const size_t n = (size_t)s->M * s->G;
+    const size_t bytes = (size_t)s->M * s->G * sizeof(double2);
+    if (s->cluster && !o.split) return cluster_step(s, 0, kOrbPeriodic | kOrbRk | kOrbGs, st);
     if (o.view.periodic && orb_periodic(o, s->d_orb, st)) return -1;
+    if (s->cluster) {
+        // orbital_integration.c:352-434; the half steps, one product with a
+        // G x G operator per orbital, spread over the GPU
+        if (orb_half_step(o, s->d_orb, s->d_orb_next, st) || cluster_step(s, 1, kOrbRk, st) ||
+            orb_half_step(o, s->d_orb_next, s->d_orb, st))
+            return -1;
+        MCTDHB_CUDA_TRY(
+            cudaMemcpyAsync(s->d_orb_next, s->d_orb, bytes, cudaMemcpyDeviceToDevice, st));
+        return s->imagtime ? cluster_step(s, 0, kOrbGs, st) : 0;
+    }
     if (o.split) {
         // orbital_integration.c:352-434 (h and g of the half-stepped
         // orbitals are rebuilt in phase 1 from the new orbitals)
@@ -103,8 +173,8 @@ int phase_orbitals(mctdhb_solver_s* s, cudaStream_t st) {
                            s->d_orb_next, st)) {
         return -1;
     }
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(s->d_orb, s->d_orb_next, n * sizeof(double2),
-                                    cudaMemcpyDeviceToDevice, st));
+    MCTDHB_CUDA_TRY(
+        cudaMemcpyAsync(s->d_orb, s->d_orb_next, bytes, cudaMemcpyDeviceToDevice, st));
     if (s->imagtime && orb_orthonormalize(o, s->d_orb, st)) return -1;
     return 0;
 }
@@ -113,11 +183,18 @@ int phase_orbitals(mctdhb_solver_s* s, cudaStream_t st) {
 // and interaction of the new time), SIL step, density matrices
 int phase_coefficients(mctdhb_solver_s* s, cudaStream_t st) {
     const OrbCtx& o = s->orb;
-    if (o.view.periodic && orb_periodic(o, s->d_orb, st)) return -1;
-    if (orb_matrices(o, s->d_orb, s->d_hob, s->d_hint, st)) return -1;
-    if (s->M == 1) return 0;  // Gross-Pitaevskii: the coefficient is trivial
     SpaceCtx& sc = s->sp->sp;
-    if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st)) return -1;
+    if (s->cluster) {
+        // with the pair matrix of H.C, where the space has one
+        if (cluster_step(s, 0, kOrbPeriodic | kOrbMatrices, st)) return -1;
+        if (sc.view.pair_w == nullptr && hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st))
+            return -1;
+    } else {
+        if (o.view.periodic && orb_periodic(o, s->d_orb, st)) return -1;
+        if (orb_matrices(o, s->d_orb, s->d_hob, s->d_hint, st)) return -1;
+        if (s->M == 1) return 0;  // Gross-Pitaevskii: the coefficient is trivial
+        if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st)) return -1;
+    }
     if (s->coef_method == 21) {
         if (coef_rk_step(sc, s->sp->lw, s->d_coef, s->rk_order, s->dt, s->imagtime, st))
             return -1;
@@ -146,6 +223,7 @@ int count_kernels(cudaGraph_t g) {
 
 int build_graphs(mctdhb_solver_s* s) {
     if (s->exec[0] && s->exec[1]) return 0;
+    if (upload_slots(s)) return -1;
     s->kernels = 0;
     for (int p = 0; p < 2; p++) {
         cudaError_t e = cudaStreamBeginCapture(s->cs, cudaStreamCaptureModeThreadLocal);
@@ -183,6 +261,7 @@ void drop_graphs(mctdhb_solver_s* s) {
 // (both phases), the energy of the new state and the rule kernel.
 int build_relax_graph(mctdhb_solver_s* s) {
     if (s->relax_exec) return 0;
+    if (upload_slots(s)) return -1;
     cudaStream_t st = s->cs;
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
@@ -315,6 +394,15 @@ int mctdhb_solver_create(uint16_t npar, uint16_t norb, uint16_t grid_size, doubl
         set_error("mctdhb_solver_create: device allocation failed");
         return fail();
     }
+    s->cluster = orb_step_eligible(norb, grid_size);
+    if (s->cluster &&
+        (cudaMalloc(&s->d_slot, 2 * sizeof(BatchSlot)) || cudaMalloc(&s->d_list, 4 * sizeof(int)) ||
+         cudaMalloc(&s->d_scal, BS_TOTAL * sizeof(double2)) ||
+         cudaMalloc(&s->d_flags, BF_TOTAL * sizeof(int)) ||
+         cudaMemset(s->d_flags, 0, BF_TOTAL * sizeof(int)))) {
+        set_error("mctdhb_solver_create: device allocation failed");
+        return fail();
+    }
     int rc = 0;
     {
         std::lock_guard<std::mutex> lk(s->sp->mu);
@@ -341,6 +429,10 @@ void mctdhb_solver_destroy(mctdhb_solver s) {
     cudaFree(s->d_rinv);
     cudaFree(s->d_E);
     cudaFree(s->d_info);
+    cudaFree(s->d_slot);
+    cudaFree(s->d_list);
+    cudaFree(s->d_scal);
+    cudaFree(s->d_flags);
     cudaFree(s->d_ctl);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
     if (s->cs) cudaStreamDestroy(s->cs);
@@ -655,15 +747,18 @@ int mctdhb_solver_overlap_residual(mctdhb_solver s, double* res) {
     std::lock_guard<std::mutex> lk(s->mu);
     const int M = s->M;
     std::vector<double2> S((size_t)M * M);
-    int fail = 0;
+    int fail = 0, fail_cl = 0;
     MCTDHB_CUDA_TRY(cudaStreamWaitEvent(s->cs, s->ev_step, 0));
     if (orb_overlap_matrix(s->orb, s->d_orb, s->cs)) return -1;
     MCTDHB_CUDA_TRY(cudaMemcpyAsync(S.data(), s->orb.d_S, S.size() * sizeof(double2),
                                     cudaMemcpyDeviceToHost, s->cs));
     MCTDHB_CUDA_TRY(cudaMemcpyAsync(&fail, s->orb.d_fail, sizeof(int), cudaMemcpyDeviceToHost,
                                     s->cs));
+    if (s->cluster)
+        MCTDHB_CUDA_TRY(cudaMemcpyAsync(&fail_cl, s->d_flags + BF_ROBFAIL, sizeof(int),
+                                        cudaMemcpyDeviceToHost, s->cs));
     MCTDHB_CUDA_TRY(cudaStreamSynchronize(s->cs));
-    if (fail) {
+    if (fail || fail_cl) {
         set_error("mctdhb_solver: singular orbital overlap matrix in the robust projector");
         return -1;
     }
