@@ -39,6 +39,7 @@
 #include "moves.cuh"
 #include "orbital.h"
 #include "orbstep.cuh"
+#include "smallsys.h"
 
 using namespace mctdhb;
 
@@ -144,6 +145,7 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
 struct HostSlot {
     bool used = false;
     bool running = false;
+    bool small = false;  // steps on the small-space path (smallsys.h)
     size_t off = 0, bytes = 0;
     BatchSlot d{};
     JobLayout L{};
@@ -165,10 +167,15 @@ struct mctdhb_batch_s {
     // work lists (device) and their pinned host images: vector tiles, and the
     // per-M lists LIST_HG, LIST_HY, LIST_G2 (batch.h)
     size_t cap_vec = 0, cap[kBatchLists] = {};
-    int* d_list = nullptr;  // [0] count, [1..] slots
+    // slot lists: [0] count, [1..] slots.  d_list every running slot, then at
+    // multiples of max_slots + 1 the slots on the general path and, for each
+    // orbital count M, the small ones (list_at)
+    int* d_list = nullptr;
     BatchTile* d_vec = nullptr;
     BatchTile* d_tl[kBatchLists] = {};
-    int* d_cnt = nullptr;  // count block (batch.h)
+    // count blocks (batch.h): the general path's tiles, then every slot's (a
+    // list holds the tiles of the small slots behind those of the others)
+    int* d_cnt = nullptr;
     int* h_list = nullptr;
     BatchTile* h_vec = nullptr;
     BatchTile* h_tl[kBatchLists] = {};
@@ -181,14 +188,16 @@ struct mctdhb_batch_s {
     BatchTile* h_pro_g = nullptr;
     int* h_flags = nullptr;
     double2* h_scal = nullptr;
-    unsigned present_mask = 0;  // orbital counts present in the lists
+    unsigned present_mask = 0;  // orbital counts on the general path
+    unsigned small_mask = 0;    // orbital counts of the small slots
     bool lists_dirty = true;
     cudaStream_t st = nullptr;
-    cudaStream_t side[kNumM] = {};
+    cudaStream_t side[kNumM] = {}, side_small[kNumM] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[kNumM] = {};
+    cudaEvent_t ev_fork_small = nullptr, ev_join_small[kNumM] = {};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    unsigned graph_mask = 0;
+    unsigned graph_mask = 0, graph_small = 0;
     int kernels = 0;
     // the pair contraction's launch variant per orbital count, chosen by the
     // autotuner when the step graph is captured (or set by the caller)
@@ -201,6 +210,13 @@ namespace {
 
 int* cnt_vec(int* c) { return c; }
 constexpr int kCntInts = kBatchCntAll;  // with the monitor flags
+
+// slot lists of d_list / h_list: 0 all, 1 the general path, 2 + M the small
+// slots of orbital count M
+constexpr int kSlotLists = 2 + kNumM;
+int* list_at(int* base, int max_slots, int which) {
+    return base + (size_t)which * (max_slots + 1);
+}
 
 void drop_graph(mctdhb_batch_s* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -243,37 +259,53 @@ void arena_give(mctdhb_batch_s* b, size_t off, size_t bytes) {
 // the step's work lists from the running slots, uploaded on the engine stream
 int rebuild_lists(mctdhb_batch_s* b) {
     MCTDHB_CUDA_TRY(cudaStreamSynchronize(b->st));  // the pinned images are free to rewrite
-    int ns = 0;
     size_t nv = 0;
-    std::memset(b->h_cnt, 0, kCntInts * sizeof(int));
-    unsigned mask = 0;
+    std::memset(b->h_cnt, 0, 2 * kCntInts * sizeof(int));
+    int* all = b->h_cnt + kCntInts;
+    auto list = [&](int which) { return list_at(b->h_list, b->max_slots, which); };
+    for (int l = 0; l < kSlotLists; l++) list(l)[0] = 0;
+    auto add = [&](int which, int slot) { list(which)[++list(which)[0]] = slot; };
+    unsigned mask = 0, small = 0;
     for (int s = 0; s < b->max_slots; s++) {
         const HostSlot& h = b->hs[s];
         if (!h.used || !h.running) continue;
-        b->h_list[1 + ns++] = s;
+        add(0, s);
+        if (h.small) {
+            add(2 + h.d.M, s);
+            small |= 1u << h.d.M;
+            continue;
+        }
+        add(1, s);
         for (int t = 0; t < h.L.vtiles; t++) b->h_vec[nv++] = BatchTile{s, (uint32_t)t};
         mask |= 1u << h.d.M;
     }
-    b->h_list[0] = ns;
     cnt_vec(b->h_cnt)[0] = (int)nv;
     size_t n[kBatchLists] = {};
     for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++) {
-        for (int li = 0; li < kBatchLists; li++) batch_offs(b->h_cnt, li)[M] = (int)n[li];
-        for (int q = 0; q < ns; q++) {
-            const int s = b->h_list[1 + q];
-            const HostSlot& h = b->hs[s];
-            if (h.d.M != M) continue;
-            BatchTile* const* tl = b->h_tl;
-            auto push = [&](int li, uint32_t idx) {
-                if (n[li] < b->cap[li]) tl[li][n[li]] = BatchTile{s, idx};
-                n[li]++;
-            };
-            for (uint32_t r = 0; r < h.L.nc; r += kBatchHcRows) push(LIST_HG, r);
-            for (int t = 0; t < h.L.ytiles; t++) push(LIST_HY, (uint32_t)t);
-            for (int g = 0; g < h.L.gs[2]; g++) push(LIST_G2, (uint32_t)g);
-        }
+        for (int li = 0; li < kBatchLists; li++)
+            batch_offs(b->h_cnt, li)[M] = batch_offs(all, li)[M] = (int)n[li];
+        auto push_slots = [&](int which) {
+            const int* sl = list(which);
+            for (int q = 1; q <= sl[0]; q++) {
+                const int s = sl[q];
+                const HostSlot& h = b->hs[s];
+                if (h.d.M != M) continue;
+                BatchTile* const* tl = b->h_tl;
+                auto push = [&](int li, uint32_t idx) {
+                    if (n[li] < b->cap[li]) tl[li][n[li]] = BatchTile{s, idx};
+                    n[li]++;
+                };
+                for (uint32_t r = 0; r < h.L.nc; r += kBatchHcRows) push(LIST_HG, r);
+                for (int t = 0; t < h.L.ytiles; t++) push(LIST_HY, (uint32_t)t);
+                for (int g = 0; g < h.L.gs[2]; g++) push(LIST_G2, (uint32_t)g);
+            }
+        };
+        push_slots(1);
         for (int li = 0; li < kBatchLists; li++)
             batch_cnts(b->h_cnt, li)[M] = (int)n[li] - batch_offs(b->h_cnt, li)[M];
+        push_slots(2 + M);
+        for (int li = 0; li < kBatchLists; li++)
+            batch_cnts(all, li)[M] = (int)n[li] - batch_offs(all, li)[M];
     }
     bool over = nv > b->cap_vec;
     for (int li = 0; li < kBatchLists; li++) over = over || n[li] > b->cap[li];
@@ -282,9 +314,12 @@ int rebuild_lists(mctdhb_batch_s* b) {
         return -1;
     }
     cudaStream_t st = b->st;
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(b->d_list, b->h_list, (1 + ns) * sizeof(int),
-                                    cudaMemcpyHostToDevice, st));
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(b->d_cnt, b->h_cnt, kCntInts * sizeof(int),
+    for (int l = 0; l < kSlotLists; l++) {
+        const int* src = list(l);
+        MCTDHB_CUDA_TRY(cudaMemcpyAsync(list_at(b->d_list, b->max_slots, l), src,
+                                        (1 + src[0]) * sizeof(int), cudaMemcpyHostToDevice, st));
+    }
+    MCTDHB_CUDA_TRY(cudaMemcpyAsync(b->d_cnt, b->h_cnt, 2 * kCntInts * sizeof(int),
                                     cudaMemcpyHostToDevice, st));
     if (nv)
         MCTDHB_CUDA_TRY(cudaMemcpyAsync(b->d_vec, b->h_vec, nv * sizeof(BatchTile),
@@ -294,6 +329,7 @@ int rebuild_lists(mctdhb_batch_s* b) {
             MCTDHB_CUDA_TRY(cudaMemcpyAsync(b->d_tl[li], b->h_tl[li], n[li] * sizeof(BatchTile),
                                             cudaMemcpyHostToDevice, st));
     b->present_mask = mask;
+    b->small_mask = small;
     b->lists_dirty = false;
     return 0;
 }
@@ -373,18 +409,39 @@ int per_group(mctdhb_batch_s* b, unsigned mask, F&& launch) {
     return 0;
 }
 
-// the launch sequence of one batch step (captured into the step graph)
-int enqueue_step(mctdhb_batch_s* b, unsigned mask) {
+// the small slots' parts on streams of their own, one per orbital count,
+// beside what is enqueued on the engine's stream until join_small
+int fork_small(mctdhb_batch_s* b, unsigned mask, std::initializer_list<int> parts) {
+    if (mask == 0) return 0;
+    MCTDHB_CUDA_TRY(cudaEventRecord(b->ev_fork_small, b->st));
+    for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++) {
+        if (!(mask >> M & 1)) continue;
+        cudaStream_t st = b->side_small[M];
+        MCTDHB_CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork_small, 0));
+        const int* l = list_at(b->d_list, b->max_slots, 2 + M);
+        for (int p : parts)
+            if (small_batch_launch(M, b->d_slots, l + 1, l, b->max_slots, p, st)) return -1;
+        MCTDHB_CUDA_TRY(cudaEventRecord(b->ev_join_small[M], st));
+    }
+    return 0;
+}
+int join_small(mctdhb_batch_s* b, unsigned mask) {
+    for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++)
+        if (mask >> M & 1)
+            MCTDHB_CUDA_TRY(cudaStreamWaitEvent(b->st, b->ev_join_small[M], 0));
+    return 0;
+}
+
+// SIL and densities of the slots on the general path
+int enqueue_general(mctdhb_batch_s* b, unsigned mask) {
     cudaStream_t st = b->st;
     const BatchSlot* S = b->d_slots;
-    const int* nL = b->d_list;  // count in element 0, slots from element 1
-    const int* sl = b->d_list + 1;
+    const int* nL = list_at(b->d_list, b->max_slots, 1);
+    const int* sl = nL + 1;
     const BatchTile* V = b->d_vec;
     const int* nV = cnt_vec(b->d_cnt);
     const int vgrid = num_sms() * 8, sgrid = b->max_slots;
     const int lz = b->lz;
-    int* mon = batch_mon(b->d_cnt);
-    if (orb_step_launch(S, sl, nL, sgrid, kOrbStep, mon, st)) return -1;
     auto hc = [&](int iter) {
         return per_group(b, mask, [&](int M, cudaStream_t s) {
             return hc_group(M, S, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt, iter, s, 3,
@@ -413,21 +470,44 @@ int enqueue_step(mctdhb_batch_s* b, unsigned mask) {
     bt_reduce_kernel<<<sgrid, kBatchVecThreads, 0, st>>>(S, sl, nL, 1, BS_MISC + 2, 0);
     bt_renorm_kernel<<<vgrid, kBatchVecThreads, 0, st>>>(S, V, nV);
     MCTDHB_CUDA_TRY(cudaGetLastError());
-    // densities, rho1 synchronisation, energy, stop rules
-    if (per_group(b, mask, [&](int M, cudaStream_t s) {
-            return dens_group(M, S, b->d_tl[LIST_G2], b->d_cnt, sl, nL, sgrid, s);
-        }))
+    return per_group(b, mask, [&](int M, cudaStream_t s) {
+        return dens_group(M, S, b->d_tl[LIST_G2], b->d_cnt, sl, nL, sgrid, s);
+    });
+}
+
+// the launch sequence of one batch step (captured into the step graph)
+int enqueue_step(mctdhb_batch_s* b, unsigned mask, unsigned small) {
+    cudaStream_t st = b->st;
+    const BatchSlot* S = b->d_slots;
+    const int* nL = b->d_list;  // count in element 0, slots from element 1
+    const int* sl = b->d_list + 1;
+    const int sgrid = b->max_slots;
+    int* mon = batch_mon(b->d_cnt);
+    if (orb_step_launch(S, sl, nL, sgrid, kOrbStep, mon, st)) return -1;
+    // coefficients and densities: the small slots in three launches per
+    // orbital count, beside the others
+    if (fork_small(b, small, {kSmallLanczos, kSmallCombine, kSmallDens}) ||
+        (mask && enqueue_general(b, mask)) || join_small(b, small))
         return -1;
+    // rho1 synchronisation, energy, stop rules
     bt_tail_kernel<<<sgrid, kBatchVecThreads, 0, st>>>(S, sl, nL, 0, mon);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     // the monitor: the eigen residual of the slots whose energy rule passed
     // in this step with eig_tol set (driver.c:47-67); every launch returns at
     // once when no slot of its orbital count needs it
-    if (hc(kBatchMonIter)) return -1;
-    bt_resid_kernel<<<vgrid, kBatchVecThreads, 0, st>>>(S, V, nV);
-    bt_monitor_kernel<<<sgrid, kBatchVecThreads, 0, st>>>(S, sl, nL);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
-    return 0;
+    if (fork_small(b, small, {kSmallMonitor})) return -1;
+    if (mask) {
+        const int* gl = list_at(b->d_list, b->max_slots, 1);
+        if (per_group(b, mask, [&](int M, cudaStream_t s) {
+                return hc_group(M, S, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt,
+                                kBatchMonIter, s, 3, b->pair_v[M]);
+            }))
+            return -1;
+        bt_resid_kernel<<<num_sms() * 8, kBatchVecThreads, 0, st>>>(S, b->d_vec, cnt_vec(b->d_cnt));
+        bt_monitor_kernel<<<sgrid, kBatchVecThreads, 0, st>>>(S, gl + 1, gl);
+        MCTDHB_CUDA_TRY(cudaGetLastError());
+    }
+    return join_small(b, small);
 }
 
 int count_graph_kernels(cudaGraph_t g) {
@@ -462,7 +542,7 @@ int tune_group(mctdhb_batch_s* b, int M) {
     if (b->pair_v_forced[M]) return 0;
     uint64_t rows = 0;
     for (const HostSlot& h : b->hs)
-        if (h.used && h.running && h.d.M == M) rows += h.L.D2;
+        if (h.used && h.running && !h.small && h.d.M == M) rows += h.L.D2;
     int bucket = 0;
     while ((1ull << bucket) < rows) bucket++;
     BatchTuneCtx ctx{b, M};
@@ -473,17 +553,19 @@ int tune_group(mctdhb_batch_s* b, int M) {
 }
 
 int ensure_graph(mctdhb_batch_s* b) {
-    if (b->exec && b->graph_mask == b->present_mask) return 0;
+    if (b->exec && b->graph_mask == b->present_mask && b->graph_small == b->small_mask) return 0;
     drop_graph(b);
     for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++)
         if (b->present_mask >> M & 1)
             if (prepare_group(M) || tune_group(b, M)) return -1;
+    for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++)
+        if ((b->small_mask >> M & 1) && small_prepare(M)) return -1;
     cudaError_t e = cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
         set_error("batch: capture: %s", cudaGetErrorString(e));
         return -1;
     }
-    const int rc = enqueue_step(b, b->present_mask);
+    const int rc = enqueue_step(b, b->present_mask, b->small_mask);
     e = cudaStreamEndCapture(b->st, &b->graph);
     if (rc) {
         if (b->graph) cudaGraphDestroy(b->graph);
@@ -496,6 +578,7 @@ int ensure_graph(mctdhb_batch_s* b) {
         return -1;
     }
     b->graph_mask = b->present_mask;
+    b->graph_small = b->small_mask;
     b->kernels = count_graph_kernels(b->graph);
     return 0;
 }
@@ -556,14 +639,15 @@ int mctdhb_batch_create(int max_slots, size_t arena_bytes, int lanczos_iter, mct
                cudaMalloc(&b->d_slots, max_slots * sizeof(BatchSlot)) ||
                cudaMalloc(&b->d_scal, (size_t)max_slots * BS_TOTAL * sizeof(double2)) ||
                cudaMalloc(&b->d_flags, (size_t)max_slots * BF_TOTAL * sizeof(int)) ||
-               cudaMalloc(&b->d_list, (max_slots + 1) * sizeof(int)) ||
+               cudaMalloc(&b->d_list, (size_t)kSlotLists * (max_slots + 1) * sizeof(int)) ||
                cudaMalloc(&b->d_vec, b->cap_vec * sizeof(BatchTile)) ||
-               cudaMalloc(&b->d_cnt, kCntInts * sizeof(int)) ||
+               cudaMalloc(&b->d_cnt, 2 * kCntInts * sizeof(int)) ||
                cudaMalloc(&b->d_pro, (2 + kCntInts) * sizeof(int)) ||
                cudaMalloc(&b->d_pro_g, kBatchMaxSlices * sizeof(BatchTile)) ||
-               cudaMallocHost(&b->h_list, (max_slots + 1) * sizeof(int)) ||
+               cudaMallocHost(&b->h_list,
+                              (size_t)kSlotLists * (max_slots + 1) * sizeof(int)) ||
                cudaMallocHost(&b->h_vec, b->cap_vec * sizeof(BatchTile)) ||
-               cudaMallocHost(&b->h_cnt, kCntInts * sizeof(int)) ||
+               cudaMallocHost(&b->h_cnt, 2 * kCntInts * sizeof(int)) ||
                cudaMallocHost(&b->h_pro, (2 + kCntInts) * sizeof(int)) ||
                cudaMallocHost(&b->h_pro_g, kBatchMaxSlices * sizeof(BatchTile));
     for (int li = 0; li < kBatchLists && !bad; li++)
@@ -580,13 +664,16 @@ int mctdhb_batch_create(int max_slots, size_t arena_bytes, int lanczos_iter, mct
         cudaMallocHost(&b->h_flags, (size_t)max_slots * BF_TOTAL * sizeof(int)) ||
         cudaMallocHost(&b->h_scal, (size_t)max_slots * BS_TOTAL * sizeof(double2)) ||
         cudaStreamCreateWithPriority(&b->st, cudaStreamNonBlocking, prio_hi) ||
-        cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) {
+        cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) ||
+        cudaEventCreateWithFlags(&b->ev_fork_small, cudaEventDisableTiming)) {
         set_error("mctdhb_batch_create: device allocation of %zu bytes failed", b->arena_bytes);
         return fail();
     }
     for (int M = 0; M < kNumM; M++)
         if (cudaStreamCreateWithPriority(&b->side[M], cudaStreamNonBlocking, prio_hi) ||
-            cudaEventCreateWithFlags(&b->ev_join[M], cudaEventDisableTiming)) {
+            cudaStreamCreateWithPriority(&b->side_small[M], cudaStreamNonBlocking, prio_hi) ||
+            cudaEventCreateWithFlags(&b->ev_join[M], cudaEventDisableTiming) ||
+            cudaEventCreateWithFlags(&b->ev_join_small[M], cudaEventDisableTiming)) {
             set_error("mctdhb_batch_create: stream creation failed");
             return fail();
         }
@@ -622,6 +709,8 @@ void mctdhb_batch_destroy(mctdhb_batch b) {
     for (int M = 0; M < kNumM; M++) {
         if (b->side[M]) cudaStreamDestroy(b->side[M]);
         if (b->ev_join[M]) cudaEventDestroy(b->ev_join[M]);
+        if (b->side_small[M]) cudaStreamDestroy(b->side_small[M]);
+        if (b->ev_join_small[M]) cudaEventDestroy(b->ev_join_small[M]);
     }
     cudaFreeHost(b->h_list);
     cudaFreeHost(b->h_vec);
@@ -631,6 +720,7 @@ void mctdhb_batch_destroy(mctdhb_batch b) {
     cudaFreeHost(b->h_flags);
     cudaFreeHost(b->h_scal);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
+    if (b->ev_fork_small) cudaEventDestroy(b->ev_fork_small);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
 }
@@ -680,6 +770,7 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     h.off = off;
     h.bytes = L.total;
     h.L = L;
+    h.small = small_eligible(job->npar, job->norb, L.D2);
     const int N = job->npar, M = job->norb, G = job->grid_size;
     const size_t n = (size_t)M * G;
     char* base = b->arena + off;
@@ -841,7 +932,7 @@ int mctdhb_batch_step(mctdhb_batch b, int nsteps) {
     }
     std::lock_guard<std::mutex> lk(b->mu);
     if (b->lists_dirty && rebuild_lists(b)) return -1;
-    if (b->present_mask == 0) return 0;  // nothing running
+    if ((b->present_mask | b->small_mask) == 0) return 0;  // nothing running
     if (ensure_graph(b)) return -1;
     for (int i = 0; i < nsteps; i++) MCTDHB_CUDA_TRY(cudaGraphLaunch(b->exec, b->st));
     return 0;
@@ -1025,8 +1116,8 @@ int mctdhb_batch_launch_hc(mctdhb_batch b, int norb, int parts) {
     std::lock_guard<std::mutex> lk(b->mu);
     if (b->lists_dirty && rebuild_lists(b)) return -1;
     if (prepare_group(norb)) return -1;
-    return hc_group(norb, b->d_slots, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt, 0, b->st,
-                    parts, b->pair_v[norb]);
+    return hc_group(norb, b->d_slots, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt + kCntInts, 0,
+                    b->st, parts, b->pair_v[norb]);
 }
 
 int mctdhb_batch_variant(mctdhb_batch b, int norb) {

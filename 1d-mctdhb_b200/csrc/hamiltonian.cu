@@ -27,6 +27,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "smallsys.h"
 #include "wide.h"
 
 namespace mctdhb {
@@ -285,6 +286,14 @@ int hc_variant(const SpaceView& sp, const double2* C, double2* HC, const double2
 
 int hc_apply(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,
              const HcEpilogue& ep, cudaStream_t st) {
+    if (sp.pair_y != nullptr && ep.flag == nullptr && ep.prev == nullptr &&
+        small_eligible(sp.N, sp.M, sp.dim2, kSmallHcMacs)) {
+        SmallSys s{};
+        s.sp = sp;
+        s.C = const_cast<double2*>(C);  // read only here
+        s.out = HC;
+        return small_launch(s, kSmallHc, 0, st);
+    }
     if (sp.pair_y != nullptr)
         return sp.M > kMaxTemplOrb ? wide_hc(sp, C, HC, ep, st) : hcp_apply(sp, C, HC, ep, st);
     const int v = hc_variant(sp, C, HC, tab, ep, st);

@@ -25,6 +25,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "small_linalg.cuh"
+#include "smallsys.h"
 
 namespace mctdhb {
 
@@ -374,6 +375,28 @@ int lanczos_fetch(const LanczosWork& w, int m, int* iters, double2* diag, double
 int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 prop_dt,
              int imagtime, cudaStream_t st) {
     const uint32_t n = s.dim;
+    if (m <= kBatchMaxLz && s.view.pair_y != nullptr &&
+        small_eligible(s.N, s.M, s.view.dim2)) {
+        SmallSys y{};
+        y.sp = s.view;
+        y.C = d_C;
+        y.V = w.V;
+        y.out = w.out;
+        y.diag = w.scal + S_DIAG;
+        y.offd = w.scal + S_OFFD;
+        y.y = w.scal + S_Y;
+        y.misc = w.scal + S_MISC;
+        y.norm2 = w.scal + S_MISC + 3;
+        y.iflag = w.iflag;
+        y.m = m;
+        y.pdt = prop_dt;
+        y.shift = y.renorm = imagtime ? 1 : 0;
+        for (int i = 0; i < m; i++)
+            if (small_launch(y, kSmallProduct, i, st) ||
+                (i < m - 1 && small_launch(y, kSmallOrth, i, st)))
+                return -1;
+        return small_launch(y, kSmallCombine, 0, st);
+    }
     MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, d_C, (size_t)n * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, st));
     if (lanczos_run(s, w, m, st)) return -1;

@@ -1,0 +1,54 @@
+// smallsys.h -- H.C, the short iterative Lanczos step and the densities of a
+// small Fock space in one launch (smallsys.cuh).
+#pragma once
+#include "batch.h"
+#include "common.cuh"
+#include "kernels.h"
+
+namespace mctdhb {
+
+// Spaces this path takes: 2..8 orbitals, N >= 2, and a contraction of at most
+// so many complex multiply-adds (rows of the (N-2)-space times pairs^2): one
+// product is two cluster-wide passes on eight SMs, which save launches; beyond,
+// the whole GPU's tensor cores win.  Measured on one B200:
+//   one product   0.02 M (N=10 M=4)  8.4 us against 12.0 us; 0.23 M (N=24 M=4)
+//                 level; 0.45 M (N=30 M=4) 16.7 us against 13 us
+//   a Lanczos iteration adds 6 us here and 12 us of launches there: level at
+//                 0.7-0.9 M (N=11 M=6, N=16 M=5: a product takes 19-22 us)
+constexpr double kSmallHcMacs = 2.5e5, kSmallStepMacs = 7e5;
+bool small_eligible(int N, int M, uint32_t D2, double macs = kSmallStepMacs);
+
+// what one system's step works on; every pointer is device memory
+struct SmallSys {
+    SpaceView sp;     // with pair_w and the scratch pair_y
+    double2* C;       // coefficients, in and out
+    double2* V;       // m x nc Krylov vectors (V[0] may be C)
+    double2* out;     // nc
+    double2 *diag, *offd, *y;  // m each
+    double2* misc;    // [0] max beta, [1] 1 / beta
+    double2* norm2;   // |C|^2 before the renormalisation
+    int* iflag;       // [0] breakdown, [1] vectors built, [2] eigensolver status
+    double2 *rho1, *rho2;
+    int m;            // Krylov vectors, at most kBatchMaxLz
+    double2 pdt;      // exp(-i H pdt)
+    int shift;        // exponents less their maximum (a step that renormalises)
+    int renorm;
+};
+
+// parts of a step
+constexpr int kSmallHc = 0;       // out = H C
+constexpr int kSmallProduct = 1;  // iteration i of the Lanczos recurrence: H v_i, alpha_i
+constexpr int kSmallOrth = 2;     // and the reorthogonalisation, beta_i
+constexpr int kSmallLanczos = 3;  // the whole recurrence (batched slots)
+constexpr int kSmallCombine = 4;  // C <- exp(-i H pdt) C from the recurrence
+constexpr int kSmallDens = 5;     // rho1, rho2 of C (batched slots)
+constexpr int kSmallMonitor = 6;  // eigen residual where due (batched slots)
+
+int small_launch(const SmallSys& s, int part, int i, cudaStream_t st);
+// a part of the step of the batched slots of orbital count M in the list
+// (count in *nlist, at most nslots)
+int small_batch_launch(int M, const BatchSlot* slots, const int* list, const int* nlist,
+                       int nslots, int part, cudaStream_t st);
+int small_prepare(int M);  // launch attributes (before any stream capture)
+
+}  // namespace mctdhb

@@ -9,12 +9,14 @@
 // the fly); they exist for drop-in callers that read the reference's
 // MultiConfiguration fields.
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "common.cuh"
 #include "engine.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "smallsys.h"
 #include "wide.h"
 
 namespace mctdhb {
@@ -57,62 +59,65 @@ int space_init(SpaceCtx& s, int N, int M) {
         for (int L = 0; L <= N; L++) T[(size_t)m * (N + 1) + L] = (uint32_t)binom_u64(L + m, m + 1);
     std::vector<double> sq(N + 3);
     for (int x = 0; x < N + 3; x++) sq[x] = std::sqrt((double)x);
-    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_T, T.size() * sizeof(uint32_t)));
-    MCTDHB_CUDA_TRY(cudaMemcpy(s.d_T, T.data(), T.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_sq, sq.size() * sizeof(double)));
-    MCTDHB_CUDA_TRY(cudaMemcpy(s.d_sq, sq.data(), sq.size() * sizeof(double), cudaMemcpyHostToDevice));
+    const int E = dens_descriptors(M, nullptr);
+    std::vector<int> desc((size_t)5 * E);
+    dens_descriptors(M, desc.data());
+    // one allocation and one upload: rank table, square roots, density
+    // descriptors, then the room of the H.C coefficient table
+    auto al = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t o_sq = al(T.size() * sizeof(uint32_t));
+    const size_t o_desc = o_sq + al(sq.size() * sizeof(double));
+    const size_t o_tab = o_desc + al(desc.size() * sizeof(int));
+    std::vector<char> host(o_tab, 0);
+    std::memcpy(host.data(), T.data(), T.size() * sizeof(uint32_t));
+    std::memcpy(host.data() + o_sq, sq.data(), sq.size() * sizeof(double));
+    std::memcpy(host.data() + o_desc, desc.data(), desc.size() * sizeof(int));
+    char* base = nullptr;
+    MCTDHB_CUDA_TRY(cudaMalloc(&base, o_tab + (size_t)hc_table_size(M) * sizeof(double2)));
+    s.d_T = (uint32_t*)base;
+    s.d_sq = (double*)(base + o_sq);
+    s.d_dens_desc = (int*)(base + o_desc);
+    s.d_tab = (double2*)(base + o_tab);
+    MCTDHB_CUDA_TRY(cudaMemcpy(base, host.data(), o_tab, cudaMemcpyHostToDevice));
     s.view.N = N;
     s.view.M = M;
     s.view.dim = s.dim;
     s.view.T = s.d_T;
     s.view.sq = s.d_sq;
-    // H.C coefficient table
-    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_tab, (size_t)hc_table_size(M) * sizeof(double2)));
-    // density descriptors + partials
-    const int E = dens_descriptors(M, nullptr);
-    std::vector<int> desc((size_t)5 * E);
-    dens_descriptors(M, desc.data());
-    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_dens_desc, desc.size() * sizeof(int)));
-    MCTDHB_CUDA_TRY(cudaMemcpy(s.d_dens_desc, desc.data(), desc.size() * sizeof(int),
-                               cudaMemcpyHostToDevice));
-    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_dens_part, dens_partial_elems(s.view) * sizeof(double2)));
     if (dens_prepare(s.view, nullptr, nullptr, nullptr)) return -1;
-    // pair-space H.C: the pair matrix and its D(N-2, M) x P scratch; when the
-    // scratch cannot be had the space keeps the per-row kernel
-    // More than 8 orbitals: taken only where the room left still holds every
-    // Lanczos workspace a caller may ask for (64 vectors and the callers' own),
-    // so no call that ran beside the per-row kernel runs out of memory now.
+    // Density partials and, for the pair-space H.C, the pair matrix and its
+    // D(N-2, M) x P scratch, in one allocation (a large one costs 0.3 ms and
+    // as much to give back).  When the scratch cannot be had the space keeps
+    // the per-row kernel.  More than 8 orbitals: taken only where the room
+    // left still holds every Lanczos workspace a caller may ask for (64
+    // vectors and the callers' own), so no call that ran beside the per-row
+    // kernel runs out of memory now.
+    const size_t part = dens_partial_elems(s.view);
     bool pair = hcp_eligible(N, M);
     if (wide_eligible(N, M)) {
         size_t free_b = 0, total_b = 0;
         MCTDHB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
         pair = hcp_scratch_bytes(N, M) + (size_t)72 * dim * sizeof(double2) <= free_b;
     }
+    if (pair) pair = hcp_prepare(M) == 0 && (M > kMaxTemplOrb || small_prepare(M) == 0);
     if (pair) {
-        const size_t P = (size_t)M * (M + 1) / 2;
-        double2 *w = nullptr, *y = nullptr;
-        if (cudaMalloc(&w, (P * P + 1) * sizeof(double2)) == cudaSuccess &&
-            cudaMalloc(&y, hcp_scratch_bytes(N, M)) == cudaSuccess && hcp_prepare(M) == 0) {
+        const size_t P = (size_t)M * (M + 1) / 2, W = P * P + 1;
+        const size_t bytes = (part + W) * sizeof(double2) + hcp_scratch_bytes(N, M);
+        if (cudaMalloc(&s.d_dens_part, bytes) == cudaSuccess) {
             s.view.dim2 = (uint32_t)fock_dimension(N - 2, M);
-            s.view.pair_w = w;
-            s.view.pair_y = y;
-        } else {
-            cudaGetLastError();  // clear the allocation failure
-            cudaFree(w);
-            cudaFree(y);
+            s.view.pair_w = s.d_dens_part + part;
+            s.view.pair_y = s.view.pair_w + W;
+            return 0;
         }
+        cudaGetLastError();  // clear the allocation failure
     }
+    MCTDHB_CUDA_TRY(cudaMalloc(&s.d_dens_part, part * sizeof(double2)));
     return 0;
 }
 
 void space_release(SpaceCtx& s) {
-    cudaFree(s.d_T);
-    cudaFree(s.d_sq);
-    cudaFree(s.d_tab);
-    cudaFree(s.d_dens_desc);
-    cudaFree(s.d_dens_part);
-    cudaFree(s.view.pair_w);
-    cudaFree(s.view.pair_y);
+    cudaFree(s.d_T);  // with the other tables
+    cudaFree(s.d_dens_part);  // with the pair matrix and scratch
     s = SpaceCtx();
 }
 
