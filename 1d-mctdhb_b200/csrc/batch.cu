@@ -94,7 +94,7 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     // rho2 Gram slices: consecutive row tiles, at most kBatchMaxSlices (rho1
     // follows from rho2: no rho1 Gram pass)
     {
-        const uint64_t ntr = (L.D2 + gram_rows(M, 2) - 1) / gram_rows(M, 2);
+        const uint64_t ntr = (L.D2 + gram_rows(M) - 1) / gram_rows(M);
         L.gk[2] = (int)std::max<uint64_t>(1, (ntr + kBatchMaxSlices - 1) / kBatchMaxSlices);
         L.gs[2] = (int)((ntr + L.gk[2] - 1) / L.gk[2]);
     }
@@ -127,7 +127,7 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     L.o_out = take((size_t)dim * z);
     L.o_part = take((size_t)kBatchMaxLz * L.vtiles * z);
     L.o_py = take((size_t)L.D2 * P * z);
-    L.o_gpart = take((size_t)L.gs[2] * gram_entries(M, 2) * z);
+    L.o_gpart = take((size_t)L.gs[2] * gram_entries(M) * z);
     if (split && !periodic && der != 0 && der != kDerFiniteDiff) {
         set_error("batch: the split step's FFT exponential needs periodic boundaries");
         return -1;

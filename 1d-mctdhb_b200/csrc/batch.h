@@ -136,8 +136,8 @@ __host__ __device__ constexpr int batch_pair_rows(int M) {
 //                      H V[0] of the slots whose eigen residual is due;
 //                      variant: the contraction's launch variant (0 or 2,
 //                      pairhc_tmpl.cuh)
-//   gram_batch_launch  rho1 / rho2 of V[0] of the slots of orbital count M
-//                      (`list` / `nlist`: the slots, one finalize block each)
+//   gram_batch_launch  rho2 of V[0] of the slots of orbital count M (`list` /
+//                      `nlist`: the slots; rho1 follows in bt_tail_kernel)
 //   batch_prepare      launch attributes (call before any stream capture)
 template <int M>
 int hcp_batch_launch(const BatchSlot* slots, const BatchTile* hy, const BatchTile* hg,

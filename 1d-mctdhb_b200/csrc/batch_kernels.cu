@@ -12,8 +12,8 @@
 //   SIL                 tridiagonal eigenproblem, C = V U exp(-i D dt) U^T e1,
 //                       renormalisation in imaginary time
 //                       (coefficients_integration.c:59-160)
-//   densities           Gram-matrix rho1 / rho2 (per M, batch_tmpl.cuh)
-//   bt_tail_kernel      rho1 regularisation and inverse (synchronize.c:42-57),
+//   densities           Gram-matrix rho2 (per M, batch_tmpl.cuh)
+//   bt_tail_kernel      rho1 from rho2, its regularisation and inverse (synchronize.c:42-57),
 //                       energy (integrator_monitor.c:56-88), step count and
 //                       the imaginary-time stop rule (driver.c:47-67)
 // Vector kernels walk tiles of kBatchVecRows rows; every per-slot sum is
@@ -23,6 +23,7 @@
 #include "batch.h"
 #include "batch_kernels.h"
 #include "common.cuh"
+#include "gram_tmpl.cuh"
 #include "moves.cuh"
 #include "orbital_dev.cuh"
 #include "small_linalg.cuh"
@@ -300,7 +301,8 @@ __global__ void __launch_bounds__(32)
     }
 }
 
-// rho1 regularisation and inverse, energy, step count, stop rules.
+// rho1 from rho2, its regularisation and inverse, energy, step count, stop
+// rules.
 // prologue: set-up of a new slot (no step counted; the energy seeds the
 // imaginary-time stop rule as driver.c:229 does).
 __global__ void __launch_bounds__(kBatchVecThreads)
@@ -308,6 +310,8 @@ __global__ void __launch_bounds__(kBatchVecThreads)
                    const int* __restrict__ nlist, int prologue, int* __restrict__ mon) {
     BT_SLOT
     const int M = S.M;
+    rho1_from_rho2(S.N, M, S.rho2, S.rho1, threadIdx.x, blockDim.x);
+    __syncthreads();
     if (threadIdx.x < 32) {
         // the first warp, on copies in shared memory
         __shared__ double2 r1[kBatchMaxOrb * kBatchMaxOrb], ri[kBatchMaxOrb * kBatchMaxOrb];

@@ -186,59 +186,50 @@ __global__ void __launch_bounds__(kBatchHcRows)
 
 // rho2 Gram partial of slice `idx` of a slot: its gk[2] consecutive row
 // tiles of the (N-2)-boson space, summed into gpart (gram_tmpl.cuh building
-// blocks); rho1 follows from rho2 in bgram_finalize_kernel
+// blocks)
 template <int M>
 __global__ void __launch_bounds__(kGramThreads, 2)
     bgram_kernel(const BatchSlot* __restrict__ slots, const BatchTile* __restrict__ tiles,
                  const int* __restrict__ cnt) {
-    constexpr int R = 2;
-    using GS = GramShape<M, R>;
+    using GS = GramShape<M>;
     extern __shared__ double2 As[];
     const int nt = batch_cnt(cnt, LIST_G2, M);
     const BatchTile* list = tiles + batch_off(cnt, LIST_G2, M);
-    const GramRole<M, R> role(threadIdx.x);
+    GramAcc<M> acc(threadIdx.x);
     for (int k = blockIdx.x; k < nt; k += gridDim.x) {
         const BatchTile tl = list[k];
         const BatchSlot& S = slots[tl.slot];
         if (S.flags[BF_STATE] != SLOT_RUNNING) continue;  // block-uniform
         const uint32_t Dp = S.sp.dim2;
         const uint32_t ntr = (Dp + GS::ROWS - 1) / GS::ROWS;
-        const uint32_t t0 = tl.idx * (uint32_t)S.gk[R];
-        const uint32_t t1 = min(t0 + (uint32_t)S.gk[R], ntr);
-        double2 acc[GS::RT][GS::RT];
-#pragma unroll
-        for (int a = 0; a < GS::RT; a++)
-#pragma unroll
-            for (int b = 0; b < GS::RT; b++) acc[a][b] = make_double2(0.0, 0.0);
+        const uint32_t t0 = tl.idx * (uint32_t)S.gk[2];
+        const uint32_t t1 = min(t0 + (uint32_t)S.gk[2], ntr);
+        acc.clear();
         for (uint32_t tr = t0; tr < t1; tr++) {
-            gram_gather<M, R>(S.sp, Dp, S.V, tr, As, threadIdx.x);
+            gram_gather<M>(S.sp, Dp, S.V, tr, As, threadIdx.x);
             __syncthreads();
-            gram_accumulate<M, R>(As, role, acc);
+            acc.add(As);
             __syncthreads();
         }
-        gram_store<M, R>(role, acc, As, S.gpart + (size_t)tl.idx * gram_entries(M, 2));
+        acc.store(As, S.gpart + (size_t)tl.idx * GS::ENT);
     }
 }
 
-// rho2 of every running slot of orbital count M: fixed-order sum of the
-// slot's slices and the reference's symmetric fill (gram_fill); then rho1
-// from rho2 (rho1_from_rho2: every batched job has two or more bosons)
+// rho2 of the running slots of orbital count M (blockIdx.x), 32 entries a
+// block (blockIdx.y): fixed-order sum of the slot's slices and the reference's
+// symmetric fill (gram_fill); rho1 follows from rho2 in bt_tail_kernel
 template <int M>
 __global__ void __launch_bounds__(kBatchVecThreads)
     bgram_finalize_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
                           const int* __restrict__ nlist) {
+    static_assert(kBatchVecThreads == 256, "gram_sum_parts");
     if ((int)blockIdx.x >= *nlist) return;
     const BatchSlot& S = slots[list[blockIdx.x]];
     if (S.M != M || S.flags[BF_STATE] != SLOT_RUNNING) return;  // block-uniform
-    constexpr int ENT2 = gram_entries(M, 2);
-    const int ns = S.gs[2];
-    for (int e = threadIdx.x; e < ENT2; e += blockDim.x) {
-        double2 v = make_double2(0.0, 0.0);
-        for (int q = 0; q < ns; q++) v = cadd(v, S.gpart[(size_t)q * ENT2 + e]);
-        gram_fill<M>(2, e, v, S.rho1, S.rho2);
-    }
-    __syncthreads();  // the block's rho2 stores are visible to the whole block
-    rho1_from_rho2<M>(S.sp.N, S.rho2, S.rho1, threadIdx.x, blockDim.x);
+    constexpr int ENT = gram_entries(M);
+    const int e = blockIdx.y * 32 + (threadIdx.x & 31);
+    const double2 v = gram_sum_parts(S.gpart + e, S.gs[2], ENT, e < ENT);
+    if (threadIdx.x < 32 && e < ENT) gram_fill<M>(e, v, S.rho2);
 }
 
 template <int M, int V>
@@ -270,7 +261,7 @@ int batch_prepare() {
         if (batch_y_attr<M, 0>() || batch_y_attr<M, 2>() || batch_y_attr<M, 3>()) return -1;
         MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bgram_kernel<M>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             gram_smem(M, 2)));
+                                             gram_smem(M)));
         return 0;
     });
 }
@@ -308,9 +299,10 @@ int hcp_batch_launch(const BatchSlot* slots, const BatchTile* hy, const BatchTil
 template <int M>
 int gram_batch_launch(const BatchSlot* slots, const BatchTile* g2, const int* cnt,
                       const int* list, const int* nlist, int nblocks, cudaStream_t st) {
-    bgram_kernel<M><<<num_sms() * 2, kGramThreads, gram_smem(M, 2), st>>>(slots, g2, cnt);
+    bgram_kernel<M><<<num_sms() * 2, kGramThreads, gram_smem(M), st>>>(slots, g2, cnt);
     MCTDHB_CUDA_TRY(cudaGetLastError());
-    bgram_finalize_kernel<M><<<std::max(nblocks, 1), kBatchVecThreads, 0, st>>>(slots, list, nlist);
+    const dim3 fin(std::max(nblocks, 1), (gram_entries(M) + 31) / 32);
+    bgram_finalize_kernel<M><<<fin, kBatchVecThreads, 0, st>>>(slots, list, nlist);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;
 }

@@ -4,7 +4,7 @@
 namespace mctdhb {
 template int dens_launch_tmpl<4>(const SpaceView&, const double2*, double2*, int, int,
                                   cudaStream_t);
-template int gram_apply_tmpl<4>(const SpaceView&, uint32_t, uint32_t, const double2*, double2*,
+template int gram_apply_tmpl<4>(const SpaceView&, uint32_t, const double2*, double2*,
                                   double2*, double2*, cudaStream_t);
 template int gram_prepare_tmpl<4>();
 }

@@ -174,35 +174,34 @@ static int dens_slices(const SpaceView& sp) {
     return dens_templated(sp.M) ? dens_grid(sp) : dens_grid(sp) * 4;
 }
 
-// rows of the one- and two-boson-annihilated spaces (0 when empty)
-static uint32_t annihilated_dim(const SpaceView& sp, int R) {
-    return sp.N >= R ? (uint32_t)fock_dimension(sp.N - R, sp.M) : 0u;
+// rows of the two-boson-annihilated space (0 when empty)
+static uint32_t annihilated_dim(const SpaceView& sp) {
+    return sp.N >= 2 ? (uint32_t)fock_dimension(sp.N - 2, sp.M) : 0u;
 }
 
 size_t gram_partial_elems(const SpaceView& sp) {
-    return (size_t)gram_blocks(sp.M, 2, annihilated_dim(sp, 2)) * gram_entries(sp.M, 2) +
-           (size_t)gram_blocks(sp.M, 1, annihilated_dim(sp, 1)) * gram_entries(sp.M, 1);
+    return (size_t)gram_blocks(sp.M, annihilated_dim(sp)) * gram_entries(sp.M);
 }
 
 size_t dens_partial_elems(const SpaceView& sp) {
     const size_t per_row = (size_t)dens_slices(sp) * dens_ep(sp.M);
     if (wide_eligible(sp.N, sp.M))
-        return std::max(per_row, wide_gram_elems(sp.M, annihilated_dim(sp, 2)));
+        return std::max(per_row, wide_gram_elems(sp.M, annihilated_dim(sp)));
     return dens_templated(sp.M) ? std::max(per_row, gram_partial_elems(sp)) : per_row;
 }
 
 // M <= 8: the Gram-matrix kernels (gram_tmpl.cuh)
 static int gram_apply(const SpaceView& sp, const double2* C, double2* partial, double2* rho1,
                       double2* rho2, cudaStream_t st) {
-    const uint32_t D2 = annihilated_dim(sp, 2), D1 = annihilated_dim(sp, 1);
+    const uint32_t D2 = annihilated_dim(sp);
     switch (sp.M) {
-        case 2: return gram_apply_tmpl<2>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 3: return gram_apply_tmpl<3>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 4: return gram_apply_tmpl<4>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 5: return gram_apply_tmpl<5>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 6: return gram_apply_tmpl<6>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 7: return gram_apply_tmpl<7>(sp, D2, D1, C, partial, rho1, rho2, st);
-        case 8: return gram_apply_tmpl<8>(sp, D2, D1, C, partial, rho1, rho2, st);
+        case 2: return gram_apply_tmpl<2>(sp, D2, C, partial, rho1, rho2, st);
+        case 3: return gram_apply_tmpl<3>(sp, D2, C, partial, rho1, rho2, st);
+        case 4: return gram_apply_tmpl<4>(sp, D2, C, partial, rho1, rho2, st);
+        case 5: return gram_apply_tmpl<5>(sp, D2, C, partial, rho1, rho2, st);
+        case 6: return gram_apply_tmpl<6>(sp, D2, C, partial, rho1, rho2, st);
+        case 7: return gram_apply_tmpl<7>(sp, D2, C, partial, rho1, rho2, st);
+        case 8: return gram_apply_tmpl<8>(sp, D2, C, partial, rho1, rho2, st);
     }
     set_error("gram_apply: %d orbitals outside 2..8", sp.M);
     return -1;
@@ -276,7 +275,7 @@ int dens_apply(const SpaceView& sp, const double2* C, double2* partial, double2*
                double2* rho2, const int* d_desc, cudaStream_t st) {
     if (dens_templated(sp.M)) return gram_apply(sp, C, partial, rho1, rho2, st);
     if (wide_eligible(sp.N, sp.M))
-        return wide_dens(sp, annihilated_dim(sp, 2), C, partial, rho1, rho2, st);
+        return wide_dens(sp, annihilated_dim(sp), C, partial, rho1, rho2, st);
     return dens_apply_rows(sp, C, partial, rho1, rho2, d_desc, st);
 }
 

@@ -53,12 +53,12 @@ int hc_launch_tmpl(const SpaceView& sp, const double2* C, double2* HC, const dou
 template <int M>
 int dens_launch_tmpl(const SpaceView& sp, const double2* C, double2* partial, int grid,
                      int variant, cudaStream_t st);
-// rho1/rho2 as Gram matrices of the one- and two-boson-annihilated states
-// (gram_tmpl.cuh): D2 = D(N-2, M), D1 = D(N-1, M) rows; partial holds
-// gram_partial_elems(M, D2, D1) complex
+// rho1/rho2 from the Gram matrix of the two-boson-annihilated states
+// (gram_tmpl.cuh): D2 = D(N-2, M) rows; partial holds gram_partial_elems
+// complex
 template <int M>
-int gram_apply_tmpl(const SpaceView& sp, uint32_t D2, uint32_t D1, const double2* C,
-                    double2* partial, double2* rho1, double2* rho2, cudaStream_t st);
+int gram_apply_tmpl(const SpaceView& sp, uint32_t D2, const double2* C, double2* partial,
+                    double2* rho1, double2* rho2, cudaStream_t st);
 template <int M>
 int gram_prepare_tmpl();
 

@@ -341,7 +341,7 @@ struct SmallRun {
     }
 
     // rho2 as the Gram matrix of the A planes (in the scratch of Y), a warp an
-    // entry of the upper triangle; rho1 as its partial trace
+    // entry of the upper triangle
     __device__ __forceinline__ void densities() {
         const uint32_t D2 = sp.dim2;
         double2* A = s.sp.pair_y;
@@ -384,8 +384,7 @@ struct SmallRun {
                     s.rho2[k + t * M + q * M2 + l * M3] = acc;
             }
         }
-        cl.sync();
-        if (rank == 0) rho1_from_rho2<M>(sp.N, s.rho2, s.rho1, threadIdx.x, kSmThreads);
+        // rho1 follows from rho2 in bt_tail_kernel
     }
 };
 
@@ -428,7 +427,6 @@ __global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
     s.misc = S.scal + BS_MISC;
     s.norm2 = S.scal + BS_MISC + 2;
     s.iflag = S.flags;
-    s.rho1 = S.rho1;
     s.rho2 = S.rho2;
     s.m = S.lz;
     s.pdt = S.pdt;

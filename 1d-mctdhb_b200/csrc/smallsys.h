@@ -28,7 +28,7 @@ struct SmallSys {
     double2* misc;    // [0] max beta, [1] 1 / beta
     double2* norm2;   // |C|^2 before the renormalisation
     int* iflag;       // [0] breakdown, [1] vectors built, [2] eigensolver status
-    double2 *rho1, *rho2;
+    double2* rho2;
     int m;            // Krylov vectors, at most kBatchMaxLz
     double2 pdt;      // exp(-i H pdt)
     int shift;        // exponents less their maximum (a step that renormalises)
@@ -41,7 +41,7 @@ constexpr int kSmallProduct = 1;  // iteration i of the Lanczos recurrence: H v_
 constexpr int kSmallOrth = 2;     // and the reorthogonalisation, beta_i
 constexpr int kSmallLanczos = 3;  // the whole recurrence (batched slots)
 constexpr int kSmallCombine = 4;  // C <- exp(-i H pdt) C from the recurrence
-constexpr int kSmallDens = 5;     // rho1, rho2 of C (batched slots)
+constexpr int kSmallDens = 5;     // rho2 of C (batched slots)
 constexpr int kSmallMonitor = 6;  // eigen residual where due (batched slots)
 
 int small_launch(const SmallSys& s, int part, int i, cudaStream_t st);
