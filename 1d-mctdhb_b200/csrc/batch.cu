@@ -126,7 +126,7 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     L.o_V = take((size_t)lz * dim * z);
     L.o_out = take((size_t)dim * z);
     L.o_part = take((size_t)kBatchMaxLz * L.vtiles * z);
-    L.o_py = take((size_t)L.D2 * P * z);
+    L.o_py = take((size_t)pair_ld(L.D2) * P * z);
     L.o_gpart = take((size_t)L.gs[2] * gram_entries(M) * z);
     if (split && !periodic && der != 0 && der != kDerFiniteDiff) {
         set_error("batch: the split step's FFT exponential needs periodic boundaries");
@@ -815,6 +815,7 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     d.sp.T = (const uint32_t*)P(L.o_T);
     d.sp.sq = (const double*)P(L.o_sq);
     d.sp.dim2 = L.D2;
+    d.sp.ldy = pair_ld(L.D2);
     d.sp.pair_w = (double2*)P(L.o_pw);
     d.sp.pair_y = (double2*)P(L.o_py);
     d.g = (const double*)P(L.o_g);

@@ -26,14 +26,14 @@ __device__ __forceinline__ bool bt_hc_active(const BatchSlot& S, int iter) {
 // Pair contraction Y = A W^T of V[iter] for every tile of list LIST_HY:
 // warp-specialised and double-buffered as hcp_y_kernel.  Consecutive tiles
 // may belong to different slots, so the producer warps stage a tile's W with
-// its A (skipped when the buffer already holds that slot's W) and publish
-// the tile's output row, size, Y plane and real-W flag in shared memory; the
-// consumers start on the tensor cores without a chain of global loads.  The
-// next tile's descriptor is loaded one tile ahead.
+// its A and publish the tile's output row, size, Y plane and real-W flag in
+// shared memory; the consumers start on the tensor cores without a chain of
+// global loads.
 struct PairTileMeta {
     double2* Y;
-    uint32_t row0, D2;
+    uint32_t row0, D2, ld;
     int active, real;
+    int wbuf;  // variant 3: how many times W has been staged before this tile's
 };
 
 template <int M, int V>
@@ -41,76 +41,137 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
     bhcp_y_kernel(const BatchSlot* __restrict__ slots, const BatchTile* __restrict__ tiles,
                   const int* __restrict__ cnt, int iter) {
     using PS_ = PairHcShape<M, V>;
-    constexpr int P = PS_::P, PS = PS_::PS, ROWS = PS_::ROWS;
+    constexpr int P = PS_::P, PS = PS_::PS, ROWS = PS_::ROWS, WW = PS_::WWORDS;
     static_assert(ROWS == batch_pair_rows(M), "tile rows of the host lists");
     extern __shared__ double2 smem[];
-    __shared__ PairTileMeta meta[2];
-    constexpr int WS = PS_::WS;
-    double2* Wb = smem;               // two buffers of P x WS
-    double2* Ab = smem + 2 * P * WS;  // two buffers of ROWS x PS
+    double2* Ab = smem;                  // two buffers of ROWS x PS
+    double2* Wb = smem + 2 * ROWS * PS;  // two buffers of W
+    void* tab = Wb + 2 * WW;
     if (iter == kBatchMonIter && batch_mon(cnt)[M] == 0) return;  // no residual due
     const int nt = batch_cnt(cnt, LIST_HY, M);
     const BatchTile* list = tiles + batch_off(cnt, LIST_HY, M);
-    const int t = threadIdx.x;
-    __shared__ uint64_t bar_full[2], bar_empty[2];  // variant 3's handover
-    if constexpr (PS_::MBAR) {
-        if (t == 0) {
-            mbar_init(&bar_full[0], PS_::PRODUCERS);
-            mbar_init(&bar_full[1], PS_::PRODUCERS);
-            mbar_init(&bar_empty[0], PS_::CONSUMERS);
-            mbar_init(&bar_empty[1], PS_::CONSUMERS);
+    const int t = threadIdx.x, lane = t & 31;
+    const int vin = iter < 0 ? 0 : iter;  // input vector V[vin]
+    const int pt = t - PS_::CONSUMERS;
+    auto tables = [&](const SpaceView& sp) {  // the view on the staged tables
+        SpaceView v = sp;
+        if (pair_tab_fits(sp.N, M)) {
+            v.sq = (const double*)tab;
+            v.T = (const uint32_t*)((const double*)tab + sp.N + 3);
+        }
+        return v;
+    };
+    if constexpr (PS_::PIPE) {
+        // Chunks of 32 rows from producer warp to consumer warp (hcp_y_kernel,
+        // variant 3): pair w takes rows 32 w .. 32 w + 31 of every tile.  When
+        // the slot changes, all producer warps meet, stage its tables and W
+        // (into the buffer of the slot before the last, once every consumer
+        // warp has left that slot) and go on; the consumers of a tile wait for
+        // its W.  A wait that runs out marks the tile's job aborted; after one
+        // the warp waits for nothing more, so the others are not held up.
+        __shared__ PairTileMeta meta[PS_::PW][2];
+        __shared__ uint64_t full[PS_::PW][2], empty[PS_::PW][2], wfull[2], wdone[2];
+        if (t < 2 * PS_::PW) {
+            mbar_init(&full[t >> 1][t & 1], 32);
+            mbar_init(&empty[t >> 1][t & 1], 32 * PS_::CPP);
+        }
+        if (t < 2) {
+            mbar_init(&wfull[t], PS_::PRODUCERS);
+            mbar_init(&wdone[t], PS_::CONSUMERS);
         }
         __syncthreads();
+        bool lost = false;
+        auto wait = [&](uint64_t* bar, unsigned parity, int slot) {
+            if (!lost && !mbar_wait(bar, parity)) {
+                lost = true;
+                slots[slot].flags[BF_STATE] = SLOT_ABORTED;
+            }
+        };
+        const int w = t >= PS_::CONSUMERS ? pt >> 5 : (t >> 5) / PS_::CPP;
+        double2* ring = Ab + w * 2 * 32 * PS;
+        int i = 0;
+        if (t >= PS_::CONSUMERS) {
+            pair_regs_dec<PS_::CREG, PS_::PREG>();
+            int slot = -1, ver = -1;
+            BatchTile next{};
+            if ((int)blockIdx.x < nt) next = list[blockIdx.x];
+            for (int k = blockIdx.x; k < nt; k += gridDim.x, i++) {
+                const BatchTile tl = next;
+                if (k + (int)gridDim.x < nt) next = list[k + gridDim.x];
+                const BatchSlot& S = slots[tl.slot];
+                const int buf = i & 1;
+                if (tl.slot != slot) {
+                    slot = tl.slot;
+                    ver++;
+                    pair_producer_barrier<PS_::PRODUCERS>();  // nobody reads the old tables
+                    pair_stage_tab(S.sp, tab, pt, PS_::PRODUCERS);
+                    if (ver >= 2) wait(&wdone[ver & 1], ((ver >> 1) - 1) & 1, tl.slot);
+                    pair_stage_w<M, V>(S.sp.pair_w, Wb + (ver & 1) * WW, pt, PS_::PRODUCERS);
+                    mbar_arrive(&wfull[ver & 1]);
+                    pair_producer_barrier<PS_::PRODUCERS>();
+                }
+                if (i >= 2) wait(&empty[w][buf], ((i >> 1) - 1) & 1, tl.slot);
+                const uint32_t row0 = tl.idx * (uint32_t)ROWS + w * 32;
+                const bool active = bt_hc_active(S, iter) && row0 < S.sp.dim2;
+                if (lane == 0)
+                    meta[w][buf] = PairTileMeta{S.sp.pair_y, row0, S.sp.dim2, S.sp.ldy, active,
+                                                active && S.sp.pair_w[P * P].x != 0.0, ver};
+                if (active)
+                    pair_gather_row<M, V>(tables(S.sp), S.V + (size_t)vin * S.nc, row0 + lane,
+                                          ring + buf * 32 * PS, lane);
+                mbar_arrive(&full[w][buf]);
+            }
+        } else {
+            pair_regs_inc<PS_::CREG>();
+            int ver = -1;
+            for (int k = blockIdx.x; k < nt; k += gridDim.x, i++) {
+                const int buf = i & 1, slot = list[k].slot;
+                wait(&full[w][buf], (i >> 1) & 1, slot);
+                const PairTileMeta tm = meta[w][buf];
+                if (tm.wbuf != ver) {
+                    if (ver >= 0) mbar_arrive(&wdone[ver & 1]);
+                    ver = tm.wbuf;
+                    wait(&wfull[ver & 1], (ver >> 1) & 1, slot);
+                }
+                if (tm.active && !lost)
+                    pair_strips<M, V>(ring + buf * 32 * PS, Wb + (ver & 1) * WW,
+                                      (t >> 5) % PS_::CPP, PS_::CPP, 2, lane, tm.row0, tm.D2,
+                                      tm.ld, tm.Y, tm.real != 0);
+                mbar_arrive(&empty[w][buf]);
+            }
+        }
+        return;
     }
     // Producers and consumers run their own loops and meet at one block
     // barrier per tile (named barrier 1 over all threads): the producers
-    // fill buffer buf ^ 1 while the consumers contract buffer buf.
+    // fill buffer buf ^ 1 while the consumers contract buffer buf.  W is
+    // skipped when the buffer already holds the slot's; the next tile's
+    // descriptor is loaded one tile ahead.
+    __shared__ PairTileMeta meta[2];
     if (t >= PS_::CONSUMERS) {
-        const int pt = t - PS_::CONSUMERS;
-        const int vin = iter < 0 ? 0 : iter;  // input vector V[vin]
         int wslot[2] = {-1, -1};  // slot whose W each buffer holds (same in every producer)
         int tslot = -1;           // slot whose tables the shared table area holds
-        void* tab = Ab + 2 * ROWS * PS;
         auto fill = [&](const BatchTile tl, int buf) {
             const BatchSlot& S = slots[tl.slot];
             const bool active = bt_hc_active(S, iter);
             if (pt == 0)
-                meta[buf] = PairTileMeta{S.sp.pair_y, tl.idx * (uint32_t)ROWS, S.sp.dim2, active,
-                                         active && S.sp.pair_w[P * P].x != 0.0};
-            if (!active) return;
+                meta[buf] = PairTileMeta{S.sp.pair_y, tl.idx * (uint32_t)ROWS, S.sp.dim2, S.sp.ldy,
+                                         active, active && S.sp.pair_w[P * P].x != 0.0, 0};
             if (wslot[buf] != tl.slot) {
-                pair_stage_w<M, V>(S.sp.pair_w, Wb + buf * P * WS, pt, PS_::PRODUCERS);
+                pair_stage_w<M, V>(S.sp.pair_w, Wb + buf * WW, pt, PS_::PRODUCERS);
                 wslot[buf] = tl.slot;
             }
             // the slot's rank tables: the previous fill's reads ended at the
             // last block barrier; the producers meet before the new reads
-            SpaceView tv = S.sp;
             if (tslot != tl.slot) {
-                tv = pair_stage_tab(S.sp, tab, pt, PS_::PRODUCERS);
+                pair_stage_tab(S.sp, tab, pt, PS_::PRODUCERS);
                 pair_producer_barrier<PS_::PRODUCERS>();
                 tslot = tl.slot;
-            } else if (pair_tab_fits(S.sp.N, M)) {
-                tv.sq = (const double*)tab;
-                tv.T = (const uint32_t*)((const double*)tab + S.sp.N + 3);
             }
-            pair_gather<M, V>(tv, S.V + (size_t)vin * S.nc, tl.idx,
-                              Ab + (size_t)buf * ROWS * PS, pt, PS_::PRODUCERS);
+            if (active)
+                pair_gather<M, V>(tables(S.sp), S.V + (size_t)vin * S.nc, tl.idx,
+                                  Ab + (size_t)buf * ROWS * PS, pt, PS_::PRODUCERS);
         };
-        if constexpr (PS_::MBAR) {
-            // item i goes to buffer i & 1 once the consumers released it
-            // (their item i - 2), then the buffer is marked full
-            int i = 0;
-            for (int k = blockIdx.x; k < nt; k += gridDim.x, i++) {
-                const int buf = i & 1;
-                if (i >= 2 && !mbar_wait(&bar_empty[buf], ((i >> 1) - 1) & 1)) {
-                    slots[list[k].slot].flags[BF_STATE] = SLOT_ABORTED;  // handover lost
-                    return;
-                }
-                fill(list[k], buf);
-                mbar_arrive(&bar_full[buf]);
-            }
-            return;
-        }
         BatchTile next{};
         if ((int)blockIdx.x < nt) fill(list[blockIdx.x], 0);
         if ((int)(blockIdx.x + gridDim.x) < nt) next = list[blockIdx.x + gridDim.x];
@@ -125,29 +186,13 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
             pair_tile_barrier<PS_::THREADS>();
         }
     } else {
-        if constexpr (PS_::MBAR) {
-            int i = 0;
-            for (int k = blockIdx.x; k < nt; k += gridDim.x, i++) {
-                const int buf = i & 1;
-                if (!mbar_wait(&bar_full[buf], (i >> 1) & 1)) {
-                    slots[list[k].slot].flags[BF_STATE] = SLOT_ABORTED;  // handover lost
-                    return;
-                }
-                const PairTileMeta tm = meta[buf];
-                if (tm.active)
-                    pair_consume<M, V>(Ab + (size_t)buf * ROWS * PS, Wb + buf * P * WS, t,
-                                       tm.row0, tm.D2, tm.Y, tm.real != 0);
-                mbar_arrive(&bar_empty[buf]);
-            }
-            return;
-        }
         pair_tile_barrier<PS_::THREADS>();
         int buf = 0;
         for (int k = blockIdx.x; k < nt; k += gridDim.x, buf ^= 1) {
             const PairTileMeta tm = meta[buf];
             if (tm.active)
-                pair_consume<M, V>(Ab + (size_t)buf * ROWS * PS, Wb + buf * P * WS, t, tm.row0,
-                                   tm.D2, tm.Y, tm.real != 0);
+                pair_consume<M, V>(Ab + (size_t)buf * ROWS * PS, Wb + buf * WW, t, tm.row0, tm.D2,
+                                   tm.ld, tm.Y, tm.real != 0);
             pair_tile_barrier<PS_::THREADS>();
         }
     }
@@ -235,7 +280,7 @@ __global__ void __launch_bounds__(kBatchVecThreads)
 template <int M, int V>
 constexpr size_t batch_y_smem() {
     using PS_ = PairHcShape<M, V>;
-    return (2 * (size_t)PS_::P * PS_::WS + 2 * (size_t)PS_::ROWS * PS_::PS) * sizeof(double2) +
+    return (2 * (size_t)PS_::WWORDS + 2 * (size_t)PS_::ROWS * PS_::PS) * sizeof(double2) +
            kPairTabBytes;
 }
 

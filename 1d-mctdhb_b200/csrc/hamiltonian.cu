@@ -161,7 +161,8 @@ bool hcp_eligible(int N, int M) { return N >= 2 && M >= 2 && M <= kMaxTemplOrb; 
 
 size_t hcp_scratch_bytes(int N, int M) {
     if (!hcp_eligible(N, M) && !wide_eligible(N, M)) return 0;
-    return (size_t)fock_dimension(N - 2, M) * (size_t)(M * (M + 1) / 2) * sizeof(double2);
+    return (size_t)pair_ld((uint32_t)fock_dimension(N - 2, M)) * (size_t)(M * (M + 1) / 2) *
+           sizeof(double2);
 }
 
 int hcp_prepare(int M) {

@@ -92,7 +92,8 @@ int space_init(SpaceCtx& s, int N, int M) {
     // left still holds every Lanczos workspace a caller may ask for (64
     // vectors and the callers' own), so no call that ran beside the per-row
     // kernel runs out of memory now.
-    const size_t part = dens_partial_elems(s.view);
+    // (the scratch starts on 128 bytes)
+    const size_t part = (dens_partial_elems(s.view) + 7) / 8 * 8;
     bool pair = hcp_eligible(N, M);
     if (wide_eligible(N, M)) {
         size_t free_b = 0, total_b = 0;
@@ -101,10 +102,11 @@ int space_init(SpaceCtx& s, int N, int M) {
     }
     if (pair) pair = hcp_prepare(M) == 0 && (M > kMaxTemplOrb || small_prepare(M) == 0);
     if (pair) {
-        const size_t P = (size_t)M * (M + 1) / 2, W = P * P + 1;
+        const size_t P = (size_t)M * (M + 1) / 2, W = (P * P + 1 + 7) / 8 * 8;
         const size_t bytes = (part + W) * sizeof(double2) + hcp_scratch_bytes(N, M);
         if (cudaMalloc(&s.d_dens_part, bytes) == cudaSuccess) {
             s.view.dim2 = (uint32_t)fock_dimension(N - 2, M);
+            s.view.ldy = pair_ld(s.view.dim2);
             s.view.pair_w = s.d_dens_part + part;
             s.view.pair_y = s.view.pair_w + W;
             return 0;
