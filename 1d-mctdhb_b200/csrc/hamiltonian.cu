@@ -287,7 +287,7 @@ int hc_variant(const SpaceView& sp, const double2* C, double2* HC, const double2
 
 int hc_apply(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,
              const HcEpilogue& ep, cudaStream_t st) {
-    if (sp.pair_y != nullptr && ep.flag == nullptr && ep.prev == nullptr &&
+    if (sp.pair_y != nullptr && ep.flag == nullptr && ep.part == nullptr &&
         small_eligible(sp.N, sp.M, sp.dim2, kSmallHcMacs)) {
         SmallSys s{};
         s.sp = sp;

@@ -8,14 +8,32 @@
 
 namespace mctdhb {
 
-// Optional fused epilogue of the H.C kernel, used by the Lanczos recurrence
+// Optional fused epilogue of the H.C kernels, used by the Lanczos recurrence
 // (multiconfig_lanczos.c:78-82): out = H v - beta * prev.  `flag` != 0 turns
 // the launch into a no-op (a breakdown detected on the device earlier in the
 // same step).
+//
+// The kernels that form H.C in two passes (contraction, gather-back) also take
+// the rest of an iteration's row work in their second pass, where the row is at
+// hand: `scale` (1 / beta) when the product was taken of the vector before its
+// scaling, which then is `out` itself; the scaled vector stored to `v`; and
+// alpha = <v, out> from `part` (a partial per block), added by the last block
+// to finish into *alpha.  For N=30 M=8 that is two passes over 165 MB vectors
+// and four launches less an iteration; on small vectors the launches count.
 struct HcEpilogue {
     const int* flag = nullptr;
     const double2* prev = nullptr;
     const double* beta = nullptr;
+    const double* scale = nullptr;  // H C times *scale; v = out * *scale before out is written
+    const double2* dot = nullptr;   // scale null: the vector of alpha (v takes a copy)
+    double2* v = nullptr;
+    double2* part = nullptr;
+    double2* alpha = nullptr;
+    int* counter = nullptr;  // blocks done, 0 between launches
+    // first iteration: the recurrence's state for `m` vectors is set up with alpha
+    int* init_flags = nullptr;
+    double2 *init_max = nullptr, *init_offd = nullptr;
+    int m = 0;
 };
 
 // Deterministic block reduction of one complex value per thread; thread 0
@@ -39,6 +57,81 @@ __device__ __forceinline__ void block_reduce_store(double2 v, double2* out) {
             s.y += red[i].y;
         }
         out[blockIdx.x] = s;
+    }
+}
+
+// Whether the calling block is the last of the grid to come here; every thread
+// calls it, after the block's global stores.  The last one sees the stores of
+// all and sets the counter back to 0.
+__device__ __forceinline__ bool last_block(int* counter) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+        if (last) *counter = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
+// the sum of n partials by the calling warp: lanes take strided partials in
+// order, then a butterfly; every lane gets it
+__device__ __forceinline__ double2 warp_sum_partials(const double2* part, int n) {
+    double2 s = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int b = threadIdx.x & 31; b < n; b += 32) {
+        const double2 p = __ldcg(part + b);
+        s.x += p.x;
+        s.y += p.y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    return s;
+}
+
+// the epilogue of one row: `h` = (H C)_row; adds the row's term of alpha
+__device__ __forceinline__ void hc_row_epilogue(const HcEpilogue& ep, uint32_t row, double2 h,
+                                                double2* out, double2& alpha) {
+    double2 v = make_double2(0.0, 0.0);
+    if (ep.scale != nullptr) {
+        const double s = *ep.scale;
+        v = out[row];
+        v = make_double2(v.x * s, v.y * s);
+        h = make_double2(h.x * s, h.y * s);
+    } else if (ep.dot != nullptr) {
+        v = ep.dot[row];
+    }
+    if (ep.v != nullptr) ep.v[row] = v;
+    if (ep.prev != nullptr) {
+        const double2 pv = __ldg(ep.prev + row);
+        const double b = *ep.beta;
+        h.x -= b * pv.x;
+        h.y -= b * pv.y;
+    }
+    out[row] = h;
+    alpha.x = fma(v.x, h.x, fma(v.y, h.y, alpha.x));
+    alpha.y = fma(v.x, h.y, fma(-v.y, h.x, alpha.y));
+}
+
+// the sum of alpha over the grid; every thread calls it
+__device__ __forceinline__ void hc_alpha_epilogue(const HcEpilogue& ep, double2 alpha) {
+    if (ep.part == nullptr) return;
+    block_reduce_store(alpha, ep.part);
+    if (!last_block(ep.counter) || threadIdx.x >= 32) return;
+    const double2 s = warp_sum_partials(ep.part, gridDim.x);
+    if (threadIdx.x != 0) return;
+    *ep.alpha = s;
+    if (ep.init_flags != nullptr) {
+        ep.init_flags[0] = 0;
+        ep.init_flags[1] = ep.m;
+        ep.init_flags[2] = 0;
+        *ep.init_max = make_double2(0.0, 0.0);
+        *ep.init_offd = make_double2(0.0, 0.0);
     }
 }
 

@@ -94,8 +94,8 @@ int vec_dot(const double2* a, const double2* b, uint32_t n, double2* part, int g
 template <int NK>
 __global__ void __launch_bounds__(256)
     lz_sub_dots_kernel(int i, int k0, const double2* __restrict__ V, uint32_t n,
-                       double2* __restrict__ out, const double2* __restrict__ scal,
-                       const int* __restrict__ iflag, double2* __restrict__ part) {
+                       double2* __restrict__ out, double2* __restrict__ scal,
+                       int* __restrict__ iflag, double2* __restrict__ part) {
     if (iflag[0]) return;
     const double2 alpha = scal[S_DIAG + i];
     double2 acc[NK];
@@ -114,11 +114,17 @@ __global__ void __launch_bounds__(256)
     }
 #pragma unroll
     for (int k = 0; k < NK; k++) block_reduce_store(acc[k], part + (size_t)k * gridDim.x);
+    // the last block adds the partials, a warp a dot
+    if (!last_block(iflag + 3)) return;
+    for (int k = threadIdx.x >> 5; k < NK; k += 8) {
+        const double2 s = warp_sum_partials(part + (size_t)k * gridDim.x, gridDim.x);
+        if ((threadIdx.x & 31) == 0) scal[S_ORTHO + k0 + k] = s;
+    }
 }
 
 template <int NK>
 static void sub_dots_launch(int nk, int vg, cudaStream_t st, int i, int k0, const double2* V,
-                            uint32_t n, double2* out, const double2* scal, const int* iflag,
+                            uint32_t n, double2* out, double2* scal, int* iflag,
                             double2* part) {
     if (nk == NK)
         lz_sub_dots_kernel<NK><<<vg, 256, 0, st>>>(i, k0, V, n, out, scal, iflag, part);
@@ -126,10 +132,25 @@ static void sub_dots_launch(int nk, int vg, cudaStream_t st, int i, int k0, cons
         sub_dots_launch<NK - 1>(nk, vg, st, i, k0, V, n, out, scal, iflag, part);
 }
 
-// out -= sum_{k<=i} o_k v_k; partial |out|^2
+// b_i = sqrt(norm2); breakdown test; 1/b_i
+__device__ __forceinline__ void lz_set_beta(int i, double norm2, double2* scal, int* iflag) {
+    const double beta = sqrt(norm2);
+    scal[S_OFFD + i] = make_double2(beta, 0.0);
+    double mx = scal[S_MISC + 0].x;
+    if (mx < beta) mx = beta;
+    scal[S_MISC + 0].x = mx;
+    if (beta == 0.0 || beta / mx < 1e-14) {
+        iflag[0] = 1;
+        iflag[1] = i + 1;
+        return;
+    }
+    scal[S_MISC + 1] = make_double2(1.0 / beta, 0.0);
+}
+
+// out -= sum_{k<=i} o_k v_k; |out|^2 by the last block, and beta_i from it
 __global__ void __launch_bounds__(256)
     lz_orth_kernel(int i, const double2* __restrict__ V, uint32_t n, double2* __restrict__ out,
-                   const double2* __restrict__ scal, const int* __restrict__ iflag,
+                   double2* __restrict__ scal, int* __restrict__ iflag,
                    double2* __restrict__ part) {
     if (iflag[0]) return;
     double acc = 0.0;
@@ -144,32 +165,9 @@ __global__ void __launch_bounds__(256)
         acc += o.x * o.x + o.y * o.y;
     }
     block_reduce_store(make_double2(acc, 0.0), part);
-}
-
-// b_i = sqrt(sum part); breakdown test; 1/b_i
-__global__ void lz_norm_kernel(int i, const double2* __restrict__ part, int np,
-                               double2* __restrict__ scal, int* __restrict__ iflag) {
-    __shared__ double sh[256];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < np; b += blockDim.x) s += part[b].x;
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x != 0 || iflag[0]) return;
-    const double beta = sqrt(sh[0]);
-    scal[S_OFFD + i] = make_double2(beta, 0.0);
-    double mx = scal[S_MISC + 0].x;
-    if (mx < beta) mx = beta;
-    scal[S_MISC + 0].x = mx;
-    if (beta == 0.0 || beta / mx < 1e-14) {
-        iflag[0] = 1;
-        iflag[1] = i + 1;
-        return;
-    }
-    scal[S_MISC + 1] = make_double2(1.0 / beta, 0.0);
+    if (!last_block(iflag + 3) || threadIdx.x >= 32) return;
+    const double2 s = warp_sum_partials(part, gridDim.x);
+    if (threadIdx.x == 0) lz_set_beta(i, s.x, scal, iflag);
 }
 
 __global__ void lz_scale_kernel(int i, const double2* __restrict__ out, double2* __restrict__ V,
@@ -257,16 +255,25 @@ __global__ void __launch_bounds__(32)
     }
 }
 
-// C = sum_j V_j y_j
-__global__ void lz_combine_kernel(const double2* __restrict__ V, uint32_t n,
-                                  const double2* __restrict__ scal, const int* __restrict__ iflag,
-                                  double2* __restrict__ C) {
+// C = sum_j V_j y_j; norm: |C|^2 too, by the last block, for a step that
+// renormalises
+__global__ void __launch_bounds__(256)
+    lz_combine_kernel(const double2* __restrict__ V, uint32_t n, double2* __restrict__ scal,
+                      int* __restrict__ iflag, double2* __restrict__ C, int norm,
+                      double2* __restrict__ part) {
     const int it = iflag[1];
+    double acc = 0.0;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         double2 s = make_double2(0.0, 0.0);
         for (int j = 0; j < it; j++) s = cfma(V[(size_t)j * n + r], scal[S_Y + j], s);
         C[r] = s;
+        acc += s.x * s.x + s.y * s.y;
     }
+    if (!norm) return;
+    block_reduce_store(make_double2(acc, 0.0), part);
+    if (!last_block(iflag + 3) || threadIdx.x >= 32) return;
+    const double2 s = warp_sum_partials(part, gridDim.x);
+    if (threadIdx.x == 0) scal[S_MISC + 3] = s;
 }
 
 __global__ void norm2_kernel(const double2* __restrict__ a, uint32_t n, double2* __restrict__ part) {
@@ -300,6 +307,7 @@ int lanczos_alloc(LanczosWork& w, const SpaceCtx& s, int mmax) {
     MCTDHB_CUDA_TRY(cudaMalloc(&w.scal, S_TOTAL * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMemset(w.scal, 0, S_TOTAL * sizeof(double2)));
     MCTDHB_CUDA_TRY(cudaMalloc(&w.iflag, 4 * sizeof(int)));
+    MCTDHB_CUDA_TRY(cudaMemset(w.iflag, 0, 4 * sizeof(int)));  // [3]: blocks done (last_block)
     return 0;
 }
 
@@ -315,42 +323,70 @@ void lanczos_free(LanczosWork& w) {
 // shared memory of lz_small_kernel: the eigenvectors and the exponentials
 constexpr int kSmallSmem = kSlots * kSlots * (int)sizeof(double) + kSlots * (int)sizeof(double2);
 
+// The recurrence from the vector C (stored to w.V[0] unless it is w.V).  Where
+// H.C runs in two passes an iteration is four launches: contraction of the
+// unscaled vector, gather-back with the scaling, the stored v_i and alpha_i,
+// the dots, the subtraction with beta_i.  The per-row H.C gathers its input in
+// the pass that writes its output, so there the vector is scaled first and
+// alpha taken after.
+static int lanczos_from(const SpaceCtx& s, LanczosWork& w, const double2* C, int m,
+                        cudaStream_t st) {
+    const uint32_t n = s.dim;
+    const int vg = w.vec_grid;
+    const bool passes = s.view.pair_y != nullptr;
+    if (!passes && C != w.V)
+        MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, C, (size_t)n * sizeof(double2),
+                                        cudaMemcpyDeviceToDevice, st));
+    if (!passes) lz_init_kernel<<<1, 32, 0, st>>>(w.scal, w.iflag, m);
+    for (int i = 0; i < m; i++) {
+        double2* v = w.V + (size_t)i * n;
+        HcEpilogue ep;
+        if (i > 0 || !passes) ep.flag = w.iflag;
+        if (i > 0) {
+            ep.prev = v - n;
+            ep.beta = &(w.scal + S_OFFD + i - 1)->x;
+        }
+        if (passes) {
+            ep.part = w.part;
+            ep.alpha = w.scal + S_DIAG + i;
+            ep.counter = w.iflag + 3;
+            if (i == 0) {
+                ep.dot = C;
+                ep.v = C != w.V ? v : nullptr;
+                ep.init_flags = w.iflag;
+                ep.init_max = w.scal + S_MISC;
+                ep.init_offd = w.scal + S_OFFD + m - 1;
+                ep.m = m;
+            } else {
+                ep.scale = &(w.scal + S_MISC + 1)->x;
+                ep.v = v;
+            }
+            if (hc_apply(s.view, i == 0 ? C : w.out, w.out, s.d_tab, ep, st)) return -1;
+        } else {
+            if (i > 0)
+                lz_scale_kernel<<<vg, 256, 0, st>>>(i - 1, w.out, w.V, n, w.scal, w.iflag);
+            if (hc_apply(s.view, v, w.out, s.d_tab, ep, st)) return -1;
+            // after a breakdown the value is never read (iterations < i + 1)
+            if (vec_dot(v, w.out, n, w.part, vg, w.scal + S_DIAG + i, st)) return -1;
+        }
+        if (i == m - 1) break;
+        for (int k0 = 0; k0 <= i; k0 += kDotChunk) {
+            const int k1 = std::min(i, k0 + kDotChunk - 1);
+            sub_dots_launch<kDotChunk>(k1 - k0 + 1, vg, st, i, k0, w.V, n, w.out, w.scal,
+                                       w.iflag, w.part);
+        }
+        lz_orth_kernel<<<vg, 256, 0, st>>>(i, w.V, n, w.out, w.scal, w.iflag, w.part);
+        MCTDHB_CUDA_TRY(cudaGetLastError());
+    }
+    return 0;
+}
+
 int lanczos_run(const SpaceCtx& s, LanczosWork& w, int m, cudaStream_t st) {
     if (m < 1 || m > w.mmax) {
         set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
         return -1;
     }
-    const uint32_t n = s.dim;
-    const int vg = w.vec_grid;
-    lz_init_kernel<<<1, 32, 0, st>>>(w.scal, w.iflag, m);
-    HcEpilogue ep;
-    ep.flag = w.iflag;
-    if (hc_apply(s.view, w.V, w.out, s.d_tab, ep, st)) return -1;
-    // a_0 = <v0, H v0>: fixed-geometry reduction, independent of the H.C
-    // launch variant
-    if (vec_dot(w.V, w.out, n, w.part, vg, w.scal + S_DIAG, st)) return -1;
-    for (int i = 0; i < m - 1; i++) {
-        for (int k0 = 0; k0 <= i; k0 += kDotChunk) {
-            const int k1 = std::min(i, k0 + kDotChunk - 1);
-            sub_dots_launch<kDotChunk>(k1 - k0 + 1, vg, st, i, k0, w.V, n, w.out, w.scal,
-                                       w.iflag, w.part);
-            MCTDHB_CUDA_TRY(cudaGetLastError());
-            if (reduce_rows(w.part, k1 - k0 + 1, vg, w.scal + S_ORTHO + k0, st)) return -1;
-        }
-        lz_orth_kernel<<<vg, 256, 0, st>>>(i, w.V, n, w.out, w.scal, w.iflag, w.part);
-        lz_norm_kernel<<<1, 256, 0, st>>>(i, w.part, vg, w.scal, w.iflag);
-        lz_scale_kernel<<<vg, 256, 0, st>>>(i, w.out, w.V, n, w.scal, w.iflag);
-        MCTDHB_CUDA_TRY(cudaGetLastError());
-        HcEpilogue e2;
-        e2.flag = w.iflag;
-        e2.prev = w.V + (size_t)i * n;
-        e2.beta = &(w.scal + S_OFFD + i)->x;
-        if (hc_apply(s.view, w.V + (size_t)(i + 1) * n, w.out, s.d_tab, e2, st)) return -1;
-        // a_{i+1}; after a breakdown the value is never read (iterations < i+2)
-        if (vec_dot(w.V + (size_t)(i + 1) * n, w.out, n, w.part, vg, w.scal + S_DIAG + i + 1, st))
-            return -1;
-    }
-    return 0;
+    return lanczos_from(s, w, w.V, m, st);
 }
 
 // diag[0..it-1] and offd[0..min(it, m-1)-1] as the reference leaves them
@@ -397,16 +433,16 @@ int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 pro
                 return -1;
         return small_launch(y, kSmallCombine, 0, st);
     }
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, d_C, (size_t)n * sizeof(double2),
-                                    cudaMemcpyDeviceToDevice, st));
-    if (lanczos_run(s, w, m, st)) return -1;
+    if (m < 1 || m > w.mmax) {
+        set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
+        return -1;
+    }
+    if (lanczos_from(s, w, d_C, m, st)) return -1;
     lz_small_kernel<<<1, 32, kSmallSmem, st>>>(imagtime ? 2 : 0, prop_dt, w.scal, w.iflag,
                                                nullptr);
-    lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C);
+    lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C, imagtime, w.part);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     if (imagtime) {
-        norm2_kernel<<<w.vec_grid, 256, 0, st>>>(d_C, n, w.part);
-        if (reduce_rows(w.part, 1, w.vec_grid, w.scal + S_MISC + 3, st)) return -1;
         renorm_kernel<<<w.vec_grid, 256, 0, st>>>(d_C, n, w.scal + S_MISC + 3);
         MCTDHB_CUDA_TRY(cudaGetLastError());
     }
@@ -511,12 +547,14 @@ int sil_norm2(const LanczosWork& w, double* out) {
 int lowest_state(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double* d_energy,
                  cudaStream_t st) {
     const uint32_t n = s.dim;
-    MCTDHB_CUDA_TRY(cudaMemcpyAsync(w.V, d_C, (size_t)n * sizeof(double2),
-                                    cudaMemcpyDeviceToDevice, st));
-    if (lanczos_run(s, w, m, st)) return -1;
+    if (m < 1 || m > w.mmax) {
+        set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
+        return -1;
+    }
+    if (lanczos_from(s, w, d_C, m, st)) return -1;
     lz_small_kernel<<<1, 32, kSmallSmem, st>>>(1, make_double2(0.0, 0.0), w.scal, w.iflag,
                                                d_energy);
-    lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C);
+    lz_combine_kernel<<<w.vec_grid, 256, 0, st>>>(w.V, n, w.scal, w.iflag, d_C, 0, w.part);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;
 }

@@ -669,22 +669,22 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
 }
 
 // (HC)_i gathered back from Y, then the Lanczos epilogue
-template <int M>
-__global__ void __launch_bounds__(256)
+template <int M, bool LZ>
+__global__ void __launch_bounds__(256, M < 8 ? 5 : 4)
     hcp_g_kernel(SpaceView sp, const double2* __restrict__ Y, double2* __restrict__ HC,
                  HcEpilogue ep) {
     if (ep.flag != nullptr && *ep.flag != 0) return;
+    double2 alpha = make_double2(0.0, 0.0);
+#pragma unroll 1
     for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < sp.dim;
          row += gridDim.x * blockDim.x) {
-        double2 acc = pair_gather_back<M>(sp, Y, row);
-        if (ep.prev != nullptr) {
-            const double2 pv = __ldg(ep.prev + row);
-            const double b = *ep.beta;
-            acc.x -= b * pv.x;
-            acc.y -= b * pv.y;
-        }
-        HC[row] = acc;
+        const double2 h = pair_gather_back<M>(sp, Y, row);
+        if constexpr (LZ)
+            hc_row_epilogue(ep, row, h, HC, alpha);
+        else
+            HC[row] = h;
     }
+    if constexpr (LZ) hc_alpha_epilogue(ep, alpha);
 }
 
 template <int M, int V>
@@ -728,7 +728,10 @@ int hcp_launch_v(const SpaceView& sp, const double2* C, double2* HC, const HcEpi
             const uint32_t need = (sp.dim + 255) / 256;
             const int gg =
                 (int)std::max<uint32_t>(1u, std::min<uint32_t>(need, (uint32_t)num_sms() * 8));
-            hcp_g_kernel<M><<<gg, 256, 0, st>>>(sp, sp.pair_y, HC, ep);
+            if (ep.part != nullptr)
+                hcp_g_kernel<M, true><<<gg, 256, 0, st>>>(sp, sp.pair_y, HC, ep);
+            else
+                hcp_g_kernel<M, false><<<gg, 256, 0, st>>>(sp, sp.pair_y, HC, ep);
             MCTDHB_CUDA_TRY(cudaGetLastError());
         }
         return 0;

@@ -200,63 +200,61 @@ __global__ void __launch_bounds__(kWideThreads)
 // (HC)_i gathered back from Y: 64 rows a block, four threads a row (each a
 // quarter of the pairs, added in order), then the Lanczos epilogue
 __global__ void __launch_bounds__(kWideThreads)
-    wide_g_kernel(SpaceView sp, const double2* __restrict__ Y, double2* __restrict__ HC,
-                  HcEpilogue ep) {
+    wide_g_kernel(SpaceView sp, const double2* __restrict__ Y, double2* HC, HcEpilogue ep) {
     extern __shared__ double2 smem[];
     if (ep.flag != nullptr && *ep.flag != 0) return;
     const int M = sp.M, N = sp.N, P = wide_pairs(M), t = threadIdx.x;
     double2* part = smem;  // 4 x kWideGRows
     const WideRows rows = wide_rows_at(part + 4 * kWideGRows, M, kWideGRows);
-    const uint32_t row0 = blockIdx.x * kWideGRows;
     const int r = t % kWideGRows, sub = t / kWideGRows;
-    const uint32_t row = min(row0 + r, sp.dim - 1u);
-    if (sub == 0) {
-        int L[kMaxOrb];
-        wide_unrank(sp, N, sp.dim, row, rows.n + r, kWideGRows, L);
-        // suffix sums of T_y(L_y) - T_y(L_y - d); an L_y below d only occurs
-        // for y below the orbitals of a pair that cannot be removed
-        uint32_t v1 = 0, v2 = 0;
-        rows.U1[(M - 1) * kWideGRows + r] = 0u;
-        rows.U2[(M - 1) * kWideGRows + r] = 0u;
-        for (int x = M - 2; x >= 0; x--) {
-            const uint32_t* Tx = sp.T + x * (N + 1);
-            const uint32_t t0 = __ldg(Tx + L[x]);
-            v1 += t0 - __ldg(Tx + max(L[x] - 1, 0));
-            v2 += t0 - __ldg(Tx + max(L[x] - 2, 0));
-            rows.U1[x * kWideGRows + r] = v1;
-            rows.U2[x * kWideGRows + r] = v2;
+    double2 alpha = make_double2(0.0, 0.0);
+    for (uint32_t row0 = blockIdx.x * kWideGRows; row0 < sp.dim; row0 += gridDim.x * kWideGRows) {
+        const uint32_t row = min(row0 + r, sp.dim - 1u);
+        if (sub == 0) {
+            int L[kMaxOrb];
+            wide_unrank(sp, N, sp.dim, row, rows.n + r, kWideGRows, L);
+            // suffix sums of T_y(L_y) - T_y(L_y - d); an L_y below d only occurs
+            // for y below the orbitals of a pair that cannot be removed
+            uint32_t v1 = 0, v2 = 0;
+            rows.U1[(M - 1) * kWideGRows + r] = 0u;
+            rows.U2[(M - 1) * kWideGRows + r] = 0u;
+            for (int x = M - 2; x >= 0; x--) {
+                const uint32_t* Tx = sp.T + x * (N + 1);
+                const uint32_t t0 = __ldg(Tx + L[x]);
+                v1 += t0 - __ldg(Tx + max(L[x] - 1, 0));
+                v2 += t0 - __ldg(Tx + max(L[x] - 2, 0));
+                rows.U1[x * kWideGRows + r] = v1;
+                rows.U2[x * kWideGRows + r] = v2;
+            }
         }
-    }
-    __syncthreads();
-    const uint32_t D2 = sp.dim2, base = D2 - sp.dim + row;
-    double2 acc = make_double2(0.0, 0.0);
-    const int per = (P + 3) / 4, p0 = sub * per, p1 = min(p0 + per, P);
-    unsigned short ks = wide_pair(M, min(p0, P - 1));
-    int k = ks >> 8, s = ks & 255;
-    for (int p = p0; p < p1; p++) {
-        const int nk = rows.n[k * kWideGRows + r], ns = rows.n[s * kWideGRows + r] - (k == s);
-        if (nk >= 1 && ns >= 1) {
-            const double f = __ldg(sp.sq + nk) * __ldg(sp.sq + ns);
-            const uint32_t m = base +
-                               (rows.U1[k * kWideGRows + r] - rows.U1[s * kWideGRows + r]) +
-                               rows.U2[s * kWideGRows + r];
-            const double2 y = __ldg(Y + (size_t)p * D2 + m);
-            acc.x = fma(f, y.x, acc.x);
-            acc.y = fma(f, y.y, acc.y);
+        __syncthreads();
+        const uint32_t D2 = sp.dim2, base = D2 - sp.dim + row;
+        double2 acc = make_double2(0.0, 0.0);
+        const int per = (P + 3) / 4, p0 = sub * per, p1 = min(p0 + per, P);
+        unsigned short ks = wide_pair(M, min(p0, P - 1));
+        int k = ks >> 8, s = ks & 255;
+        for (int p = p0; p < p1; p++) {
+            const int nk = rows.n[k * kWideGRows + r], ns = rows.n[s * kWideGRows + r] - (k == s);
+            if (nk >= 1 && ns >= 1) {
+                const double f = __ldg(sp.sq + nk) * __ldg(sp.sq + ns);
+                const uint32_t m = base +
+                                   (rows.U1[k * kWideGRows + r] - rows.U1[s * kWideGRows + r]) +
+                                   rows.U2[s * kWideGRows + r];
+                const double2 y = __ldg(Y + (size_t)p * D2 + m);
+                acc.x = fma(f, y.x, acc.x);
+                acc.y = fma(f, y.y, acc.y);
+            }
+            if (++s == M) s = ++k;
         }
-        if (++s == M) s = ++k;
+        part[sub * kWideGRows + r] = acc;
+        __syncthreads();
+        if (sub == 0 && row0 + r < sp.dim) {
+            for (int u = 1; u < 4; u++) acc = cadd(acc, part[u * kWideGRows + r]);
+            hc_row_epilogue(ep, row, acc, HC, alpha);
+        }
+        __syncthreads();
     }
-    part[sub * kWideGRows + r] = acc;
-    __syncthreads();
-    if (sub != 0 || row0 + r >= sp.dim) return;
-    for (int u = 1; u < 4; u++) acc = cadd(acc, part[u * kWideGRows + r]);
-    if (ep.prev != nullptr) {
-        const double2 pv = __ldg(ep.prev + row);
-        const double b = *ep.beta;
-        acc.x -= b * pv.x;
-        acc.y -= b * pv.y;
-    }
-    HC[row] = acc;
+    hc_alpha_epilogue(ep, alpha);
 }
 
 // One block's share of a 64 x 64 super-tile (si <= sj) of the Gram matrix:
@@ -404,8 +402,9 @@ int wide_hc(const SpaceView& sp, const double2* C, double2* HC, const HcEpilogue
         wide_y_kernel<2><<<gy, kWideThreads, sm, st>>>(sp, C, sp.pair_w, sp.pair_y, ep);
     else
         wide_y_kernel<1><<<gy, kWideThreads, sm, st>>>(sp, C, sp.pair_w, sp.pair_y, ep);
-    wide_g_kernel<<<(sp.dim + kWideGRows - 1) / kWideGRows, kWideThreads, wide_g_smem(sp.M), st>>>(
-        sp, sp.pair_y, HC, ep);
+    const int gg = (int)std::min<uint32_t>((sp.dim + kWideGRows - 1) / kWideGRows,
+                                           (uint32_t)num_sms() * 8);
+    wide_g_kernel<<<gg, kWideThreads, wide_g_smem(sp.M), st>>>(sp, sp.pair_y, HC, ep);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
