@@ -187,7 +187,7 @@ struct mctdhb_batch_s {
     int* h_pro = nullptr;
     BatchTile* h_pro_g = nullptr;
     int* h_flags = nullptr;
-    double2* h_scal = nullptr;
+    double2* h_scal = nullptr;  // of all slots, then kFetchWords of mctdhb_batch_fetch
     unsigned present_mask = 0;  // orbital counts on the general path
     unsigned small_mask = 0;    // orbital counts of the small slots
     bool lists_dirty = true;
@@ -593,6 +593,25 @@ uint32_t binom_u32(int n, int k) {
 
 }  // namespace
 
+// whether mctdhb_batch_fetch reads the arrays through the pinned words: they
+// fit, and no destination is device memory (which the copies refuse)
+static bool fetch_packed(const BatchSlot& d, void* orbitals, void* coef, void* rho1, void* rho2) {
+    const size_t M2 = (size_t)d.M * d.M;
+    const size_t words = kFetchHead + (orbitals ? (size_t)d.M * d.G : 0) + (coef ? d.nc : 0) +
+                         (rho1 ? M2 : 0) + (rho2 ? M2 * M2 : 0);
+    if (words > kFetchWords) return false;
+    for (const void* p : {orbitals, coef, rho1, rho2}) {
+        cudaPointerAttributes at;
+        if (p == nullptr) continue;
+        if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type == cudaMemoryTypeDevice) return false;
+    }
+    return true;
+}
+
 extern "C" {
 
 size_t mctdhb_batch_job_bytes(const mctdhb_job* job, int lanczos_iter) {
@@ -662,7 +681,8 @@ int mctdhb_batch_create(int max_slots, size_t arena_bytes, int lanczos_iter, mct
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
     if (bad ||
         cudaMallocHost(&b->h_flags, (size_t)max_slots * BF_TOTAL * sizeof(int)) ||
-        cudaMallocHost(&b->h_scal, (size_t)max_slots * BS_TOTAL * sizeof(double2)) ||
+        cudaMallocHost(&b->h_scal,
+                       ((size_t)max_slots * BS_TOTAL + kFetchWords) * sizeof(double2)) ||
         cudaStreamCreateWithPriority(&b->st, cudaStreamNonBlocking, prio_hi) ||
         cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) ||
         cudaEventCreateWithFlags(&b->ev_fork_small, cudaEventDisableTiming)) {
@@ -990,6 +1010,28 @@ int mctdhb_batch_fetch(mctdhb_batch b, int slot, void* orbitals, void* coef, voi
     const BatchSlot& d = h.d;
     cudaStream_t st = b->st;
     const size_t n = (size_t)d.M * d.G, M2 = (size_t)d.M * d.M;
+    if (fetch_packed(d, orbitals, coef, rho1, rho2)) {
+        const BatchFetch f = {{d.orb, d.V, d.rho1, d.rho2},
+                              {orbitals ? (uint32_t)n : 0u, coef ? d.nc : 0u,
+                               rho1 ? (uint32_t)M2 : 0u, rho2 ? (uint32_t)(M2 * M2) : 0u},
+                              d.scal,
+                              d.flags};
+        const uint32_t most = std::max(std::max(f.n[0], f.n[1]), std::max(f.n[2], f.n[3]));
+        double2* stage = b->h_scal + (size_t)b->max_slots * BS_TOTAL;
+        bt_fetch_kernel<<<most / kBatchVecThreads + 1, kBatchVecThreads, 0, st>>>(f, stage);
+        MCTDHB_CUDA_TRY(cudaGetLastError());
+        MCTDHB_CUDA_TRY(cudaStreamSynchronize(st));
+        void* to[4] = {orbitals, coef, rho1, rho2};
+        const double2* from = stage + kFetchHead;
+        for (int a = 0; a < 4; a++) {
+            if (f.n[a] > 0) std::memcpy(to[a], from, f.n[a] * sizeof(double2));
+            from += f.n[a];
+        }
+        if (energy) *energy = stage[0].x;
+        if (steps) *steps = (uint32_t)stage[1].x;
+        if (converged) *converged = (int)stage[1].y;
+        return 0;
+    }
     int fl[BF_TOTAL];
     double2 sc[BS_TOTAL];
     if (orbitals)

@@ -148,4 +148,20 @@ int gram_batch_launch(const BatchSlot* slots, const BatchTile* g2, const int* cn
 template <int M>
 int batch_prepare();
 
+// A slot's results read to the host (mctdhb_batch_fetch): one launch writes the
+// energy, the counters and the wanted arrays (n[a] = 0: not wanted) behind one
+// another into pinned host memory, from where the host hands them out.  Six
+// copies to pageable memory, each with its own wait, took 31 us for a small
+// job; this takes 10 us (32 jobs of N=2..10, 4 steps and a fetch each: 2,759 to
+// 2,082 us).  Above kFetchWords the copies stay with the copy engine.
+constexpr int kFetchHead = 2;
+constexpr size_t kFetchWords = 16384;  // 256 KB
+struct BatchFetch {
+    const double2* src[4];
+    uint32_t n[4];
+    const double2* scal;
+    const int* flags;
+};
+__global__ void bt_fetch_kernel(BatchFetch f, double2* out);
+
 }  // namespace mctdhb

@@ -428,6 +428,21 @@ __global__ void __launch_bounds__(kBatchVecThreads)
 
 #undef BT_SLOT
 
+__global__ void __launch_bounds__(kBatchVecThreads)
+    bt_fetch_kernel(BatchFetch f, double2* __restrict__ out) {
+    const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    if (t0 == 0) {
+        out[0] = make_double2(f.scal[BS_MISC + 3].x, 0.0);
+        out[1] = make_double2((double)f.flags[BF_STEPS], (double)f.flags[BF_CONV]);
+    }
+    double2* o = out + kFetchHead;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        for (uint32_t i = t0; i < f.n[a]; i += nt) o[i] = f.src[a][i];
+        o += f.n[a];
+    }
+}
+
 void bt_subdots(int i, int grid, cudaStream_t st, const BatchSlot* slots, const BatchTile* tiles,
                 const int* ntiles) {
     subdots_launch<kBatchMaxLz - 2>(i, grid, st, slots, tiles, ntiles);
