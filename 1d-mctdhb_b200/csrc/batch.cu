@@ -51,9 +51,9 @@ size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 struct JobLayout {
     uint32_t nc = 0, D1 = 0, D2 = 0;
     int vtiles = 0, ytiles = 0, gs[3] = {0, 0, 0}, gk[3] = {0, 0, 0};
-    size_t o_orb, o_stage, o_H, o_pot, o_w, o_Q, o_hob, o_hint, o_pw, o_lint, o_rho1, o_rho2,
+    size_t o_orb, o_stage, o_H, o_pot, o_w, o_hob, o_hint, o_pw, o_lint, o_rho1, o_rho2,
         o_rinv,
-        o_work, o_T, o_sq, o_g, o_V, o_out, o_part, o_py, o_gpart, o_half, o_B, total;
+        o_T, o_sq, o_g, o_V, o_out, o_part, o_py, o_gpart, o_half, o_B, total;
 };
 
 // der: 0 / 302 finite differences, 300 DVR, 301 spectral (periodic only);
@@ -111,7 +111,6 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     L.o_H = take(n * z);
     L.o_pot = take((size_t)G * sizeof(double));
     L.o_w = take((size_t)G * sizeof(double));
-    L.o_Q = take(M4 * z);
     L.o_hob = take(M2 * z);
     L.o_hint = take(M4 * z);
     L.o_pw = take((P * P + 1) * z);  // + the real-W flag (pairhc_tmpl.cuh)
@@ -119,7 +118,6 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     L.o_rho1 = take(M2 * z);
     L.o_rho2 = take(M4 * z);
     L.o_rinv = take(M2 * z);
-    L.o_work = take((3 * M2 + M + 2) * z);
     L.o_T = take((size_t)(M - 1) * (N + 1) * sizeof(uint32_t));
     L.o_sq = take((size_t)(N + 3) * sizeof(double));
     L.o_g = take(sizeof(double));
@@ -349,7 +347,7 @@ int hc_group(int M, const BatchSlot* slots, const BatchTile* hy, const BatchTile
     return 0;
 }
 
-// the batched contraction variants (0 and 2, pairhc_tmpl.cuh)
+// the batched contraction variants (0, 2 and 3, pairhc_tmpl.cuh)
 bool batch_v_ok(int M, int v) {
     return M >= kBatchMinOrb && M <= kBatchMaxOrb &&
            (v == 3 || ((v == 0 || v == 2) && pair_variant_ok(M, v)));
@@ -842,13 +840,11 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     d.orb = (double2*)P(L.o_orb);
     d.stage = (double2*)P(L.o_stage);
     d.H = (double2*)P(L.o_H);
-    d.Q = (double2*)P(L.o_Q);
     d.hob = (double2*)P(L.o_hob);
     d.hint = (double2*)P(L.o_hint);
     d.rho1 = (double2*)P(L.o_rho1);
     d.rho2 = (double2*)P(L.o_rho2);
     d.rinv = (double2*)P(L.o_rinv);
-    d.work = (double2*)P(L.o_work);
     d.V = (double2*)P(L.o_V);
     d.out = (double2*)P(L.o_out);
     d.part = (double2*)P(L.o_part);

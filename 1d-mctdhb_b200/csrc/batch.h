@@ -75,7 +75,7 @@ struct BatchSlot {
     OrbView ov;   // grid, equation coefficients, Simpson weights, trap
     SpaceView sp; // with the pair matrix sp.pair_w and its scratch sp.pair_y
     const double* g;     // contact interaction (device scalar)
-    double2 *orb, *stage, *H, *Q, *hob, *hint, *rho1, *rho2, *rinv, *work;
+    double2 *orb, *stage, *H, *hob, *hint, *rho1, *rho2, *rinv;
     double2* orb_next;   // a copy of the orbitals after the Runge-Kutta step (null: none)
     double2 *V;          // lz x nc Krylov vectors; V[0] holds the coefficients
     // split step (split: 1): the half-step operator (orbital.h,
@@ -134,7 +134,7 @@ __host__ __device__ constexpr int batch_pair_rows(int M) {
 //                      slot of orbital count M: pair contraction (parts & 1),
 //                      gather-back (parts & 2); iter = kBatchMonIter: out =
 //                      H V[0] of the slots whose eigen residual is due;
-//                      variant: the contraction's launch variant (0 or 2,
+//                      variant: the contraction's launch variant (0, 2 or 3,
 //                      pairhc_tmpl.cuh)
 //   gram_batch_launch  rho2 of V[0] of the slots of orbital count M (`list` /
 //                      `nlist`: the slots; rho1 follows in bt_tail_kernel)

@@ -31,6 +31,11 @@
 // imaginary tile for both sides: 5 loads feed 45 products of 16 cycles.
 // FP64 FMA register tiles, which read 8 operands for 16 complex FMAs, ran at
 // 0.41 of the FP64 peak by the algorithmic count.
+// What bounds it now: at N=60 M=6 the products alone take 611 us (512 us at the
+// FP64 MMA peak) and the gathers alone, L2-bound, 365 us; together 770 us (903
+// with the FMA tiles).  Eight producer and four consumer warps a block around a
+// ring of 32-row chunks gave 786 us, with one block an SM 765 us: the gathers
+// need 16 warps an SM, which leaves the products too few.
 //
 // Work split.  A block takes tiles of 128 or 256 rows: every thread unranks its
 // row and gathers its share of the row's A values into shared memory (gram.h
@@ -69,7 +74,7 @@ inline constexpr PairList<M> kPairs{};
 // of a space of N >= Np bosons (row stride N + 1): occupations n[] and the
 // suffix sums U1, U2 of the rank offsets of adding one / two bosons.
 // GEN: generic table loads (the table may be staged in shared memory).
-template <int M, int R, bool GEN = false>
+template <int M, bool GEN = false>
 __device__ __forceinline__ void gram_unrank(const uint32_t* __restrict__ T, int N, int Np,
                                             uint32_t Dp, uint32_t row, int (&n)[M],
                                             uint32_t (&U1)[M], uint32_t (&U2)[M]) {
@@ -93,7 +98,7 @@ __device__ __forceinline__ void gram_unrank(const uint32_t* __restrict__ T, int 
         const uint32_t* Tx = T + x * (N + 1);
         const uint32_t t0 = tab_ld<GEN>(Tx + L[x]);
         U1[x] = U1[x + 1] + (tab_ld<GEN>(Tx + L[x] + 1) - t0);
-        if constexpr (R == 2) U2[x] = U2[x + 1] + (tab_ld<GEN>(Tx + L[x] + 2) - t0);
+        U2[x] = U2[x + 1] + (tab_ld<GEN>(Tx + L[x] + 2) - t0);
     }
 }
 
@@ -147,7 +152,7 @@ __device__ __forceinline__ void gram_gather(const SpaceView& sp, uint32_t Dp,
     const uint32_t rr = live ? row : Dp - 1u;
     int n[M];
     uint32_t U1[M], U2[M];
-    gram_unrank<M, 2>(sp.T, N, N - 2, Dp, rr, n, U1, U2);
+    gram_unrank<M>(sp.T, N, N - 2, Dp, rr, n, U1, U2);
     const uint32_t j0 = sp.dim - Dp + rr;
     // sqrt(n_x + 1), sqrt(n_x + 2) once per orbital; rows past the end are
     // zero through them

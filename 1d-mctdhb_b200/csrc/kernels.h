@@ -18,8 +18,10 @@ namespace mctdhb {
 // hand: `scale` (1 / beta) when the product was taken of the vector before its
 // scaling, which then is `out` itself; the scaled vector stored to `v`; and
 // alpha = <v, out> from `part` (a partial per block), added by the last block
-// to finish into *alpha.  For N=30 M=8 that is two passes over 165 MB vectors
-// and four launches less an iteration; on small vectors the launches count.
+// to finish into *alpha.  There `prev` is looked at only with `part`.  At N=30
+// M=8 this takes two passes over 165 MB vectors and four launches out of an
+// iteration and costs the gather-back 150 us (800 to 945 us): even.  It is for
+// the small vectors, where launches count: N=20 M=6 drop-in calls 748 to 711 us.
 struct HcEpilogue {
     const int* flag = nullptr;
     const double2* prev = nullptr;

@@ -250,7 +250,7 @@ __device__ __forceinline__ void pair_gather_row(const SpaceView& sp,
     row = min(row, D2 - 1u);
     int n[M];
     uint32_t U1[M], U2[M];
-    gram_unrank<M, 2, true>(sp.T, sp.N, sp.N - 2, D2, row, n, U1, U2);
+    gram_unrank<M, true>(sp.T, sp.N, sp.N - 2, D2, row, n, U1, U2);
     const uint32_t j0 = sp.dim - D2 + row;
     // sqrt(n_x + 1), sqrt(n_x + 2) once per orbital
     double s1[M], s2[M];

@@ -74,7 +74,7 @@ struct SmallRun {
     __device__ __forceinline__ void amplitudes(uint32_t row, const double2* C, double2 (&a)[P]) {
         int n[M];
         uint32_t U1[M], U2[M];
-        gram_unrank<M, 2, true>(sp.T, sp.N, sp.N - 2, sp.dim2, row, n, U1, U2);
+        gram_unrank<M, true>(sp.T, sp.N, sp.N - 2, sp.dim2, row, n, U1, U2);
         const uint32_t j0 = sp.dim - sp.dim2 + row;
         double s1[M], s2[M];
 #pragma unroll

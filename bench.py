@@ -973,7 +973,7 @@ def run_single(mb, torch, name, steps, warmup):
                    "gather_model_note": "32 nc + 16 G bytes (one 16-byte gather per distinct "
                                         "coupling) / time: the rate a gather-per-coupling H.C "
                                         "would need to match this launch"},
-            "density": {"kernels": f"gram_kernel<{M},2> + finalize + rho1 from rho2",
+            "density": {"kernels": f"gram_kernel<{M}> + finalize + rho1 from rho2",
                         "ms_per_launch": t_dn * 1e3, "gram_flops": f_dn,
                         "gram_tflops": f_dn / t_dn / 1e12}}
 
