@@ -406,6 +406,9 @@ __device__ inline int sync_rho1_warp(int n, double2* rho1, double2* rinv, double
 
 // tridiag_ql by one warp: every lane runs the scalar recurrence on its own
 // copies of d and e, lane k rotates row k (k + 32) of z (shared by the warp).
+// c and s are quotients: as products by a rounded 1 / r they moved c^2 + s^2
+// off 1 and the error of a Lanczos step against 80-bit arithmetic was 4.9e-16
+// instead of 4.3e-16 (mean of 120 steps of 5,000 to 10,600 configurations).
 __device__ inline int tridiag_ql_warp(int n, double* d, double* e, double* z) {
     const int lane = threadIdx.x & 31;
     for (int k = lane; k < n; k += 32)
@@ -436,9 +439,8 @@ __device__ inline int tridiag_ql_warp(int n, double* d, double* e, double* z) {
                     deflated = true;
                     break;
                 }
-                const double ri = 1.0 / r;
-                s = f * ri;
-                c = g * ri;
+                s = f / r;
+                c = g / r;
                 g = d[i + 1] - p;
                 r = (d[i] - g) * s + 2.0 * c * b;
                 p = s * r;
