@@ -54,6 +54,38 @@ static int ensure_lanczos(mctdhb_space_s* h, int m) {
     return lanczos_alloc(h->lw, h->sp, std::max(m, 16));
 }
 
+// One product above 8 orbitals for a caller.  Calls on one space may overlap
+// there (other streams, other threads, a Step of the same space), so it stays
+// off the scratch that the space keeps for its Lanczos steps; products share
+// one of their own, and one on another stream than the last waits for that
+// one's event (a scratch from a stream-ordered pool for each call cost 6 us of
+// the 23-35 us a product takes).  A capture can wait for no event from outside
+// it: there the product runs row by row, which needs no scratch; in place, which
+// row by row is not possible, it takes the space's.
+static int apply_wide(mctdhb_space_s* h, const double2* C, double2* HC, cudaStream_t st) {
+    SpaceView v = h->sp.view;
+    const HcEpilogue ep;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        if (C != HC) v.pair_y = nullptr;
+        return hc_apply(v, C, HC, h->sp.d_tab, ep, st);
+    }
+    v.pair_y = h->sp.call_y;
+    std::lock_guard<std::mutex> lk(h->call_mu);
+    MCTDHB_CUDA_TRY(cudaStreamGetId(st, &id));
+    if (h->call_done == nullptr) {
+        MCTDHB_CUDA_TRY(cudaEventCreateWithFlags(&h->call_done, cudaEventDisableTiming));
+    } else if (id != h->call_stream) {
+        MCTDHB_CUDA_TRY(cudaStreamWaitEvent(st, h->call_done, 0));
+    }
+    h->call_stream = id;
+    const int rc = hc_apply(v, C, HC, h->sp.d_tab, ep, st);
+    MCTDHB_CUDA_TRY(cudaEventRecord(h->call_done, st));
+    return rc;
+}
+
 // ---------------------------------------------------------------------------
 // device-resident API
 // ---------------------------------------------------------------------------
@@ -81,6 +113,7 @@ void mctdhb_space_destroy(mctdhb_space h) {
     if (!h) return;
     lanczos_free(h->lw);
     space_release(h->sp);
+    if (h->call_done) cudaEventDestroy(h->call_done);
     delete h;
 }
 
@@ -100,9 +133,10 @@ int mctdhb_dev_apply_hamiltonian(mctdhb_space h, const void* d_coef, void* d_hc,
         set_error("mctdhb_dev_apply_hamiltonian: null argument");
         return -1;
     }
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (h->sp.call_y != nullptr) return apply_wide(h, (const double2*)d_coef, (double2*)d_hc, st);
     HcEpilogue ep;
-    return hc_apply(h->sp.view, (const double2*)d_coef, (double2*)d_hc, h->sp.d_tab, ep,
-                    (cudaStream_t)stream);
+    return hc_apply(h->sp.view, (const double2*)d_coef, (double2*)d_hc, h->sp.d_tab, ep, st);
 }
 
 int mctdhb_dev_density_matrices(mctdhb_space h, const void* d_coef, void* d_rho1, void* d_rho2,

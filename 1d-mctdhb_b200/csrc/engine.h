@@ -20,6 +20,7 @@ struct SpaceCtx {
     double2* d_tab = nullptr;       // H.C coefficient table (moves.cuh layout)
     int* d_dens_desc = nullptr;     // density element descriptors
     double2* d_dens_part = nullptr; // density partial sums
+    double2* call_y = nullptr;      // above 8 orbitals: pair scratch of callers' own products
 };
 
 int space_init(SpaceCtx& s, int N, int M);
@@ -79,4 +80,9 @@ struct mctdhb_space_s {
     mctdhb::SpaceCtx sp;
     mctdhb::LanczosWork lw;
     std::mutex mu;
+    // callers' own products above 8 orbitals (capi.cu): the event after the
+    // last one and its stream
+    std::mutex call_mu;
+    cudaEvent_t call_done = nullptr;
+    unsigned long long call_stream = 0;
 };

@@ -35,12 +35,10 @@ namespace mctdhb {
 // ---------------------------------------------------------------------------
 // coefficient table (hob row-major M*M, hint M^4) -> packed table
 // ---------------------------------------------------------------------------
-__global__ void hc_prep_kernel(int M, const double2* __restrict__ hob,
-                               const double2* __restrict__ hint,
-                               double2* __restrict__ tab) {
-    // one thread does the (tiny) enumeration in order; the table is a few KB
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    hc_pack_table(M, hob, hint, tab);
+__global__ void __launch_bounds__(256)
+    hc_prep_kernel(int M, const double2* __restrict__ hob, const double2* __restrict__ hint,
+                   double2* __restrict__ tab) {
+    hc_pack_table(M, hob, hint, tab, threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -179,15 +177,15 @@ int hcp_prepare(int M) {
 }
 
 int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, double2* d_tab,
-            cudaStream_t st) {
-    // the packed table is read by the per-row kernels alone: a space with pair
-    // scratch forms the pair matrix only (the table took one thread 52 us at
-    // four orbitals, 105 us at six)
-    if (sp.pair_y == nullptr)
-        hc_prep_kernel<<<1, 32, 0, st>>>(sp.M, d_hob, d_hint, d_tab);
-    else if (sp.M > kMaxTemplOrb)
-        return wide_prep(sp, d_hob, d_hint, st);
-    else
+            cudaStream_t st, bool rows) {
+    // The packed table is read by the per-row kernels alone: up to 8 orbitals a
+    // space with pair scratch forms the pair matrix only.  Above 8 the callers'
+    // own products still run row by row inside a capture (capi.cu); `rows`
+    // false: a space that takes no such calls.
+    if (sp.pair_y == nullptr || (rows && sp.M > kMaxTemplOrb))
+        hc_prep_kernel<<<1, 256, 0, st>>>(sp.M, d_hob, d_hint, d_tab);
+    if (sp.pair_y != nullptr && sp.M > kMaxTemplOrb) return wide_prep(sp, d_hob, d_hint, st);
+    if (sp.pair_y != nullptr)
         hcp_w_kernel<<<1, 256, 0, st>>>(sp.N, sp.M, d_hob, d_hint, sp.pair_w);
     MCTDHB_CUDA_TRY(cudaGetLastError());
     return 0;

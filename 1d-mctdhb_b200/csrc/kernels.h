@@ -188,9 +188,10 @@ int tune_lookup(const char* kernel, int N, int M);  // -1 when not tuned
 void tune_set(const char* kernel, int N, int M, int variant);  // a caller's choice
 
 // hamiltonian.cu
-// the packed coefficient table of h, g (and the pair matrix when sp has one)
+// what H.C reads of h, g: the pair matrix when sp has one, else the packed
+// coefficient table; above 8 orbitals both (rows: false leaves the table out)
 int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, double2* d_tab,
-            cudaStream_t st);
+            cudaStream_t st, bool rows = true);
 // whether the pair-space H.C applies to (N, M), and its scratch size in bytes
 bool hcp_eligible(int N, int M);
 size_t hcp_scratch_bytes(int N, int M);

@@ -150,39 +150,40 @@ __host__ __device__ void density_element_task(int M, int t, Fn&& f) {
 }
 
 // Packed H.C coefficient table (layout above) from h (M x M row-major) and
-// g (hint[k + sM + qM^2 + lM^3]); the caller runs it on one thread.
+// g (hint[k + sM + qM^2 + lM^3]) by threads t, t + nt, ...: a thread takes
+// orbital pairs (k, s) and writes what the layout holds for each.
 __device__ inline void hc_pack_table(int M, const double2* __restrict__ hob,
-                                     const double2* __restrict__ hint, double2* __restrict__ tab) {
+                                     const double2* __restrict__ hint, double2* __restrict__ tab,
+                                     int t, int nt) {
     const int M2 = M * M, M3 = M2 * M;
     auto g = [&](int a, int b, int c, int d) { return hint[a + b * M + c * M2 + d * M3]; };
-    int p = 0;
-    for (int k = 0; k < M; k++) tab[p++] = hob[k * M + k];
-    for (int k = 0; k < M; k++) tab[p++] = cscale(g(k, k, k, k), 0.5);
-    for (int k = 0; k < M; k++)
-        for (int s = k + 1; s < M; s++) tab[p++] = cscale(g(k, s, k, s), 2.0);
-    for (int k = 0; k < M; k++)
-        for (int l = 0; l < M; l++) {
-            if (l == k) continue;
-            double2 gk = g(k, k, k, l);
-            double2 h = hob[k * M + l];
-            tab[p++] = make_double2(h.x - gk.x, h.y - gk.y);
-            for (int s = 0; s < M; s++) {
-                if (s == k)
-                    tab[p++] = gk;
-                else if (s == l)
-                    tab[p++] = g(k, l, l, l);
-                else
-                    tab[p++] = cscale(g(k, s, s, l), 2.0);
-            }
+    for (int k = t; k < M; k += nt) {
+        tab[k] = hob[k * M + k];
+        tab[M + k] = cscale(g(k, k, k, k), 0.5);
+    }
+    for (int i = t; i < M2; i += nt) {
+        const int k = i / M, s = i % M;
+        if (s > k) tab[2 * M + k * (2 * M - k - 1) / 2 + s - k - 1] = cscale(g(k, s, k, s), 2.0);
+        if (s != k) {  // one boson s -> k, spectators x
+            const int l = s;
+            double2* p = tab + hc_ndiag(M) + (k * (M - 1) + (l > k ? l - 1 : l)) * (M + 1);
+            const double2 gk = g(k, k, k, l), h = hob[k * M + l];
+            *p++ = make_double2(h.x - gk.x, h.y - gk.y);
+            for (int x = 0; x < M; x++)
+                p[x] = x == k ? gk : x == l ? g(k, l, l, l) : cscale(g(k, x, x, l), 2.0);
         }
-    for (int k = 0; k < M; k++)
-        for (int s = k; s < M; s++)
-            for (int q = 0; q < M; q++)
-                for (int l = q; l < M; l++) {
-                    if (q == k || q == s || l == k || l == s) continue;
-                    double f = (k == s && q == l) ? 0.5 : ((k == s || q == l) ? 1.0 : 2.0);
-                    tab[p++] = cscale(g(k, s, q, l), f);
-                }
+        if (s < k) continue;
+        // two bosons to (k, s); the pairs before it, `eq` of them of equal orbitals
+        const int eq = k + (s > k), u = k * M - k * (k - 1) / 2 + s - k;
+        double2* p = tab + hc_ndiag(M) + hc_nsingle(M) + eq * (M * (M - 1) / 2) +
+                     (u - eq) * ((M - 1) * (M - 2) / 2);
+        for (int q = 0; q < M; q++)
+            for (int l = q; l < M; l++) {
+                if (q == k || q == s || l == k || l == s) continue;
+                const double f = (k == s && q == l) ? 0.5 : ((k == s || q == l) ? 1.0 : 2.0);
+                *p++ = cscale(g(k, s, q, l), f);
+            }
+    }
 }
 
 // Entry (P, Q) (pair_w_of), or e = P * npairs + Q (pair_w_entry), of the pair

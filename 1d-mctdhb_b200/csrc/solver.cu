@@ -187,13 +187,13 @@ int phase_coefficients(mctdhb_solver_s* s, cudaStream_t st) {
     if (s->cluster) {
         // with the pair matrix of H.C, where the space has one
         if (cluster_step(s, 0, kOrbPeriodic | kOrbMatrices, st)) return -1;
-        if (sc.view.pair_w == nullptr && hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st))
+        if (sc.view.pair_w == nullptr && hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st, false))
             return -1;
     } else {
         if (o.view.periodic && orb_periodic(o, s->d_orb, st)) return -1;
         if (orb_matrices(o, s->d_orb, s->d_hob, s->d_hint, st)) return -1;
         if (s->M == 1) return 0;  // Gross-Pitaevskii: the coefficient is trivial
-        if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st)) return -1;
+        if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st, false)) return -1;
     }
     if (s->coef_method == 21) {
         if (coef_rk_step(sc, s->sp->lw, s->d_coef, s->rk_order, s->dt, s->imagtime, st))
@@ -563,7 +563,7 @@ int mctdhb_solver_set_state(mctdhb_solver s, const void* orb, const void* coef) 
     if (orb_sync_rho1(s->orb, s->d_rho1, s->d_rinv, s->reg_fac, s->d_info, st)) return -1;
     if (orb_matrices(s->orb, s->d_orb, s->d_hob, s->d_hint, st)) return -1;
     if (s->M > 1) {
-        if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st)) return -1;
+        if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st, false)) return -1;
         HcEpilogue ep;  // tune H.C on this state before the graph is captured
         hc_variant(sc.view, s->d_coef, s->sp->lw.out, sc.d_tab, ep, st);
     }

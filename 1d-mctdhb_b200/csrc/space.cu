@@ -88,27 +88,32 @@ int space_init(SpaceCtx& s, int N, int M) {
     // Density partials and, for the pair-space H.C, the pair matrix and its
     // D(N-2, M) x P scratch, in one allocation (a large one costs 0.3 ms and
     // as much to give back).  When the scratch cannot be had the space keeps
-    // the per-row kernel.  More than 8 orbitals: taken only where the room
-    // left still holds every Lanczos workspace a caller may ask for (64
-    // vectors and the callers' own), so no call that ran beside the per-row
-    // kernel runs out of memory now.
+    // the per-row kernel.  More than 8 orbitals: twice the scratch, the second
+    // for callers' own products (capi.cu), and taken only where the room left
+    // still holds every Lanczos workspace a caller may ask for (64 vectors and
+    // the callers' own), so no call that ran beside the per-row kernel runs out
+    // of memory now.
     // (the scratch starts on 128 bytes)
     const size_t part = (dens_partial_elems(s.view) + 7) / 8 * 8;
     bool pair = hcp_eligible(N, M);
+    size_t scratch = hcp_scratch_bytes(N, M);
     if (wide_eligible(N, M)) {
+        scratch *= 2;
         size_t free_b = 0, total_b = 0;
         MCTDHB_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        pair = hcp_scratch_bytes(N, M) + (size_t)72 * dim * sizeof(double2) <= free_b;
+        pair = scratch + (size_t)72 * dim * sizeof(double2) <= free_b;
     }
     if (pair) pair = hcp_prepare(M) == 0 && (M > kMaxTemplOrb || small_prepare(M) == 0);
     if (pair) {
         const size_t P = (size_t)M * (M + 1) / 2, W = (P * P + 1 + 7) / 8 * 8;
-        const size_t bytes = (part + W) * sizeof(double2) + hcp_scratch_bytes(N, M);
+        const size_t bytes = (part + W) * sizeof(double2) + scratch;
         if (cudaMalloc(&s.d_dens_part, bytes) == cudaSuccess) {
             s.view.dim2 = (uint32_t)fock_dimension(N - 2, M);
             s.view.ldy = pair_ld(s.view.dim2);
             s.view.pair_w = s.d_dens_part + part;
             s.view.pair_y = s.view.pair_w + W;
+            if (M > kMaxTemplOrb)
+                s.call_y = s.view.pair_y + hcp_scratch_bytes(N, M) / sizeof(double2);
             return 0;
         }
         cudaGetLastError();  // clear the allocation failure

@@ -146,7 +146,13 @@ uint32_t mctdhb_space_dim(mctdhb_space sp);
  * each change of the orbital matrices). */
 int mctdhb_dev_set_matrices(mctdhb_space sp, const void* d_hob, const void* d_hint,
                             void* stream);
-/* HC = H C with the matrices of the last mctdhb_dev_set_matrices. */
+/* HC = H C with the matrices of the last mctdhb_dev_set_matrices.  From 2 to 8
+ * orbitals the product uses a scratch of the space: calls on one space must be
+ * ordered with one another and with its Lanczos steps (one stream, or events).
+ * Above 8 orbitals calls may overlap, with a step of the same space too: one on
+ * another stream than the last waits for it on the device; inside a stream
+ * capture the product runs row by row (slower, no scratch), except in place
+ * (d_hc = d_coef). */
 int mctdhb_dev_apply_hamiltonian(mctdhb_space sp, const void* d_coef, void* d_hc,
                                  void* stream);
 /* rho1 and rho2 of C in one pass. */
