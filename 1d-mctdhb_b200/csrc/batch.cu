@@ -201,6 +201,7 @@ struct mctdhb_batch_s {
     // autotuner when the step graph is captured (or set by the caller)
     int pair_v[kNumM] = {};
     bool pair_v_forced[kNumM] = {};
+    bool nowait = false;  // the contraction's handover without its waits
     std::mutex mu;
 };
 
@@ -334,15 +335,15 @@ int rebuild_lists(mctdhb_batch_s* b) {
 
 // H.C of Lanczos iteration `iter` of the slots of orbital count M
 int hc_group(int M, const BatchSlot* slots, const BatchTile* hy, const BatchTile* hg,
-             const int* cnt, int iter, cudaStream_t st, int parts = 3, int v = 0) {
+             const int* cnt, int iter, cudaStream_t st, int parts, int v, bool nowait) {
     switch (M) {
-        case 2: return hcp_batch_launch<2>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 3: return hcp_batch_launch<3>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 4: return hcp_batch_launch<4>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 5: return hcp_batch_launch<5>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 6: return hcp_batch_launch<6>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 7: return hcp_batch_launch<7>(slots, hy, hg, cnt, iter, parts, v, st);
-        case 8: return hcp_batch_launch<8>(slots, hy, hg, cnt, iter, parts, v, st);
+        case 2: return hcp_batch_launch<2>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 3: return hcp_batch_launch<3>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 4: return hcp_batch_launch<4>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 5: return hcp_batch_launch<5>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 6: return hcp_batch_launch<6>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 7: return hcp_batch_launch<7>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
+        case 8: return hcp_batch_launch<8>(slots, hy, hg, cnt, iter, parts, v, nowait, st);
     }
     return 0;
 }
@@ -443,7 +444,7 @@ int enqueue_general(mctdhb_batch_s* b, unsigned mask) {
     auto hc = [&](int iter) {
         return per_group(b, mask, [&](int M, cudaStream_t s) {
             return hc_group(M, S, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt, iter, s, 3,
-                            b->pair_v[M]);
+                            b->pair_v[M], b->nowait);
         });
     };
     // Lanczos (multiconfig_lanczos.c:12-90)
@@ -498,7 +499,7 @@ int enqueue_step(mctdhb_batch_s* b, unsigned mask, unsigned small) {
         const int* gl = list_at(b->d_list, b->max_slots, 1);
         if (per_group(b, mask, [&](int M, cudaStream_t s) {
                 return hc_group(M, S, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt,
-                                kBatchMonIter, s, 3, b->pair_v[M]);
+                                kBatchMonIter, s, 3, b->pair_v[M], b->nowait);
             }))
             return -1;
         bt_resid_kernel<<<num_sms() * 8, kBatchVecThreads, 0, st>>>(S, b->d_vec, cnt_vec(b->d_cnt));
@@ -533,7 +534,7 @@ int batch_tune_launch(void* p, int v, cudaStream_t st) {
     auto* c = (BatchTuneCtx*)p;
     if (!batch_v_ok(c->M, v)) return 1;
     return hc_group(c->M, c->b->d_slots, c->b->d_tl[LIST_HY], c->b->d_tl[LIST_HG], c->b->d_cnt,
-                    0, st, 1, v);
+                    0, st, 1, v, c->b->nowait);
 }
 
 int tune_group(mctdhb_batch_s* b, int M) {
@@ -1156,7 +1157,7 @@ int mctdhb_batch_launch_hc(mctdhb_batch b, int norb, int parts) {
     if (b->lists_dirty && rebuild_lists(b)) return -1;
     if (prepare_group(norb)) return -1;
     return hc_group(norb, b->d_slots, b->d_tl[LIST_HY], b->d_tl[LIST_HG], b->d_cnt + kCntInts, 0,
-                    b->st, parts, b->pair_v[norb]);
+                    b->st, parts, b->pair_v[norb], b->nowait);
 }
 
 int mctdhb_batch_variant(mctdhb_batch b, int norb) {
@@ -1179,6 +1180,17 @@ int mctdhb_batch_set_variant(mctdhb_batch b, int norb, int variant) {
     b->pair_v_forced[norb] = variant >= 0;
     b->pair_v[norb] = variant >= 0 ? variant : 0;
     drop_graph(b);  // captured with the old variant
+    return 0;
+}
+
+int mctdhb_batch_set_nowait(mctdhb_batch b, int on) {
+    if (!b) {
+        set_error("mctdhb_batch_set_nowait: null batch");
+        return -1;
+    }
+    std::lock_guard<std::mutex> lk(b->mu);
+    b->nowait = on != 0;
+    drop_graph(b);  // captured with the old launches
     return 0;
 }
 

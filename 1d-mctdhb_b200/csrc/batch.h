@@ -135,13 +135,14 @@ __host__ __device__ constexpr int batch_pair_rows(int M) {
 //                      gather-back (parts & 2); iter = kBatchMonIter: out =
 //                      H V[0] of the slots whose eigen residual is due;
 //                      variant: the contraction's launch variant (0, 2 or 3,
-//                      pairhc_tmpl.cuh)
+//                      pairhc_tmpl.cuh); nowait: its waits left out
 //   gram_batch_launch  rho2 of V[0] of the slots of orbital count M (`list` /
 //                      `nlist`: the slots; rho1 follows in bt_tail_kernel)
 //   batch_prepare      launch attributes (call before any stream capture)
 template <int M>
 int hcp_batch_launch(const BatchSlot* slots, const BatchTile* hy, const BatchTile* hg,
-                     const int* cnt, int iter, int parts, int variant, cudaStream_t st);
+                     const int* cnt, int iter, int parts, int variant, bool nowait,
+                     cudaStream_t st);
 template <int M>
 int gram_batch_launch(const BatchSlot* slots, const BatchTile* g2, const int* cnt,
                       const int* list, const int* nlist, int nblocks, cudaStream_t st);

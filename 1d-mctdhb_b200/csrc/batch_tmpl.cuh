@@ -36,7 +36,7 @@ struct PairTileMeta {
     int wbuf;  // variant 3: how many times W has been staged before this tile's
 };
 
-template <int M, int V>
+template <int M, int V, bool NOWAIT = false>
 __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
     bhcp_y_kernel(const BatchSlot* __restrict__ slots, const BatchTile* __restrict__ tiles,
                   const int* __restrict__ cnt, int iter) {
@@ -67,8 +67,9 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
         // the slot changes, all producer warps meet, stage its tables and W
         // (into the buffer of the slot before the last, once every consumer
         // warp has left that slot) and go on; the consumers of a tile wait for
-        // its W.  A wait that runs out marks the tile's job aborted; after one
-        // the warp waits for nothing more, so the others are not held up.
+        // its W.  A warp whose wait ran out takes no further part but for the
+        // producers' barriers (mbar_wait): it marks the job of every tile it
+        // still comes to aborted, since none of their Y is complete.
         __shared__ PairTileMeta meta[PS_::PW][2];
         __shared__ uint64_t full[PS_::PW][2], empty[PS_::PW][2], wfull[2], wdone[2];
         if (t < 2 * PS_::PW) {
@@ -81,11 +82,12 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
         }
         __syncthreads();
         bool lost = false;
-        auto wait = [&](uint64_t* bar, unsigned parity, int slot) {
-            if (!lost && !mbar_wait(bar, parity)) {
-                lost = true;
-                slots[slot].flags[BF_STATE] = SLOT_ABORTED;
-            }
+        auto wait = [&](uint64_t* bar, unsigned parity) {
+            lost = lost || !__all_sync(0xffffffffu, mbar_wait<NOWAIT>(bar, parity));
+        };
+        auto give_up = [&](int slot) {
+            const BatchSlot& S = slots[slot];
+            if (lane == 0 && bt_hc_active(S, iter)) S.flags[BF_STATE] = SLOT_ABORTED;
         };
         const int w = t >= PS_::CONSUMERS ? pt >> 5 : (t >> 5) / PS_::CPP;
         double2* ring = Ab + w * 2 * 32 * PS;
@@ -105,12 +107,18 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
                     ver++;
                     pair_producer_barrier<PS_::PRODUCERS>();  // nobody reads the old tables
                     pair_stage_tab(S.sp, tab, pt, PS_::PRODUCERS);
-                    if (ver >= 2) wait(&wdone[ver & 1], ((ver >> 1) - 1) & 1, tl.slot);
-                    pair_stage_w<M, V>(S.sp.pair_w, Wb + (ver & 1) * WW, pt, PS_::PRODUCERS);
-                    mbar_arrive(&wfull[ver & 1]);
+                    if (ver >= 2) wait(&wdone[ver & 1], ((ver >> 1) - 1) & 1);
+                    if (!lost) {
+                        pair_stage_w<M, V>(S.sp.pair_w, Wb + (ver & 1) * WW, pt, PS_::PRODUCERS);
+                        mbar_arrive(&wfull[ver & 1]);
+                    }
                     pair_producer_barrier<PS_::PRODUCERS>();
                 }
-                if (i >= 2) wait(&empty[w][buf], ((i >> 1) - 1) & 1, tl.slot);
+                if (i >= 2) wait(&empty[w][buf], ((i >> 1) - 1) & 1);
+                if (lost) {
+                    give_up(tl.slot);
+                    continue;
+                }
                 const uint32_t row0 = tl.idx * (uint32_t)ROWS + w * 32;
                 const bool active = bt_hc_active(S, iter) && row0 < S.sp.dim2;
                 if (lane == 0)
@@ -126,14 +134,18 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
             int ver = -1;
             for (int k = blockIdx.x; k < nt; k += gridDim.x, i++) {
                 const int buf = i & 1, slot = list[k].slot;
-                wait(&full[w][buf], (i >> 1) & 1, slot);
-                const PairTileMeta tm = meta[w][buf];
-                if (tm.wbuf != ver) {
+                wait(&full[w][buf], (i >> 1) & 1);
+                if (!lost && meta[w][buf].wbuf != ver) {
                     if (ver >= 0) mbar_arrive(&wdone[ver & 1]);
-                    ver = tm.wbuf;
-                    wait(&wfull[ver & 1], (ver >> 1) & 1, slot);
+                    ver = meta[w][buf].wbuf;
+                    wait(&wfull[ver & 1], (ver >> 1) & 1);
                 }
-                if (tm.active && !lost)
+                if (lost) {
+                    give_up(slot);
+                    continue;
+                }
+                const PairTileMeta tm = meta[w][buf];
+                if (tm.active)
                     pair_strips<M, V>(ring + buf * 32 * PS, Wb + (ver & 1) * WW,
                                       (t >> 5) % PS_::CPP, PS_::CPP, 2, lane, tm.row0, tm.D2,
                                       tm.ld, tm.Y, tm.real != 0);
@@ -296,6 +308,10 @@ int batch_y_attr() {
         MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bhcp_y_kernel<M, V>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)batch_y_smem<M, V>()));
+    if constexpr (PairHcShape<M, V>::PIPE)
+        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bhcp_y_kernel<M, V, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)batch_y_smem<M, V>()));
     return 0;
 }
 
@@ -313,13 +329,16 @@ int batch_prepare() {
 
 template <int M, int V>
 int bhcp_y_launch(const BatchSlot* slots, const BatchTile* hy, const int* cnt, int iter,
-                  cudaStream_t st) {
+                  bool nowait, cudaStream_t st) {
     if constexpr (!batch_variant_ok(M, V)) {
         set_error("batched pair contraction variant %d does not exist for %d orbitals", V, M);
         return -1;
     } else {
-        bhcp_y_kernel<M, V><<<num_sms(), PairHcShape<M, V>::THREADS, batch_y_smem<M, V>(), st>>>(
-            slots, hy, cnt, iter);
+        auto* kernel = bhcp_y_kernel<M, V>;
+        if constexpr (PairHcShape<M, V>::PIPE)
+            if (nowait) kernel = bhcp_y_kernel<M, V, true>;
+        kernel<<<num_sms(), PairHcShape<M, V>::THREADS, batch_y_smem<M, V>(), st>>>(slots, hy, cnt,
+                                                                                   iter);
         MCTDHB_CUDA_TRY(cudaGetLastError());
         return 0;
     }
@@ -327,11 +346,12 @@ int bhcp_y_launch(const BatchSlot* slots, const BatchTile* hy, const int* cnt, i
 
 template <int M>
 int hcp_batch_launch(const BatchSlot* slots, const BatchTile* hy, const BatchTile* hg,
-                     const int* cnt, int iter, int parts, int variant, cudaStream_t st) {
+                     const int* cnt, int iter, int parts, int variant, bool nowait,
+                     cudaStream_t st) {
     if (parts & 1) {
-        const int rc = variant == 3   ? bhcp_y_launch<M, 3>(slots, hy, cnt, iter, st)
-                       : variant == 2 ? bhcp_y_launch<M, 2>(slots, hy, cnt, iter, st)
-                                      : bhcp_y_launch<M, 0>(slots, hy, cnt, iter, st);
+        const int rc = variant == 3   ? bhcp_y_launch<M, 3>(slots, hy, cnt, iter, nowait, st)
+                       : variant == 2 ? bhcp_y_launch<M, 2>(slots, hy, cnt, iter, nowait, st)
+                                      : bhcp_y_launch<M, 0>(slots, hy, cnt, iter, nowait, st);
         if (rc) return -1;
     }
     if (parts & 2) {

@@ -119,6 +119,15 @@ void mctdhb_space_destroy(mctdhb_space h) {
 
 uint32_t mctdhb_space_dim(mctdhb_space h) { return h ? h->sp.dim : 0; }
 
+int mctdhb_space_set_nowait(mctdhb_space h, int on) {
+    if (!h) {
+        set_error("mctdhb_space_set_nowait: null space");
+        return -1;
+    }
+    h->sp.nowait = on != 0;
+    return 0;
+}
+
 int mctdhb_dev_set_matrices(mctdhb_space h, const void* d_hob, const void* d_hint, void* stream) {
     if (!h || !d_hob || !d_hint) {
         set_error("mctdhb_dev_set_matrices: null argument");
@@ -136,6 +145,7 @@ int mctdhb_dev_apply_hamiltonian(mctdhb_space h, const void* d_coef, void* d_hc,
     const cudaStream_t st = (cudaStream_t)stream;
     if (h->sp.call_y != nullptr) return apply_wide(h, (const double2*)d_coef, (double2*)d_hc, st);
     HcEpilogue ep;
+    ep.nowait = h->sp.nowait;
     return hc_apply(h->sp.view, (const double2*)d_coef, (double2*)d_hc, h->sp.d_tab, ep, st);
 }
 

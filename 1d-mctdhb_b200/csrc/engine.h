@@ -19,6 +19,7 @@ struct SpaceCtx {
     double* d_sq = nullptr;
     double2* d_tab = nullptr;       // H.C coefficient table (moves.cuh layout)
     int* d_dens_desc = nullptr;     // density element descriptors
+    bool nowait = false;            // the contraction's handover without its waits
     double2* d_dens_part = nullptr; // density partial sums
     double2* call_y = nullptr;      // above 8 orbitals: pair scratch of callers' own products
 };

@@ -36,6 +36,7 @@ struct HcEpilogue {
     int* init_flags = nullptr;
     double2 *init_max = nullptr, *init_offd = nullptr;
     int m = 0;
+    bool nowait = false;  // the contraction's handover without its waits (mctdhb_space_set_nowait)
 };
 
 // Deterministic block reduction of one complex value per thread; thread 0

@@ -341,6 +341,7 @@ static int lanczos_from(const SpaceCtx& s, LanczosWork& w, const double2* C, int
     for (int i = 0; i < m; i++) {
         double2* v = w.V + (size_t)i * n;
         HcEpilogue ep;
+        ep.nowait = s.nowait;
         if (i > 0 || !passes) ep.flag = w.iflag;
         if (i > 0) {
             ep.prev = v - n;
@@ -480,6 +481,7 @@ int coef_rk_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int order, dou
     // -i tf dt: tf = 1 (real time) or -i (imaginary time)
     const double2 f = imagtime ? make_double2(-dt, 0.0) : make_double2(0.0, -dt);
     HcEpilogue ep;
+    ep.nowait = s.nowait;
     auto H = [&](const double2* in, int j) {
         return hc_apply(s.view, in, V + (size_t)j * n, s.d_tab, ep, st);
     };

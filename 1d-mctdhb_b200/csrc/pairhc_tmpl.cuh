@@ -128,7 +128,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
                      mbar_addr(bar))
                  : "memory");
 }
-constexpr long long kMbarWaitCycles = 4000000000LL;
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
     unsigned done;
     asm volatile(
@@ -139,7 +138,25 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
         : "memory");
     return done != 0;
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(mbar_addr(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// Waits about 2 s at most; NOWAIT: what is not ready is lost at once.  The
+// lanes of a warp may disagree at the limit, so the callers take a vote before
+// they act on a loss.  A warp that lost a wait takes no further part: it arrives
+// on nothing that it has not waited for, so nobody takes a buffer for full or
+// empty that is not, and whoever depends on it runs out as well.
+constexpr long long kMbarWaitCycles = 4000000000LL;
+template <bool NOWAIT>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
+    if constexpr (NOWAIT) return mbar_test(bar, parity);
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(bar, parity))
@@ -524,6 +541,21 @@ __device__ __forceinline__ void pair_consume(const double2* As, const double2* W
                       real);
 }
 
+// NaN into all planes of the chunks of 32 rows c, c + step, ... < nchunk: they
+// were not handed over
+template <int M>
+__device__ __forceinline__ void pair_poison(uint32_t c, uint32_t step, uint32_t nchunk, int lane,
+                                            const SpaceView& sp, double2* __restrict__ Y) {
+    const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    for (; c < nchunk; c += step) {
+        const uint32_t m = c * 32 + lane;
+        if (m >= sp.dim2) continue;
+#pragma unroll 1
+        for (int p = 0; p < M * (M + 1) / 2; p++)
+            Y[(size_t)p * sp.ldy + m] = make_double2(nan, nan);
+    }
+}
+
 // (HC)_row = sum over pairs P = {k <= s} present in the row of
 // sqrt(n_k (n_s - [k=s])) Y_{row - e_k - e_s}(P)
 template <int M>
@@ -594,7 +626,7 @@ __device__ __forceinline__ double2 pair_gather_back(const SpaceView& sp,
 // start on 128 bytes: a fragment's 8 rows are one line).  Warp-specialised and
 // double-buffered: while the consumer warps contract rows from one A buffer,
 // the producer warps unrank and gather the next ones into the other.
-template <int M, int V>
+template <int M, int V, bool NOWAIT = false>
 __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
     hcp_y_kernel(SpaceView sp, const double2* __restrict__ C, const double2* __restrict__ W,
                  double2* __restrict__ Y, HcEpilogue ep) {
@@ -618,9 +650,16 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
         }
         __syncthreads();
         // pair w of this block takes the chunks of 32 rows blockIdx.x +
-        // w gridDim.x, ...: a small space spreads over the SMs first.  A lost
-        // handover (a wait that ran out) leaves NaN in Y, so the H.C and
-        // everything after it come out NaN instead of silently wrong.
+        // w gridDim.x, ...: a small space spreads over the SMs first.  A
+        // consumer that lost a wait leaves NaN in that chunk and all it still
+        // has to do: every row of H.C that reads one of them is NaN, and with it
+        // the dots of a Lanczos step and all that follows.  A producer that
+        // lost one stops, and its consumers run out.
+        // Where the loss is dealt with changes the code the compiler makes of
+        // the consumers' loop: at 7 orbitals in the loop (N=25 M=7: 165 us of
+        // H.C, 170 us after it), else after it (N=30 M=8: 2,955 us, 3,048 us in
+        // the loop; 2,932 us with no NaN and no vote at all).
+        constexpr bool IN_LOOP = M == 7;
         const int w = producer ? pt >> 5 : (t >> 5) / S::CPP;
         const uint32_t nchunk = (sp.dim2 + 31) / 32, step = gridDim.x * S::PW;
         double2* ring = Ab + w * 2 * 32 * PS;
@@ -631,7 +670,8 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
             pair_regs_dec<S::CREG, S::PREG>();
             for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
                 const int buf = i & 1;
-                if (i >= 2) ok = mbar_wait(&empty[w][buf], ((i >> 1) - 1) & 1);
+                if (i >= 2) ok = mbar_wait<NOWAIT>(&empty[w][buf], ((i >> 1) - 1) & 1);
+                if (!ok) return;
                 pair_gather_row<M, V>(tv, C, c * 32 + lane, ring + buf * 32 * PS, lane);
                 mbar_arrive(&full[w][buf]);
             }
@@ -639,13 +679,22 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
             pair_regs_inc<S::CREG>();
             for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
                 const int buf = i & 1;
-                ok = mbar_wait(&full[w][buf], (i >> 1) & 1);
+                ok = mbar_wait<NOWAIT>(&full[w][buf], (i >> 1) & 1);
                 pair_strips<M, V>(ring + buf * 32 * PS, Ws, (t >> 5) % S::CPP, S::CPP, 2, lane,
                                   c * 32, sp.dim2, sp.ldy, Y, real);
                 mbar_arrive(&empty[w][buf]);
+                if constexpr (IN_LOOP) {
+                    if (__any_sync(0xffffffffu, !ok)) {
+                        pair_poison<M>(c, step, nchunk, lane, sp, Y);
+                        return;
+                    }
+                } else {
+                    ok = __all_sync(0xffffffffu, ok);
+                }
             }
         }
-        if (!ok) Y[0] = make_double2(__longlong_as_double(0x7ff8000000000000LL), 0.0);
+        if (!IN_LOOP && !ok && !producer)
+            pair_poison<M>(c0 + (i - 1) * step, step, nchunk, lane, sp, Y);
         return;
     }
     __syncthreads();
@@ -694,6 +743,10 @@ int hcp_set_attr() {
         MCTDHB_CUDA_TRY(cudaFuncSetAttribute(hcp_y_kernel<M, V>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)PairHcShape<M, V>::SMEM));
+    if constexpr (PairHcShape<M, V>::PIPE)
+        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(hcp_y_kernel<M, V, true>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)PairHcShape<M, V>::SMEM));
     return 0;
 }
 
@@ -719,8 +772,10 @@ int hcp_launch_v(const SpaceView& sp, const double2* C, double2* HC, const HcEpi
             const uint32_t rows = S::PIPE ? 32 : S::ROWS, ntiles = (sp.dim2 + rows - 1) / rows;
             const int gy = (int)std::min<uint32_t>(ntiles, (uint32_t)num_sms());
             if (gy > 0) {
-                hcp_y_kernel<M, V><<<gy, S::THREADS, S::SMEM, st>>>(sp, C, sp.pair_w, sp.pair_y,
-                                                                    ep);
+                auto* kernel = hcp_y_kernel<M, V>;
+                if constexpr (S::PIPE)
+                    if (ep.nowait) kernel = hcp_y_kernel<M, V, true>;
+                kernel<<<gy, S::THREADS, S::SMEM, st>>>(sp, C, sp.pair_w, sp.pair_y, ep);
                 MCTDHB_CUDA_TRY(cudaGetLastError());
             }
         }

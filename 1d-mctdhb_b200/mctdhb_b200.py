@@ -43,6 +43,7 @@ EXPORTED = [
     "mctdhb_batch_monitor", "mctdhb_batch_lowest_state",
     "mctdhb_batch_kernel_count", "mctdhb_batch_stream", "mctdhb_batch_launch_hc",
     "mctdhb_batch_variant", "mctdhb_batch_set_variant", "mctdhb_tune_get", "mctdhb_tune_set",
+    "mctdhb_space_set_nowait", "mctdhb_batch_set_nowait",
     "mctdhb_fp64_mma_probe",
     "sync_density_matrices", "set_regulatization_factor", "get_current_regularization_factor",
     "mctdhb_step_create", "mctdhb_step_launch", "mctdhb_step_kernel_count",
@@ -233,6 +234,10 @@ def load(path=LIB_PATH):
     L.mctdhb_batch_variant.argtypes = [vp, i]
     L.mctdhb_batch_set_variant.restype = i
     L.mctdhb_batch_set_variant.argtypes = [vp, i, i]
+    L.mctdhb_space_set_nowait.restype = i
+    L.mctdhb_space_set_nowait.argtypes = [vp, i]
+    L.mctdhb_batch_set_nowait.restype = i
+    L.mctdhb_batch_set_nowait.argtypes = [vp, i]
     L.mctdhb_tune_get.restype = i
     L.mctdhb_tune_get.argtypes = [C.c_char_p, i, i]
     L.mctdhb_tune_set.restype = i
@@ -291,6 +296,10 @@ class Space:
             self.close()
         except Exception:
             pass
+
+    def set_nowait(self, on):
+        """the contraction's handover without its waits (mctdhb_space_set_nowait)"""
+        _check(load().mctdhb_space_set_nowait(self.h, int(on)), "mctdhb_space_set_nowait")
 
     def set_matrices(self, hob, hint, stream=None):
         _check(load().mctdhb_dev_set_matrices(self.h, _ptr(hob), _ptr(hint), _stream_ptr(stream)),
@@ -750,6 +759,10 @@ class Batch:
         """force a variant (-1: tune again); changes speed, never results"""
         _check(load().mctdhb_batch_set_variant(self.h, norb, variant),
                "mctdhb_batch_set_variant")
+
+    def set_nowait(self, on):
+        """the contraction's handover without its waits (mctdhb_batch_set_nowait)"""
+        _check(load().mctdhb_batch_set_nowait(self.h, int(on)), "mctdhb_batch_set_nowait")
 
     def launch_hc(self, norb, parts=3):
         """one batched H.C launch of the jobs with norb orbitals: parts = 1

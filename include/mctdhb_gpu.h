@@ -142,6 +142,13 @@ int      mctdhb_space_create(uint16_t npar, uint16_t norb, mctdhb_space* out);
 void     mctdhb_space_destroy(mctdhb_space sp);
 uint32_t mctdhb_space_dim(mctdhb_space sp);
 
+/* The contraction of H.C (variant 3) hands its rows over inside a block by
+ * bounded waits of about 2 s; a wait that runs out ends the launch with NaN in
+ * the rows of H.C that miss something, and the context stays usable.  on = 1:
+ * launches and captures after the call do not wait, so what is not ready at
+ * once is lost (to test how a caller deals with that). */
+int      mctdhb_space_set_nowait(mctdhb_space sp, int on);
+
 /* Pack h_kl and g_ksql into the coefficient table used by H.C (call after
  * each change of the orbital matrices). */
 int mctdhb_dev_set_matrices(mctdhb_space sp, const void* d_hob, const void* d_hint,
@@ -341,7 +348,8 @@ int    mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot);
 int    mctdhb_batch_step(mctdhb_batch b, int nsteps);
 int    mctdhb_batch_sync(mctdhb_batch b);
 /* per slot (arrays of max_slots, each may be NULL): state 0 empty,
- * 1 running, 2 stopped, 3 aborted (real time: overlap residual above 1e-3);
+ * 1 running, 2 stopped, 3 aborted (real time: overlap residual above 1e-3; or
+ * a handover of the contraction lost, mctdhb_batch_set_nowait);
  * steps done; current energy.  Returns the number of running jobs
  * (synchronises). */
 int    mctdhb_batch_poll(mctdhb_batch b, int* state, uint32_t* steps, double* energy);
@@ -380,6 +388,9 @@ int    mctdhb_batch_set_variant(mctdhb_batch b, int norb, int variant);
  * contraction, 2 the gather-back, 3 both; a measurement hook for timing the
  * dominant kernels of a step */
 int    mctdhb_batch_launch_hc(mctdhb_batch b, int norb, int parts);
+/* as mctdhb_space_set_nowait, for the batched contraction: a job that misses
+ * something stops with state 3 (aborted), the others go on */
+int    mctdhb_batch_set_nowait(mctdhb_batch b, int on);
 void*  mctdhb_batch_stream(mctdhb_batch b);       /* the engine's cudaStream_t */
 
 /* The autotuner (no counterpart in the reference; the reference's only
