@@ -188,6 +188,8 @@ struct mctdhb_batch_s {
     double2* h_scal = nullptr;  // of all slots, then kFetchWords of mctdhb_batch_fetch
     unsigned present_mask = 0;  // orbital counts on the general path
     unsigned small_mask = 0;    // orbital counts of the small slots
+    int orb_blocks = 0, small_blocks = 0;  // cluster sizes for the running slots
+    int orb_waves[kClusterSizes] = {}, small_waves[kNumM][kClusterSizes] = {};
     bool lists_dirty = true;
     cudaStream_t st = nullptr;
     cudaStream_t side[kNumM] = {}, side_small[kNumM] = {};
@@ -196,6 +198,7 @@ struct mctdhb_batch_s {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     unsigned graph_mask = 0, graph_small = 0;
+    int graph_orb_blocks = 0, graph_small_blocks = 0;
     int kernels = 0;
     // the pair contraction's launch variant per orbital count, chosen by the
     // autotuner when the step graph is captured (or set by the caller)
@@ -265,11 +268,13 @@ int rebuild_lists(mctdhb_batch_s* b) {
     for (int l = 0; l < kSlotLists; l++) list(l)[0] = 0;
     auto add = [&](int which, int slot) { list(which)[++list(which)[0]] = slot; };
     unsigned mask = 0, small = 0;
+    uint32_t small_rows = 0;
     for (int s = 0; s < b->max_slots; s++) {
         const HostSlot& h = b->hs[s];
         if (!h.used || !h.running) continue;
         add(0, s);
         if (h.small) {
+            small_rows = std::max(small_rows, h.L.nc);
             add(2 + h.d.M, s);
             small |= 1u << h.d.M;
             continue;
@@ -329,6 +334,18 @@ int rebuild_lists(mctdhb_batch_s* b) {
                                             cudaMemcpyHostToDevice, st));
     b->present_mask = mask;
     b->small_mask = small;
+    if (b->orb_waves[0] == 0 && (orb_step_prepare() || orb_step_waves(b->orb_waves))) return -1;
+    b->orb_blocks = cluster_blocks(b->orb_waves, list(0)[0]);
+    // the small slots of all orbital counts run beside one another
+    b->small_blocks = kClusterMax;
+    for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++) {
+        if (!(small >> M & 1)) continue;
+        if (b->small_waves[M][0] == 0 && (small_prepare(M) || small_waves(M, b->small_waves[M])))
+            return -1;
+        b->small_blocks = std::min(
+            b->small_blocks,
+            cluster_blocks(b->small_waves[M], list(0)[0] - list(1)[0], small_rows));
+    }
     b->lists_dirty = false;
     return 0;
 }
@@ -419,7 +436,8 @@ int fork_small(mctdhb_batch_s* b, unsigned mask, std::initializer_list<int> part
         MCTDHB_CUDA_TRY(cudaStreamWaitEvent(st, b->ev_fork_small, 0));
         const int* l = list_at(b->d_list, b->max_slots, 2 + M);
         for (int p : parts)
-            if (small_batch_launch(M, b->d_slots, l + 1, l, b->max_slots, p, st)) return -1;
+            if (small_batch_launch(M, b->d_slots, l + 1, l, b->max_slots, p, b->small_blocks, st))
+                return -1;
         MCTDHB_CUDA_TRY(cudaEventRecord(b->ev_join_small[M], st));
     }
     return 0;
@@ -482,7 +500,7 @@ int enqueue_step(mctdhb_batch_s* b, unsigned mask, unsigned small) {
     const int* sl = b->d_list + 1;
     const int sgrid = b->max_slots;
     int* mon = batch_mon(b->d_cnt);
-    if (orb_step_launch(S, sl, nL, sgrid, kOrbStep, mon, st)) return -1;
+    if (orb_step_launch(S, sl, nL, sgrid, kOrbStep, mon, b->orb_blocks, st)) return -1;
     // coefficients and densities: the small slots in three launches per
     // orbital count, beside the others
     if (fork_small(b, small, {kSmallLanczos, kSmallCombine, kSmallDens}) ||
@@ -552,7 +570,10 @@ int tune_group(mctdhb_batch_s* b, int M) {
 }
 
 int ensure_graph(mctdhb_batch_s* b) {
-    if (b->exec && b->graph_mask == b->present_mask && b->graph_small == b->small_mask) return 0;
+    if (b->exec && b->graph_mask == b->present_mask && b->graph_small == b->small_mask &&
+        b->graph_orb_blocks == b->orb_blocks &&
+        (b->small_mask == 0 || b->graph_small_blocks == b->small_blocks))
+        return 0;
     drop_graph(b);
     for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++)
         if (b->present_mask >> M & 1)
@@ -578,6 +599,8 @@ int ensure_graph(mctdhb_batch_s* b) {
     }
     b->graph_mask = b->present_mask;
     b->graph_small = b->small_mask;
+    b->graph_orb_blocks = b->orb_blocks;
+    b->graph_small_blocks = b->small_blocks;
     b->kernels = count_graph_kernels(b->graph);
     return 0;
 }
@@ -927,7 +950,7 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
         return undo();
     }
     if (prepare_group(M) || orb_step_prepare() ||
-        orb_step_launch(b->d_slots, pl + 1, pl, 1, kOrbMatrices, nullptr, st) ||
+        orb_step_launch(b->d_slots, pl + 1, pl, 1, kOrbMatrices, nullptr, kClusterMax, st) ||
         dens_group(M, b->d_slots, b->d_pro_g, dpc, pl + 1, pl, 1, st))
         return undo();
     bt_tail_kernel<<<1, kBatchVecThreads, 0, st>>>(b->d_slots, pl + 1, pl, 1, nullptr);

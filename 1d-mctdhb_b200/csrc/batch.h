@@ -27,6 +27,52 @@ constexpr int kBatchMinOrb = 2, kBatchMaxOrb = 8;
 constexpr int kBatchMaxGrid = 4096;
 constexpr int kBatchMonIter = -1;  // H.C launch of the monitor (eigen residual)
 
+// The orbital side of a slot, and the whole step of a small one, run on a
+// cluster of 1, 2, 4 or 8 blocks; the results do not depend on how many.  Eight
+// are the fastest for a slot by itself (a step of 4 jobs of N=12 M=4 on 512
+// points, RK5: 168 us, 261 with two blocks, 363 with one), but a block takes an
+// SM or half of one and a cluster does not cross a GPC, so 8 blocks a slot are
+// more than one wave from 9 or 17 slots.  Taken is the largest size of which all
+// slots' clusters run at once: 32 / 128 / 256 of these jobs 314 / 998 / 1,978 us
+// with 8 blocks, 200 / 365 / 622 so; of N=6 M=8 941 / 2,827 / 5,598 us, 500 /
+// 1,404 / 2,757 so.
+constexpr int kClusterMax = 8;  // the portable cluster size
+constexpr int kClusterSizes = 4;
+// A small slot's vectors stay in the L1 caches of its blocks up to about 8,192
+// rows a block (N=190 M=3, 18,336 rows, 256 jobs: 4,753 us on one block each,
+// 3,904 us on four), so a longer one takes more.
+// at[i]: clusters of 1 << i blocks that run at a time; rows: of a vector, the
+// longest (0: none)
+constexpr uint32_t kClusterRows = 8192;
+inline int cluster_blocks(const int (&at)[kClusterSizes], int n, uint32_t rows = 0) {
+    int i = kClusterSizes - 1;
+    while (i > 0 && at[i] < n && rows <= kClusterRows << (i - 1)) i--;
+    return 1 << i;
+}
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1] = {};
+    ClusterLaunch(int grid, int threads, size_t smem, int blocks, cudaStream_t st) {
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+};
+template <class K>
+int cluster_waves(K* kernel, int threads, size_t smem, int (&at)[kClusterSizes]) {
+    for (int i = 0; i < kClusterSizes; i++) {
+        ClusterLaunch c(1 << i, threads, smem, 1 << i, nullptr);
+        MCTDHB_CUDA_TRY(cudaOccupancyMaxActiveClusters(&at[i], kernel, &c.cfg));
+    }
+    return 0;
+}
+
 // per-slot device scalars (double2 units)
 constexpr int BS_DIAG = 0;
 constexpr int BS_OFFD = kBatchMaxLz;

@@ -28,10 +28,7 @@ namespace mctdhb {
 
 namespace {
 
-constexpr int kOrbCluster = 8;     // blocks per system (the portable cluster size)
 constexpr int kOrbThreads = 256;
-constexpr int kOrbAll = kOrbCluster * kOrbThreads;
-constexpr int kOrbWarps = kOrbAll / 32;
 constexpr int kOrbPiece = 256;     // grid points of one warp's sum
 constexpr int kOrbPieces = (kBatchMaxGrid + kOrbPiece - 1) / kOrbPiece;
 constexpr int kHintPiece = 64;     // grid points of one warp's g_ksql sum
@@ -44,7 +41,21 @@ struct OrbShared {
     unsigned char pq[40], pl[40];  // pair p <-> (q, l), q <= l
 };
 
-struct OrbBlock {
+// blocks, threads and warps of the cluster: constants for the single system,
+// B = 0 any number for the batch.  The batch has one instance alone: the
+// compiler fuses a b - c d into either of two multiply-adds, and two instances
+// need not agree.
+template <int B>
+struct OrbSize {
+    static constexpr int blocks = B, threads = B * kOrbThreads, warps = threads / 32;
+};
+template <>
+struct OrbSize<0> {
+    int blocks, threads, warps;
+};
+
+template <int B>
+struct OrbBlock : OrbSize<B> {
     cg::cluster_group cl = cg::this_cluster();
     OrbShared* sh;
     double2* sQ;  // M x M x P
@@ -53,12 +64,14 @@ struct OrbBlock {
 
 // the piece e of a sum, held by a whole warp (v of lane 0 .. 31 equal), into
 // every block's table
-__device__ __forceinline__ void put_piece(OrbBlock& o, int e, double2 v) {
-    if (o.lane < kOrbCluster) o.cl.map_shared_rank(o.sh, o.lane)->part[e] = v;
+template <class O>
+__device__ __forceinline__ void put_piece(O& o, int e, double2 v) {
+    if (o.lane < o.blocks) o.cl.map_shared_rank(o.sh, o.lane)->part[e] = v;
 }
 
 // out[e] = sum of the pieces e * np .. e * np + np - 1, e < n (own block)
-__device__ __forceinline__ void add_pieces(OrbBlock& o, int n, int np, double2* out) {
+template <class O>
+__device__ __forceinline__ void add_pieces(O& o, int n, int np, double2* out) {
     for (int e = threadIdx.x; e < n; e += kOrbThreads) {
         double2 v = o.sh->part[e * np];
         for (int c = 1; c < np; c++) v = cadd(v, o.sh->part[e * np + c]);
@@ -68,11 +81,11 @@ __device__ __forceinline__ void add_pieces(OrbBlock& o, int n, int np, double2* 
 }
 
 // pieces of <a_s|b_k> (Simpson) for all s, k
-template <int M>
-__device__ __forceinline__ void overlap_pieces(OrbBlock& o, const OrbView& ov, const double2* a,
+template <int M, class O>
+__device__ __forceinline__ void overlap_pieces(O& o, const OrbView& ov, const double2* a,
                                                const double2* b) {
     const int G = ov.G, np = (G + kOrbPiece - 1) / kOrbPiece;
-    for (int e = o.gwarp; e < M * M * np; e += kOrbWarps) {
+    for (int e = o.gwarp; e < M * M * np; e += o.warps) {
         const int s = e / np / M, k = e / np % M, x0 = e % np * kOrbPiece;
         const double2 *pa = a + (size_t)s * G, *pb = b + (size_t)k * G;
         double2 acc = make_double2(0.0, 0.0);
@@ -115,8 +128,8 @@ __device__ __forceinline__ double2 interacting(const double2* Qk, const double2 
 // robust projector (orbital_integration.c:22-92): P <- S^{-1} P with the full
 // overlap matrix S_sl = <y_s|y_l> of the stage orbitals; a singular S keeps
 // the simple projector's P and flags the system (BF_ROBFAIL)
-template <int M>
-__device__ void robust(OrbBlock& o, const BatchSlot& S, const double2* y) {
+template <int M, class O>
+__device__ void robust(O& o, const BatchSlot& S, const double2* y) {
     o.cl.sync();  // every block has added the pieces of P
     overlap_pieces<M>(o, S.ov, y, y);
     add_pieces(o, M * M, (S.ov.G + kOrbPiece - 1) / kOrbPiece, o.sh->b);
@@ -161,8 +174,8 @@ __constant__ Tableau kTableaux[3] = {
 // and with them the stage values there (stage[0..4]; the last is not kept);
 // the inputs of the stages alternate between stage[5] and stage[6], H phi is
 // in S.H.
-template <int M>
-__device__ void rk_step(OrbBlock& o, const BatchSlot& S) {
+template <int M, class O>
+__device__ void rk_step(O& o, const BatchSlot& S) {
     const OrbView& ov = S.ov;
     constexpr int P = M * (M + 1) / 2;
     const int G = ov.G, n = M * G, np = (G + kOrbPiece - 1) / kOrbPiece;
@@ -195,7 +208,7 @@ __device__ void rk_step(OrbBlock& o, const BatchSlot& S) {
                 if (S.orb_next) S.orb_next[t] = r;
             }
         };
-        for (int t = o.gtid; t < n; t += kOrbAll) {
+        for (int t = o.gtid; t < n; t += o.threads) {
             const int k = t / G, x = t - k * G;
             const double2* fk = in + (size_t)k * G;
             double2 f[M];
@@ -219,7 +232,7 @@ __device__ void rk_step(OrbBlock& o, const BatchSlot& S) {
             overlap_pieces<M>(o, ov, in, H);
             add_pieces(o, M * M, np, o.sh->a);
             if (rob) robust<M>(o, S, in);
-            for (int t = o.gtid; t < n; t += kOrbAll) {
+            for (int t = o.gtid; t < n; t += o.threads) {
                 const int k = t / G, x = t - k * G;
                 double2 proj = make_double2(0.0, 0.0);
 #pragma unroll
@@ -235,11 +248,12 @@ __device__ void rk_step(OrbBlock& o, const BatchSlot& S) {
 
 // linear half step of the split step, y <- Op y (orb_operator_kernel), through
 // stage[6]
-__device__ void half_step(OrbBlock& o, const BatchSlot& S, double2* y) {
+template <class O>
+__device__ void half_step(O& o, const BatchSlot& S, double2* y) {
     const int M = S.ov.M, G = S.ov.G, n = M * G;
     const int dense = S.half_dense, nn = dense ? G : G - 1;
     double2* w = S.stage + (size_t)6 * n;
-    for (int t = o.gtid; t < n; t += kOrbAll) {
+    for (int t = o.gtid; t < n; t += o.threads) {
         const int k = t / G, x = t - k * G;
         const double2* f = y + (size_t)k * G;
         double2 acc = make_double2(0.0, 0.0);
@@ -252,17 +266,17 @@ __device__ void half_step(OrbBlock& o, const BatchSlot& S, double2* y) {
         w[t] = acc;
     }
     o.cl.sync();
-    for (int t = o.gtid; t < n; t += kOrbAll) y[t] = w[t];
+    for (int t = o.gtid; t < n; t += o.threads) y[t] = w[t];
     o.cl.sync();
 }
 
 // h[j][k] + B[k][j] into sh->a[k M + j], B[k][j] = sum_a rinv[k][a]
 // sum_{s,q,l} rho2[a + sM + qM^2 + lM^3] hint[j + sM + lM^2 + qM^3]
 // (split_nonlinear_orbitals.c:63-160): one warp per (a, j)
-template <int M>
-__device__ void bmat(OrbBlock& o, const BatchSlot& S) {
+template <int M, class O>
+__device__ void bmat(O& o, const BatchSlot& S) {
     constexpr int M2 = M * M, M3 = M2 * M;
-    for (int e = o.gwarp; e < M2; e += kOrbWarps) {
+    for (int e = o.gwarp; e < M2; e += o.warps) {
         const int a = e / M, j = e % M;
         double2 acc = make_double2(0.0, 0.0);
         for (int c = o.lane; c < M3; c += 32) {
@@ -287,8 +301,8 @@ __device__ void bmat(OrbBlock& o, const BatchSlot& S) {
 // that overlap obeys ov_{k+1} = ov_k (1 - w_k |F_j[k]|^2), so the update is a
 // prefix product, which depends on F_j alone: formed once per orbital by a
 // block scan and kept in S.H.  A thread owns E consecutive points.
-template <int E>
-__device__ void gram_schmidt(OrbBlock& o, const BatchSlot& S) {
+template <int E, class O>
+__device__ void gram_schmidt(O& o, const BatchSlot& S) {
     const OrbView& ov = S.ov;
     const int M = ov.M, G = ov.G, x0 = threadIdx.x * E, warp = threadIdx.x >> 5;
     double* scan = (double*)S.H;  // M x G
@@ -368,8 +382,8 @@ __device__ void gram_schmidt(OrbBlock& o, const BatchSlot& S) {
 }
 
 // h_kl (orbital_matrices.c:22-70) and g_ksql (:73-287) of the orbitals
-template <int M>
-__device__ void matrices(OrbBlock& o, const BatchSlot& S) {
+template <int M, class O>
+__device__ void matrices(O& o, const BatchSlot& S) {
     constexpr int P = M * (M + 1) / 2, M2 = M * M, NT = (P + 7) / 8, TILES = NT * (NT + 1) / 2;
     const OrbView& ov = S.ov;
     const int G = ov.G, np = (G + kOrbPiece - 1) / kOrbPiece;
@@ -392,7 +406,7 @@ __device__ void matrices(OrbBlock& o, const BatchSlot& S) {
             }
     };
     const int gr = o.lane >> 2, kk = o.lane & 3;
-    for (int task = o.gwarp; task < TILES * hp; task += kOrbWarps) {
+    for (int task = o.gwarp; task < TILES * hp; task += o.warps) {
         const int tile = task / hp, piece = task % hp;
         int ti = 0, tj = tile;
         while (tj >= NT - ti) {
@@ -431,7 +445,7 @@ __device__ void matrices(OrbBlock& o, const BatchSlot& S) {
             }
         }
     }
-    for (int e = o.gwarp; e < P * np; e += kOrbWarps) {
+    for (int e = o.gwarp; e < P * np; e += o.warps) {
         const int p = e / np, x0 = e % np * kOrbPiece;
         const double2* fk = S.orb + (size_t)o.sh->pq[p] * G;
         const double2* fl = S.orb + (size_t)o.sh->pl[p] * G;
@@ -449,7 +463,7 @@ __device__ void matrices(OrbBlock& o, const BatchSlot& S) {
     }
     o.cl.sync();
     if (hp > 1)
-        for (int e = o.gtid; e < TILES * 64; e += kOrbAll) {
+        for (int e = o.gtid; e < TILES * 64; e += o.threads) {
             const int tile = e >> 6, cell = e & 63;
             int ti = 0, tj = tile;
             while (tj >= NT - ti) {
@@ -463,7 +477,7 @@ __device__ void matrices(OrbBlock& o, const BatchSlot& S) {
             for (int c = 1; c < hp; c++) v = cadd(v, S.stage[(size_t)(tile * hp + c) * 64 + cell]);
             fill(pr, pc, v);
         }
-    if (o.rank == kOrbCluster - 1)
+    if (o.rank == o.blocks - 1)
         for (int p = threadIdx.x; p < P; p += kOrbThreads) {
             double2 v = o.sh->part[p * np];
             for (int c = 1; c < np; c++) v = cadd(v, o.sh->part[p * np + c]);
@@ -475,8 +489,8 @@ __device__ void matrices(OrbBlock& o, const BatchSlot& S) {
     o.cl.sync();
 }
 
-template <int M>
-__device__ void run_step(OrbBlock& o, const BatchSlot& S, int parts) {
+template <int M, class O>
+__device__ void run_step(O& o, const BatchSlot& S, int parts) {
     constexpr int P = M * (M + 1) / 2, M2 = M * M, M3 = M2 * M;
     const OrbView& ov = S.ov;
     const int G = ov.G, np = (G + kOrbPiece - 1) / kOrbPiece;
@@ -586,17 +600,23 @@ constexpr size_t orb_step_smem() {
 
 }  // namespace
 
-__global__ void __cluster_dims__(kOrbCluster, 1, 1) __launch_bounds__(kOrbThreads)
+template <int B>
+__global__ void __launch_bounds__(kOrbThreads)
     orb_step_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
                     const int* __restrict__ nlist, int parts, int* __restrict__ mon) {
     // a new step: no monitor H.C due yet in any orbital count
     if (mon != nullptr && blockIdx.x == 0 && threadIdx.x < kBatchNumM) mon[threadIdx.x] = 0;
-    const int s = blockIdx.x / kOrbCluster;
+    OrbBlock<B> o;
+    if constexpr (B == 0) {
+        o.blocks = (int)o.cl.num_blocks();
+        o.threads = o.blocks * kOrbThreads;
+        o.warps = o.threads / 32;
+    }
+    const int s = blockIdx.x / o.blocks;
     if (s >= *nlist) return;  // the same in every block of the cluster
     const BatchSlot& S = slots[list[s]];
     if (S.flags[BF_STATE] != SLOT_RUNNING) return;
     extern __shared__ __align__(16) unsigned char mem[];
-    OrbBlock o;
     o.sh = (OrbShared*)mem;
     o.sQ = (double2*)(mem + sizeof(OrbShared));
     o.rank = (int)o.cl.block_rank();
@@ -618,18 +638,24 @@ __global__ void __cluster_dims__(kOrbCluster, 1, 1) __launch_bounds__(kOrbThread
 int orb_step_prepare() {
     static std::atomic<uint64_t> done{0};
     return set_attributes_once(done, []() -> int {
-        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(orb_step_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)orb_step_smem()));
+        for (auto* kernel : {orb_step_kernel<0>, orb_step_kernel<kClusterMax>})
+            MCTDHB_CUDA_TRY(cudaFuncSetAttribute(kernel,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)orb_step_smem()));
         return 0;
     });
 }
 
+int orb_step_waves(int (&at)[kClusterSizes]) {
+    return cluster_waves(orb_step_kernel<0>, kOrbThreads, orb_step_smem(), at);
+}
+
 int orb_step_launch(const BatchSlot* slots, const int* list, const int* nlist, int nslots,
-                    int parts, int* mon, cudaStream_t st) {
-    orb_step_kernel<<<nslots * kOrbCluster, kOrbThreads, orb_step_smem(), st>>>(slots, list, nlist,
-                                                                               parts, mon);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
+                    int parts, int* mon, int blocks, cudaStream_t st) {
+    const int size = blocks > 0 ? blocks : kClusterMax;
+    ClusterLaunch c(nslots * size, kOrbThreads, orb_step_smem(), size, st);
+    auto* kernel = blocks > 0 ? orb_step_kernel<0> : orb_step_kernel<kClusterMax>;
+    MCTDHB_CUDA_TRY(cudaLaunchKernelEx(&c.cfg, kernel, slots, list, nlist, parts, mon));
     return 0;
 }
 

@@ -17,12 +17,15 @@ constexpr int kOrbPost = 16;      // periodic copy again, overlap residual in re
 constexpr int kOrbMatrices = 32;  // h, g, the pair matrix, Lanczos set-up
 constexpr int kOrbStep = 63;
 
-// A cluster of kOrbCluster blocks per slot of the list; mon: the count
-// block's monitor flags, cleared by the first block (nullptr: none)
+// A cluster of `blocks` per slot of the list: 1, 2, 4 or 8, on which the results
+// do not depend, or 0 for eight by code made for eight; mon: the count block's monitor flags, cleared by the first block
+// (nullptr: none)
 int orb_step_launch(const BatchSlot* slots, const int* list, const int* nlist, int nslots,
-                    int parts, int* mon, cudaStream_t st);
+                    int parts, int* mon, int blocks, cudaStream_t st);
 // launch attributes (call before any stream capture)
 int orb_step_prepare();
+// clusters that run at a time (cluster_blocks)
+int orb_step_waves(int (&at)[kClusterSizes]);
 inline bool orb_step_eligible(int M, int G) {
     return M >= kBatchMinOrb && M <= kBatchMaxOrb && G <= kBatchMaxGrid;
 }

@@ -7,10 +7,12 @@ namespace mctdhb {
 template <int M>
 int small_prepare_tmpl();
 template <int M>
+int small_waves_tmpl(int (&at)[kClusterSizes]);
+template <int M>
 int small_launch_tmpl(const SmallSys& s, int part, int i, cudaStream_t st);
 template <int M>
 int small_batch_tmpl(const BatchSlot* slots, const int* list, const int* nlist, int nslots,
-                     int part, cudaStream_t st);
+                     int part, int blocks, cudaStream_t st);
 
 bool small_eligible(int N, int M, uint32_t D2, double macs) {
     const double P = 0.5 * M * (M + 1);
@@ -36,6 +38,12 @@ int small_prepare(int M) {
 #undef CALL
 }
 
+int small_waves(int M, int (&at)[kClusterSizes]) {
+#define CALL(m) small_waves_tmpl<m>(at)
+    MCTDHB_BY_M(CALL);
+#undef CALL
+}
+
 int small_launch(const SmallSys& s, int part, int i, cudaStream_t st) {
     const int M = s.sp.M;
 #define CALL(m) small_launch_tmpl<m>(s, part, i, st)
@@ -44,8 +52,8 @@ int small_launch(const SmallSys& s, int part, int i, cudaStream_t st) {
 }
 
 int small_batch_launch(int M, const BatchSlot* slots, const int* list, const int* nlist,
-                       int nslots, int part, cudaStream_t st) {
-#define CALL(m) small_batch_tmpl<m>(slots, list, nlist, nslots, part, st)
+                       int nslots, int part, int blocks, cudaStream_t st) {
+#define CALL(m) small_batch_tmpl<m>(slots, list, nlist, nslots, part, blocks, st)
     MCTDHB_BY_M(CALL);
 #undef CALL
 }

@@ -26,7 +26,7 @@
 
 namespace mctdhb {
 
-constexpr int kSmCluster = 8, kSmThreads = 256, kSmAll = kSmCluster * kSmThreads;
+constexpr int kSmThreads = 256, kSmAll = kClusterMax * kSmThreads;  // numbered threads
 constexpr int kSmWarps = kSmAll / 32;
 
 template <int M>
@@ -39,30 +39,55 @@ struct SmallShared {
     double2 tab[kPairTabBytes / sizeof(double2)];
 };
 
-template <int M>
-struct SmallRun {
+// blocks and threads of the cluster: constants for the single system, B = 0 any
+// number for the batch (one instance alone, as orbstep.cu says)
+template <int B>
+struct SmallSize {
+    static constexpr int blocks = B, threads = B * kSmThreads;
+};
+template <>
+struct SmallSize<0> {
+    int blocks, threads;
+};
+
+template <int M, int B>
+struct SmallRun : SmallSize<B> {
+    using SmallSize<B>::blocks;
+    using SmallSize<B>::threads;
     static constexpr int P = M * (M + 1) / 2;
     using Sh = SmallShared<M>;
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const SmallSys& s;
     Sh* sh;
     SpaceView sp;  // tables in shared memory
-    int rank, gtid, gwarp, lane;
+    int rank, lane, gtid;
 
     __device__ SmallRun(const SmallSys& sys, Sh* mem) : s(sys), sh(mem) {
+        if constexpr (B == 0) {
+            blocks = (int)cl.num_blocks();
+            threads = blocks * kSmThreads;
+        }
         rank = (int)cl.block_rank();
-        gtid = rank * kSmThreads + threadIdx.x;
-        gwarp = gtid >> 5;
         lane = threadIdx.x & 31;
+        gtid = rank * kSmThreads + threadIdx.x;
         sp = pair_stage_tab(s.sp, sh->tab, threadIdx.x, kSmThreads);
         for (int i = threadIdx.x; i < P * P; i += kSmThreads) sh->W[i] = s.sp.pair_w[i];
         cl.sync();  // own tables ready, and every block of the cluster runs
     }
 
-    // this warp's share of sum k into every block's table
-    __device__ __forceinline__ void put(int k, double2 v) {
+    // f(n) for the numbers of the 2,048 that this thread stands for, whole warps
+    // together: rows go to numbers, so that neither the sums nor who owns a row
+    // depend on how many blocks the cluster has
+    template <class F>
+    __device__ __forceinline__ void each(F&& f) {
+        const int per = kClusterMax / blocks;
+#pragma unroll 1
+        for (int b = rank * per; b < (rank + 1) * per; b++) f(b * kSmThreads + (int)threadIdx.x);
+    }
+    // the share of the warp with number n in sum k, into every block's table
+    __device__ __forceinline__ void put(int k, int n, double2 v) {
         v = warp_sum(v);
-        if (lane < kSmCluster) cl.map_shared_rank(sh, lane)->piece[k * kSmWarps + gwarp] = v;
+        if (lane < blocks) cl.map_shared_rank(sh, lane)->piece[k * kSmWarps + (n >> 5)] = v;
     }
     // sum k, in every lane (after the barrier that follows its put)
     __device__ __forceinline__ double2 total(int k) {
@@ -93,8 +118,8 @@ struct SmallRun {
     // keep every thread busy
     __device__ __forceinline__ void contract(const double2* C) {
         const uint32_t D2 = sp.dim2;
-        const int ng = max(1, min(P, (int)(kSmAll / D2))), per = (P + ng - 1) / ng;
-        for (uint32_t e = gtid; e < D2 * ng; e += kSmAll) {
+        const int ng = max(1, min(P, threads / (int)D2)), per = (P + ng - 1) / ng;
+        for (uint32_t e = gtid; e < D2 * ng; e += threads) {
             const uint32_t row = e % D2;
             const int p0 = (int)(e / D2) * per, p1 = min(p0 + per, P);
             if (p0 >= p1) continue;
@@ -166,7 +191,7 @@ struct SmallRun {
 
     __device__ __forceinline__ void hc() {
         contract(s.C);
-        for (uint32_t r = gtid; r < sp.dim; r += kSmAll) s.out[r] = back(r);
+        for (uint32_t r = gtid; r < sp.dim; r += threads) s.out[r] = back(r);
     }
 
     // The Lanczos recurrence (multiconfig_lanczos.c:12-90), the operations of
@@ -180,27 +205,33 @@ struct SmallRun {
         double beta = 0.0;
         if (i == 0) {
             if (s.V != s.C)
-                for (uint32_t r = gtid; r < nc; r += kSmAll) v[r] = s.C[r];
+                each([&](int n) {
+                    for (uint32_t r = n; r < nc; r += kSmAll) v[r] = s.C[r];
+                });
         } else {
             beta = s.offd[i - 1].x;
             const double inv = s.misc[1].x;
-            for (uint32_t r = gtid; r < nc; r += kSmAll) v[r] = cscale(s.out[r], inv);
+            each([&](int n) {
+                for (uint32_t r = n; r < nc; r += kSmAll) v[r] = cscale(s.out[r], inv);
+            });
             cl.sync();
         }
         contract(i == 0 ? s.C : v);
-        double2 acc = make_double2(0.0, 0.0);
-        for (uint32_t r = gtid; r < nc; r += kSmAll) {
-            double2 h = back(r);
-            const double2 c = i == 0 ? s.C[r] : v[r];
-            if (i > 0) {
-                const double2 pv = s.V[(size_t)(i - 1) * nc + r];
-                h.x -= beta * pv.x;
-                h.y -= beta * pv.y;
+        each([&](int n) {
+            double2 acc = make_double2(0.0, 0.0);
+            for (uint32_t r = n; r < nc; r += kSmAll) {
+                double2 h = back(r);
+                const double2 c = i == 0 ? s.C[r] : v[r];
+                if (i > 0) {
+                    const double2 pv = s.V[(size_t)(i - 1) * nc + r];
+                    h.x -= beta * pv.x;
+                    h.y -= beta * pv.y;
+                }
+                s.out[r] = h;
+                acc = cfma_conj(c, h, acc);
             }
-            s.out[r] = h;
-            acc = cfma_conj(c, h, acc);
-        }
-        put(0, acc);
+            put(0, n, acc);
+        });
         cl.sync();
         const double2 alpha = total(0);
         if (gtid == 0) {
@@ -222,39 +253,45 @@ struct SmallRun {
     __device__ __forceinline__ bool orthogonalise(int i, double2 alpha) {
         const uint32_t nc = sp.dim;
         const double2* v = s.V + (size_t)i * nc;
-        for (uint32_t r = gtid; r < nc; r += kSmAll) {
-            double2 o = s.out[r];
-            const double2 av = cmul(alpha, v[r]);
-            o.x -= av.x;
-            o.y -= av.y;
-            s.out[r] = o;
-        }
-        for (int k = 0; k <= i; k++) {
-            double2 acc = make_double2(0.0, 0.0);
-            for (uint32_t r = gtid; r < nc; r += kSmAll)
-                acc = cfma_conj(s.V[(size_t)k * nc + r], s.out[r], acc);
-            put(k, acc);
-        }
+        each([&](int n) {
+            for (uint32_t r = n; r < nc; r += kSmAll) {
+                double2 o = s.out[r];
+                const double2 av = cmul(alpha, v[r]);
+                o.x -= av.x;
+                o.y -= av.y;
+                s.out[r] = o;
+            }
+            for (int k = 0; k <= i; k++) {
+                double2 acc = make_double2(0.0, 0.0);
+                for (uint32_t r = n; r < nc; r += kSmAll)
+                    acc = cfma_conj(s.V[(size_t)k * nc + r], s.out[r], acc);
+                put(k, n, acc);
+            }
+        });
         cl.sync();
         for (int k = 0; k <= i; k++) {
             const double2 ok = total(k);
-            for (uint32_t r = gtid; r < nc; r += kSmAll) {
-                const double2 t = cmul(s.V[(size_t)k * nc + r], ok);
-                double2 o = s.out[r];
-                o.x -= t.x;
-                o.y -= t.y;
-                s.out[r] = o;
+            each([&](int n) {
+                for (uint32_t r = n; r < nc; r += kSmAll) {
+                    const double2 t = cmul(s.V[(size_t)k * nc + r], ok);
+                    double2 o = s.out[r];
+                    o.x -= t.x;
+                    o.y -= t.y;
+                    s.out[r] = o;
+                }
+            });
+        }
+        each([&](int n) {
+            double nrm = 0.0;
+            for (uint32_t r = n; r < nc; r += kSmAll) {
+                const double2 o = s.out[r];
+                nrm += o.x * o.x + o.y * o.y;
             }
-        }
-        double nrm = 0.0;
-        for (uint32_t r = gtid; r < nc; r += kSmAll) {
-            const double2 o = s.out[r];
-            nrm += o.x * o.x + o.y * o.y;
-        }
-        cl.sync();  // every warp has added the pieces of the dots
-        put(0, make_double2(nrm, 0.0));
+            // the last table: no dot is there (i < m - 1 <= kBatchMaxLz - 1)
+            put(kBatchMaxLz - 1, n, make_double2(nrm, 0.0));
+        });
         cl.sync();
-        const double beta = sqrt(total(0).x), mx = fmax(s.misc[0].x, beta);
+        const double beta = sqrt(total(kBatchMaxLz - 1).x), mx = fmax(s.misc[0].x, beta);
         const bool broke = beta == 0.0 || beta / mx < 1e-14;
         cl.sync();  // every thread has read the maximum before it changes
         if (gtid == 0) {
@@ -322,22 +359,26 @@ struct SmallRun {
             }
         }
         __syncthreads();
-        double nrm = 0.0;
-        for (uint32_t r = gtid; r < nc; r += kSmAll) {
-            double2 c = make_double2(0.0, 0.0);
-            for (int j = 0; j < built; j++) c = cfma(s.V[(size_t)j * nc + r], sh->y[j], c);
-            s.C[r] = c;
-            nrm += c.x * c.x + c.y * c.y;
-        }
+        each([&](int n) {
+            double nrm = 0.0;
+            for (uint32_t r = n; r < nc; r += kSmAll) {
+                double2 c = make_double2(0.0, 0.0);
+                for (int j = 0; j < built; j++) c = cfma(s.V[(size_t)j * nc + r], sh->y[j], c);
+                s.C[r] = c;
+                nrm += c.x * c.x + c.y * c.y;
+            }
+            if (s.renorm) put(0, n, make_double2(nrm, 0.0));
+        });
         if (!s.renorm) return;
-        put(0, make_double2(nrm, 0.0));
         cl.sync();
         const double n2 = total(0).x, rn = 1.0 / sqrt(n2);
         if (gtid == 0) *s.norm2 = make_double2(n2, 0.0);
-        for (uint32_t r = gtid; r < nc; r += kSmAll) {
-            s.C[r].x *= rn;
-            s.C[r].y *= rn;
-        }
+        each([&](int n) {
+            for (uint32_t r = n; r < nc; r += kSmAll) {
+                s.C[r].x *= rn;
+                s.C[r].y *= rn;
+            }
+        });
     }
 
     // rho2 as the Gram matrix of the A planes (in the scratch of Y), a warp an
@@ -345,7 +386,7 @@ struct SmallRun {
     __device__ __forceinline__ void densities() {
         const uint32_t D2 = sp.dim2;
         double2* A = s.sp.pair_y;
-        for (uint32_t row = gtid; row < D2; row += kSmAll) {
+        for (uint32_t row = gtid; row < D2; row += threads) {
             double2 a[P];
             amplitudes(row, s.C, a);
             static_for<P>([&](auto pi) {
@@ -355,7 +396,7 @@ struct SmallRun {
         }
         cl.sync();
         constexpr int M2 = M * M, M3 = M2 * M;
-        for (int e = gwarp; e < P * (P + 1) / 2; e += kSmWarps) {
+        for (int e = gtid >> 5; e < P * (P + 1) / 2; e += threads / 32) {
             int pa = 0, pb = e;
             while (pb >= P - pa) {
                 pb -= P - pa;
@@ -391,11 +432,11 @@ struct SmallRun {
 // one system: a part of its step (smallsys.h), iteration i of the Lanczos
 // recurrence
 template <int M>
-__global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
+__global__ void __launch_bounds__(kSmThreads)
     small_kernel(SmallSys s, int part, int i) {
     extern __shared__ __align__(16) unsigned char small_mem[];
     if ((part == kSmallProduct || part == kSmallOrth) && i > 0 && s.iflag[0]) return;  // breakdown
-    SmallRun<M> r(s, (SmallShared<M>*)small_mem);
+    SmallRun<M, kClusterMax> r(s, (SmallShared<M>*)small_mem);
     switch (part) {
         case kSmallHc: r.hc(); break;
         case kSmallProduct: r.product(i); break;
@@ -408,10 +449,10 @@ __global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
 // residual max_i |E C_i - (H C)_i| / N where it is due, and the eigen-residual
 // half of the stop rule (bt_monitor_kernel)
 template <int M>
-__global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
+__global__ void __launch_bounds__(kSmThreads)
     small_batch_kernel(const BatchSlot* __restrict__ slots, const int* __restrict__ list,
                        const int* __restrict__ nlist, int part) {
-    const int at = blockIdx.x / kSmCluster;
+    const int at = blockIdx.x / (int)cooperative_groups::this_cluster().num_blocks();
     if (at >= *nlist) return;  // the same in every block of the cluster
     const BatchSlot& S = slots[list[at]];
     if (part == kSmallMonitor ? !S.flags[BF_MON] : S.flags[BF_STATE] != SLOT_RUNNING) return;
@@ -433,7 +474,7 @@ __global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
     s.shift = 1;
     s.renorm = S.imag;
     static_assert(BF_BREAK == 0 && BF_ITERS == 1 && BF_QL == 2, "iflag is the head of the flags");
-    SmallRun<M> r(s, (SmallShared<M>*)small_mem);
+    SmallRun<M, 0> r(s, (SmallShared<M>*)small_mem);
     if (part == kSmallLanczos) {
         r.lanczos();
         return;
@@ -449,16 +490,19 @@ __global__ void __cluster_dims__(kSmCluster, 1, 1) __launch_bounds__(kSmThreads)
     r.contract(s.C);
     const double e = S.scal[BS_MISC + 3].x;
     double worst = 0.0;
-    for (uint32_t i = r.gtid; i < S.nc; i += kSmAll) {
+    for (uint32_t i = r.gtid; i < S.nc; i += r.threads) {
         const double2 c = s.C[i], h = r.back(i);
         worst = fmax(worst, hypot(e * c.x - h.x, e * c.y - h.y));
     }
     worst = warp_max_f64(worst);
-    if (r.lane < kSmCluster)
-        r.cl.map_shared_rank(r.sh, r.lane)->piece[r.gwarp] = make_double2(worst, 0.0);
+    const int warps = r.threads / 32;
+    if (r.lane < r.blocks)
+        r.cl.map_shared_rank(r.sh, r.lane)->piece[r.gtid >> 5] = make_double2(worst, 0.0);
     r.cl.sync();
     if (r.rank != 0 || threadIdx.x >= 32) return;
-    worst = warp_max_f64(fmax(r.sh->piece[r.lane].x, r.sh->piece[r.lane + 32].x));
+    worst = 0.0;
+    for (int w = r.lane; w < warps; w += 32) worst = fmax(worst, r.sh->piece[w].x);
+    worst = warp_max_f64(worst);
     if (r.lane != 0) return;
     const double res = worst / S.N;
     S.scal[BS_MISC + 6] = make_double2(res, 0.0);
@@ -482,18 +526,22 @@ int small_prepare_tmpl() {
 }
 
 template <int M>
+int small_waves_tmpl(int (&at)[kClusterSizes]) {
+    return cluster_waves(small_batch_kernel<M>, kSmThreads, sizeof(SmallShared<M>), at);
+}
+
+template <int M>
 int small_launch_tmpl(const SmallSys& s, int part, int i, cudaStream_t st) {
-    small_kernel<M><<<kSmCluster, kSmThreads, sizeof(SmallShared<M>), st>>>(s, part, i);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
+    ClusterLaunch c(kClusterMax, kSmThreads, sizeof(SmallShared<M>), kClusterMax, st);
+    MCTDHB_CUDA_TRY(cudaLaunchKernelEx(&c.cfg, small_kernel<M>, s, part, i));
     return 0;
 }
 
 template <int M>
 int small_batch_tmpl(const BatchSlot* slots, const int* list, const int* nlist, int nslots,
-                     int part, cudaStream_t st) {
-    small_batch_kernel<M><<<nslots * kSmCluster, kSmThreads, sizeof(SmallShared<M>), st>>>(
-        slots, list, nlist, part);
-    MCTDHB_CUDA_TRY(cudaGetLastError());
+                     int part, int blocks, cudaStream_t st) {
+    ClusterLaunch c(nslots * blocks, kSmThreads, sizeof(SmallShared<M>), blocks, st);
+    MCTDHB_CUDA_TRY(cudaLaunchKernelEx(&c.cfg, small_batch_kernel<M>, slots, list, nlist, part));
     return 0;
 }
 

@@ -48,7 +48,8 @@ int small_launch(const SmallSys& s, int part, int i, cudaStream_t st);
 // a part of the step of the batched slots of orbital count M in the list
 // (count in *nlist, at most nslots)
 int small_batch_launch(int M, const BatchSlot* slots, const int* list, const int* nlist,
-                       int nslots, int part, cudaStream_t st);
+                       int nslots, int part, int blocks, cudaStream_t st);
 int small_prepare(int M);  // launch attributes (before any stream capture)
+int small_waves(int M, int (&at)[kClusterSizes]);  // clusters that run at a time
 
 }  // namespace mctdhb

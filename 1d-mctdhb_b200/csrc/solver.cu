@@ -143,7 +143,7 @@ int upload_slots(mctdhb_solver_s* s) {
 // one launch of the cluster kernel on view v
 int cluster_step(mctdhb_solver_s* s, int v, int parts, cudaStream_t st) {
     const int* l = s->d_list + 2 * v;
-    return orb_step_launch(s->d_slot, l + 1, l, 1, parts, nullptr, st);
+    return orb_step_launch(s->d_slot, l + 1, l, 1, parts, nullptr, 0, st);
 }
 
 // phase 0 (orbital_integration.c:284-349): orbitals advanced with the
