@@ -812,7 +812,7 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     h.off = off;
     h.bytes = L.total;
     h.L = L;
-    h.small = small_eligible(job->npar, job->norb, L.D2);
+    h.small = small_eligible(job->npar, job->norb, L.D2, kSmallSlotMacs);
     const int N = job->npar, M = job->norb, G = job->grid_size;
     const size_t n = (size_t)M * G;
     char* base = b->arena + off;

@@ -412,8 +412,11 @@ int lanczos_fetch(const LanczosWork& w, int m, int* iters, double2* diag, double
 int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 prop_dt,
              int imagtime, cudaStream_t st) {
     const uint32_t n = s.dim;
-    if (m <= kBatchMaxLz && s.view.pair_y != nullptr &&
-        small_eligible(s.N, s.M, s.view.dim2)) {
+    if (m < 1 || m > w.mmax) {
+        set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
+        return -1;
+    }
+    if (m <= kBatchMaxLz && small_step(s.view)) {
         SmallSys y{};
         y.sp = s.view;
         y.C = d_C;
@@ -433,10 +436,6 @@ int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 pro
                 (i < m - 1 && small_launch(y, kSmallOrth, i, st)))
                 return -1;
         return small_launch(y, kSmallCombine, 0, st);
-    }
-    if (m < 1 || m > w.mmax) {
-        set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
-        return -1;
     }
     if (lanczos_from(s, w, d_C, m, st)) return -1;
     lz_small_kernel<<<1, 32, kSmallSmem, st>>>(imagtime ? 2 : 0, prop_dt, w.scal, w.iflag,

@@ -7,16 +7,28 @@
 
 namespace mctdhb {
 
-// Spaces this path takes: 2..8 orbitals, N >= 2, and a contraction of at most
-// so many complex multiply-adds (rows of the (N-2)-space times pairs^2): one
-// product is two cluster-wide passes on eight SMs, which save launches; beyond,
-// the whole GPU's tensor cores win.  Measured on one B200:
-//   one product   0.02 M (N=10 M=4)  8.4 us against 12.0 us; 0.23 M (N=24 M=4)
-//                 level; 0.45 M (N=30 M=4) 16.7 us against 13 us
-//   a Lanczos iteration adds 6 us here and 12 us of launches there: level at
-//                 0.7-0.9 M (N=11 M=6, N=16 M=5: a product takes 19-22 us)
-constexpr double kSmallHcMacs = 2.5e5, kSmallStepMacs = 7e5;
-bool small_eligible(int N, int M, uint32_t D2, double macs = kSmallStepMacs);
+// Spaces this path takes: 2..8 orbitals, N >= 2.  One product is two
+// cluster-wide passes on eight SMs, which save launches; beyond, the whole GPU's
+// tensor cores win.  Measured on one B200, here against the general path:
+//   one product, up to 0.25 M complex multiply-adds of the contraction (rows of
+//     the (N-2)-space times pairs^2): 0.02 M (N=10 M=4)  8.4 us against 12.0;
+//     0.23 M (N=24 M=4) level; 0.45 M (N=30 M=4) 16.7 against 13
+//   a step of one system (5 vectors, with densities), up to 2,048 rows, one a
+//     thread: 1,501 rows (N=1500 M=2) 82 us against 86; 1,716 (N=6 M=8) 145
+//     against 158; 1,891 (N=60 M=3) 92 against 95; 2,380 (N=13 M=5) 137 against
+//     127; 4,845 (N=16 M=5) 185 against 121; 18,336 (N=190 M=3) 230 against 111
+//   a slot of the batch, where the general path's iteration has twice the
+//     launches, up to 0.7 M: 0.69 M (N=16 M=5) 2 / 32 / 128 / 256 jobs 281 /
+//     387 / 1,174 / 2,283 us against 392 / 504 / 1,130 / 2,022; 0.43 M (N=6 M=8)
+//     363 / 526 / 1,552 / 3,039 against 496 / 625 / 1,403 / 2,542; the path
+//     follows (N, M) alone, for a job's bits
+constexpr double kSmallHcMacs = 2.5e5, kSmallSlotMacs = 7e5;
+constexpr uint32_t kSmallStepRows = 2048;
+bool small_eligible(int N, int M, uint32_t D2, double macs);
+inline bool small_step(const SpaceView& sp) {
+    return sp.pair_y != nullptr && sp.dim <= kSmallStepRows &&
+           small_eligible(sp.N, sp.M, sp.dim2, kSmallSlotMacs);
+}
 
 // what one system's step works on; every pointer is device memory
 struct SmallSys {
