@@ -655,19 +655,56 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
         // has to do: every row of H.C that reads one of them is NaN, and with it
         // the dots of a Lanczos step and all that follows.  A producer that
         // lost one stops, and its consumers run out.
-        // Where the loss is dealt with changes the code the compiler makes of
-        // the consumers' loop: at 7 orbitals in the loop (N=25 M=7: 165 us of
-        // H.C, 170 us after it), else after it (N=30 M=8: 2,955 us, 3,048 us in
-        // the loop; 2,932 us with no NaN and no vote at all).
-        constexpr bool IN_LOOP = M == 7;
         const int w = producer ? pt >> 5 : (t >> 5) / S::CPP;
         const uint32_t nchunk = (sp.dim2 + 31) / 32, step = gridDim.x * S::PW;
         double2* ring = Ab + w * 2 * 32 * PS;
         const uint32_t c0 = blockIdx.x + w * gridDim.x;
+        if constexpr (S::CREG > 0) {
+            // Five and six orbitals: with a real W the consumers need neither
+            // the A sums nor the third product and the producers set the pace,
+            // so the registers stay as launched (N=60 M=6, H.C with a real W:
+            // 1,222 us with the split, 1,168 us without).
+            auto run = [&](auto real_w) {
+                constexpr bool RE = decltype(real_w)::value;
+                int i = 0;
+                bool ok = true;
+                if (producer) {
+                    if constexpr (!RE) pair_regs_dec<S::CREG, S::PREG>();
+                    for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
+                        const int buf = i & 1;
+                        if (i >= 2) ok = mbar_wait<NOWAIT>(&empty[w][buf], ((i >> 1) - 1) & 1);
+                        if (!ok) return;
+                        pair_gather_row<M, V>(tv, C, c * 32 + lane, ring + buf * 32 * PS, lane);
+                        mbar_arrive(&full[w][buf]);
+                    }
+                } else {
+                    if constexpr (!RE) pair_regs_inc<S::CREG>();
+                    for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
+                        const int buf = i & 1;
+                        ok = mbar_wait<NOWAIT>(&full[w][buf], (i >> 1) & 1);
+                        pair_strips<M, V>(ring + buf * 32 * PS, Ws, (t >> 5) % S::CPP, S::CPP, 2,
+                                          lane, c * 32, sp.dim2, sp.ldy, Y, RE);
+                        mbar_arrive(&empty[w][buf]);
+                        ok = __all_sync(0xffffffffu, ok);
+                    }
+                    if (!ok) pair_poison<M>(c0 + (i - 1) * step, step, nchunk, lane, sp, Y);
+                }
+            };
+            if (real)
+                run(std::true_type{});
+            else
+                run(std::false_type{});
+            return;
+        }
+        // Where the loss is dealt with changes the code the compiler makes of
+        // the consumers' loop: at 7 orbitals in the loop (N=25 M=7: 166 us of
+        // H.C, 170 us after it), else after it (N=30 M=8: 2,956 us, 3,048 us in
+        // the loop; 2,932 us with no NaN and no vote at all; 3,030 us in a lambda
+        // as above).
+        constexpr bool IN_LOOP = M == 7;
         int i = 0;
         bool ok = true;
         if (producer) {
-            pair_regs_dec<S::CREG, S::PREG>();
             for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
                 const int buf = i & 1;
                 if (i >= 2) ok = mbar_wait<NOWAIT>(&empty[w][buf], ((i >> 1) - 1) & 1);
@@ -676,7 +713,6 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
                 mbar_arrive(&full[w][buf]);
             }
         } else {
-            pair_regs_inc<S::CREG>();
             for (uint32_t c = c0; c < nchunk && ok; c += step, i++) {
                 const int buf = i & 1;
                 ok = mbar_wait<NOWAIT>(&full[w][buf], (i >> 1) & 1);
