@@ -557,9 +557,18 @@ int batch_tune_launch(void* p, int v, cudaStream_t st) {
 
 int tune_group(mctdhb_batch_s* b, int M) {
     if (b->pair_v_forced[M]) return 0;
+    // Jobs in real time have a complex W from their first step on, whatever the
+    // orbitals they came with: their real-W flags are off while it tunes (every
+    // step forms W and flag anew before it reads them).
     uint64_t rows = 0;
-    for (const HostSlot& h : b->hs)
-        if (h.used && h.running && !h.small && h.d.M == M) rows += h.L.D2;
+    for (const HostSlot& h : b->hs) {
+        if (!h.used || !h.running || h.small || h.d.M != M) continue;
+        rows += h.L.D2;
+        const int P = M * (M + 1) / 2;
+        if (!h.d.imag)
+            MCTDHB_CUDA_TRY(
+                cudaMemsetAsync(h.d.sp.pair_w + P * P, 0, sizeof(double2), b->st));
+    }
     int bucket = 0;
     while ((1ull << bucket) < rows) bucket++;
     BatchTuneCtx ctx{b, M};

@@ -23,6 +23,7 @@
 #include "engine.h"
 #include "kernels.h"
 #include "moves.cuh"
+#include "smallsys.h"
 
 namespace mctdhb {
 
@@ -200,9 +201,11 @@ int mctdhb_step_create(mctdhb_space h, void* d_coef, void* d_rho1, void* d_rho2,
     cudaStream_t cs;
     MCTDHB_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     {
-        // pick the launch variants now: a capture cannot time launches
+        // pick the launch variants now: a capture cannot time launches (a
+        // small space's step launches none of them)
         HcEpilogue ep;
-        hc_variant(h->sp.view, (const double2*)d_coef, h->lw.out, h->sp.d_tab, ep, cs);
+        if (!sil_small(h->sp.view, m))
+            hc_variant(h->sp.view, (const double2*)d_coef, h->lw.out, h->sp.d_tab, ep, cs);
         if (dens_prepare(h->sp.view, (const double2*)d_coef, h->sp.d_dens_part, cs)) {
             cudaStreamDestroy(cs);
             return -1;

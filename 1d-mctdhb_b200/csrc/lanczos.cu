@@ -416,7 +416,7 @@ int sil_step(const SpaceCtx& s, LanczosWork& w, double2* d_C, int m, double2 pro
         set_error("Lanczos dimension %d outside 1..%d", m, w.mmax);
         return -1;
     }
-    if (m <= kBatchMaxLz && small_step(s.view)) {
+    if (sil_small(s.view, m)) {
         SmallSys y{};
         y.sp = s.view;
         y.C = d_C;

@@ -25,8 +25,9 @@ namespace mctdhb {
 constexpr double kSmallHcMacs = 2.5e5, kSmallSlotMacs = 7e5;
 constexpr uint32_t kSmallStepRows = 2048;
 bool small_eligible(int N, int M, uint32_t D2, double macs);
-inline bool small_step(const SpaceView& sp) {
-    return sp.pair_y != nullptr && sp.dim <= kSmallStepRows &&
+// whether a step of one system with m Lanczos vectors runs here
+inline bool sil_small(const SpaceView& sp, int m) {
+    return m <= kBatchMaxLz && sp.pair_y != nullptr && sp.dim <= kSmallStepRows &&
            small_eligible(sp.N, sp.M, sp.dim2, kSmallSlotMacs);
 }
 

@@ -19,6 +19,7 @@
 #include "kernels.h"
 #include "orbital.h"
 #include "orbstep.cuh"
+#include "smallsys.h"
 
 using namespace mctdhb;
 
@@ -564,8 +565,25 @@ int mctdhb_solver_set_state(mctdhb_solver s, const void* orb, const void* coef) 
     if (orb_matrices(s->orb, s->d_orb, s->d_hob, s->d_hint, st)) return -1;
     if (s->M > 1) {
         if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st, false)) return -1;
-        HcEpilogue ep;  // tune H.C on this state before the graph is captured
-        hc_variant(sc.view, s->d_coef, s->sp->lw.out, sc.d_tab, ep, st);
+        // Tune H.C on this state before the graph is captured, unless neither
+        // a Lanczos nor a Runge-Kutta step of this space launches the tuned
+        // kernel.  In real time W is complex from the first step on, whatever
+        // the orbitals here, and the variants differ (N=30 M=8, H.C: real W
+        // 2,529 us by variant 0, 2,646 by 3; complex 3,202 and 2,952): there
+        // the real-W flag is off while it tunes.
+        const SpaceView& v = sc.view;
+        const bool pair = v.pair_y != nullptr && s->M <= kMaxTemplOrb;
+        if (!pair || !sil_small(v, s->lanczos_m) ||
+            !small_eligible(s->N, s->M, v.dim2, kSmallHcMacs)) {
+            const int P = s->M * (s->M + 1) / 2;
+            if (pair && !s->imagtime)
+                MCTDHB_CUDA_TRY(cudaMemsetAsync(v.pair_w + P * P, 0, sizeof(double2), st));
+            HcEpilogue ep;
+            hc_variant(v, s->d_coef, s->sp->lw.out, sc.d_tab, ep, st);
+            if (pair && !s->imagtime &&
+                hc_prep(v, s->d_hob, s->d_hint, sc.d_tab, st, false))
+                return -1;
+        }
     }
     MCTDHB_CUDA_TRY(cudaStreamSynchronize(st));
     s->has_state = true;
