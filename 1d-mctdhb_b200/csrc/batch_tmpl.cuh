@@ -87,7 +87,11 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
         };
         auto give_up = [&](int slot) {
             const BatchSlot& S = slots[slot];
-            if (lane == 0 && bt_hc_active(S, iter)) S.flags[BF_STATE] = SLOT_ABORTED;
+            if (lane != 0 || !bt_hc_active(S, iter)) return;
+            if (S.flags[BF_STATE] == SLOT_RUNNING) S.flags[BF_STATE] = SLOT_ABORTED;
+            // the monitor's product (the job may have ended in this step): no
+            // residual of it, so the stop rule does not pass on old rows
+            if (iter == kBatchMonIter) S.flags[BF_MON] = 0;
         };
         const int w = t >= PS_::CONSUMERS ? pt >> 5 : (t >> 5) / PS_::CPP;
         double2* ring = Ab + w * 2 * 32 * PS;
