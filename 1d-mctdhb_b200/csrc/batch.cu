@@ -49,11 +49,11 @@ size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
 // sizes of one job's parts, in the arena order
 struct JobLayout {
-    uint32_t nc = 0, D1 = 0, D2 = 0;
-    int vtiles = 0, ytiles = 0, gs[3] = {0, 0, 0}, gk[3] = {0, 0, 0};
+    uint32_t nc = 0, D2 = 0;
+    int vtiles = 0, ytiles = 0, gs = 0, gk = 0;
     size_t o_orb, o_stage, o_H, o_pot, o_w, o_hob, o_hint, o_pw, o_lint, o_rho1, o_rho2,
         o_rinv,
-        o_T, o_sq, o_g, o_V, o_out, o_part, o_py, o_gpart, o_half, o_B, total;
+        o_T, o_sq, o_g, o_V, o_out, o_part, o_py, o_gpart, o_half, total;
 };
 
 // der: 0 / 302 finite differences, 300 DVR, 301 spectral (periodic only);
@@ -87,7 +87,6 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
         return -1;
     }
     L.nc = (uint32_t)dim;
-    L.D1 = (uint32_t)fock_dimension(N - 1, M);
     L.D2 = (uint32_t)fock_dimension(N - 2, M);
     L.vtiles = (int)((dim + kBatchVecRows - 1) / kBatchVecRows);
     L.ytiles = (int)((L.D2 + batch_pair_rows(M) - 1) / batch_pair_rows(M));
@@ -95,8 +94,8 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     // follows from rho2: no rho1 Gram pass)
     {
         const uint64_t ntr = (L.D2 + gram_rows(M) - 1) / gram_rows(M);
-        L.gk[2] = (int)std::max<uint64_t>(1, (ntr + kBatchMaxSlices - 1) / kBatchMaxSlices);
-        L.gs[2] = (int)((ntr + L.gk[2] - 1) / L.gk[2]);
+        L.gk = (int)std::max<uint64_t>(1, (ntr + kBatchMaxSlices - 1) / kBatchMaxSlices);
+        L.gs = (int)((ntr + L.gk - 1) / L.gk);
     }
     const size_t n = (size_t)M * G, M2 = (size_t)M * M, M4 = M2 * M2, z = sizeof(double2);
     const size_t P = (size_t)M * (M + 1) / 2;
@@ -125,7 +124,7 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
     L.o_out = take((size_t)dim * z);
     L.o_part = take((size_t)kBatchMaxLz * L.vtiles * z);
     L.o_py = take((size_t)pair_ld(L.D2) * P * z);
-    L.o_gpart = take((size_t)L.gs[2] * gram_entries(M) * z);
+    L.o_gpart = take((size_t)L.gs * gram_entries(M) * z);
     if (split && !periodic && der != 0 && der != kDerFiniteDiff) {
         set_error("batch: the split step's FFT exponential needs periodic boundaries");
         return -1;
@@ -135,7 +134,6 @@ int job_layout(int N, int M, int G, int lz, int der, int periodic, int split, Jo
         return -1;
     }
     L.o_half = take(split ? (periodic ? 2 * (size_t)(G - 1) - 1 : (size_t)G * G) * z : 0);
-    L.o_B = take(split ? M2 * z : 0);
     L.total = o;
     return 0;
 }
@@ -301,7 +299,7 @@ int rebuild_lists(mctdhb_batch_s* b) {
                 };
                 for (uint32_t r = 0; r < h.L.nc; r += kBatchHcRows) push(LIST_HG, r);
                 for (int t = 0; t < h.L.ytiles; t++) push(LIST_HY, (uint32_t)t);
-                for (int g = 0; g < h.L.gs[2]; g++) push(LIST_G2, (uint32_t)g);
+                for (int g = 0; g < h.L.gs; g++) push(LIST_G2, (uint32_t)g);
             }
         };
         push_slots(1);
@@ -838,11 +836,8 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     d.max_steps = job->max_steps;
     d.vtiles = L.vtiles;
     d.ytiles = L.ytiles;
-    for (int R = 0; R < 3; R++) {
-        d.gs[R] = L.gs[R];
-        d.gk[R] = L.gk[R];
-    }
-    d.D1 = L.D1;
+    d.gs = L.gs;
+    d.gk = L.gk;
     d.dt = job->dt;
     d.etol = job->energy_tol;
     d.reg_fac = reg;
@@ -901,7 +896,6 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     d.split = split;
     d.half_dense = 0;
     d.half = split ? (const double2*)P(L.o_half) : nullptr;
-    d.B = split ? (double2*)P(L.o_B) : nullptr;
     if (split && split_half_operator(G, d.ov.dx, d.ov.a2, d.ov.a1, d.ov.periodic,
                                      job->der_method == 0 ? kDerFiniteDiff : job->der_method,
                                      job->dt, d.imag, half, &d.half_dense)) {
@@ -948,8 +942,8 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     hp[1] = s;
     int* pc = hp + 2;
     batch_offs(pc, LIST_G2)[M] = 0;
-    batch_cnts(pc, LIST_G2)[M] = L.gs[2];
-    for (int q = 0; q < L.gs[2]; q++) b->h_pro_g[q] = BatchTile{s, (uint32_t)q};
+    batch_cnts(pc, LIST_G2)[M] = L.gs;
+    for (int q = 0; q < L.gs; q++) b->h_pro_g[q] = BatchTile{s, (uint32_t)q};
     const int* pl = b->d_pro;
     const int* dpc = b->d_pro + 2;
     if (cudaMemcpyAsync(b->d_pro, hp, (2 + kCntInts) * sizeof(int), cudaMemcpyHostToDevice, st) ||

@@ -82,8 +82,7 @@ constexpr int BS_Y = 3 * kBatchMaxLz;
 // [5] overlap residual of the orbitals (real time), [6] eigen residual
 // max_i |E C_i - (H C)_i| / N at its last evaluation (imaginary time)
 constexpr int BS_MISC = 4 * kBatchMaxLz;
-constexpr int BS_Z = BS_MISC + 8;  // kBatchMaxLz^2 doubles of eigenvectors
-constexpr int BS_TOTAL = BS_Z + kBatchMaxLz * kBatchMaxLz / 2;
+constexpr int BS_TOTAL = BS_MISC + 8;
 
 // per-slot device flags (ints)
 constexpr int BF_BREAK = 0;  // Lanczos breakdown in this step
@@ -100,7 +99,7 @@ constexpr int BF_TOTAL = 10;
 
 // SLOT_ABORTED: real time, overlap residual above the reference's critical
 // value (REALTIME_OVERLAP_RESIDUE_TOL, driver.c:89-95, where the reference
-// exits; the engine stops that job alone)
+// exits; the engine stops that job alone); or a lost handover (batch_tmpl.cuh)
 constexpr int SLOT_EMPTY = 0, SLOT_RUNNING = 1, SLOT_DONE = 2, SLOT_ABORTED = 3;
 constexpr double kOverlapAbort = 1e-3;     // REALTIME_OVERLAP_RESIDUE_TOL (driver.h:7)
 constexpr double kOrthoSwitch = 1e-8;      // threshold_impr_ortho (driver.c:19)
@@ -110,10 +109,7 @@ struct BatchSlot {
     uint32_t nc, max_steps;
     int vtiles;   // ceil(nc / kBatchVecRows)
     int ytiles;   // tiles of the (N-2)-boson space of the pair-space H.C
-    int gs[3];    // rho2 Gram slices of the (N-2)-boson space at index 2 (1 unused)
-    int gk[3];    // row tiles per Gram slice, index 2
-    uint32_t D1;  // D(N-1, M); D(N-2, M) is sp.dim2
-    int pad1;
+    int gs, gk;   // rho2 Gram slices of the (N-2)-boson space, row tiles per slice
     double dt, etol, reg_fac;
     double eig_tol;    // eigen-residual half of the imaginary-time stop rule (0: off)
     double ortho_tol;  // real time: overlap residual that switches the robust projector on
@@ -126,12 +122,11 @@ struct BatchSlot {
     double2 *V;          // lz x nc Krylov vectors; V[0] holds the coefficients
     // split step (split: 1): the half-step operator (orbital.h,
     // split_half_operator; dense: column-major G x G, else the circulant
-    // kernel of the G - 1 periodic points) and the M x M projection B
+    // kernel of the G - 1 periodic points)
     int split, half_dense;
     const double2* half;
-    double2* B;
     double2 *out, *part;
-    double2* gpart;      // rho2 Gram partials: gs[2] slices
+    double2* gpart;      // rho2 Gram partials: gs slices
     double2* scal;       // BS_TOTAL
     int* flags;          // BF_TOTAL
 };

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kBatchHcRows)
     }
 }
 
-// rho2 Gram partial of slice `idx` of a slot: its gk[2] consecutive row
+// rho2 Gram partial of slice `idx` of a slot: its gk consecutive row
 // tiles of the (N-2)-boson space, summed into gpart (gram_tmpl.cuh building
 // blocks)
 template <int M>
@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(kGramThreads, 2)
         if (S.flags[BF_STATE] != SLOT_RUNNING) continue;  // block-uniform
         const uint32_t Dp = S.sp.dim2;
         const uint32_t ntr = (Dp + GS::ROWS - 1) / GS::ROWS;
-        const uint32_t t0 = tl.idx * (uint32_t)S.gk[2];
-        const uint32_t t1 = min(t0 + (uint32_t)S.gk[2], ntr);
+        const uint32_t t0 = tl.idx * (uint32_t)S.gk;
+        const uint32_t t1 = min(t0 + (uint32_t)S.gk, ntr);
         acc.clear();
         for (uint32_t tr = t0; tr < t1; tr++) {
             gram_gather<M>(S.sp, Dp, S.V, tr, As, threadIdx.x);
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kBatchVecThreads)
     if (S.M != M || S.flags[BF_STATE] != SLOT_RUNNING) return;  // block-uniform
     constexpr int ENT = gram_entries(M);
     const int e = blockIdx.y * 32 + (threadIdx.x & 31);
-    const double2 v = gram_sum_parts(S.gpart + e, S.gs[2], ENT, e < ENT);
+    const double2 v = gram_sum_parts(S.gpart + e, S.gs, ENT, e < ENT);
     if (threadIdx.x < 32 && e < ENT) gram_fill<M>(e, v, S.rho2);
 }
 

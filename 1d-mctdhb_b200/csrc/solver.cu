@@ -126,7 +126,6 @@ int upload_slots(mctdhb_solver_s* s) {
     d.split = o.split;
     d.half_dense = o.half_dense;
     d.half = o.d_half;
-    d.B = o.d_B;
     d.scal = s->d_scal;
     d.flags = s->d_flags;
     h[1] = d;
