@@ -142,6 +142,7 @@ struct HostSlot {
     bool used = false;
     bool running = false;
     bool small = false;  // steps on the small-space path (smallsys.h)
+    bool real_w = false;  // W stays real (stays_real)
     size_t off = 0, bytes = 0;
     BatchSlot d{};
     JobLayout L{};
@@ -555,15 +556,15 @@ int batch_tune_launch(void* p, int v, cudaStream_t st) {
 
 int tune_group(mctdhb_batch_s* b, int M) {
     if (b->pair_v_forced[M]) return 0;
-    // Jobs in real time have a complex W from their first step on, whatever the
-    // orbitals they came with: their real-W flags are off while it tunes (every
-    // step forms W and flag anew before it reads them).
+    // Most jobs have a complex W from their first step on, whatever the orbitals
+    // they came with (stays_real): their real-W flags are off while it tunes
+    // (every step forms W and flag anew before it reads them).
     uint64_t rows = 0;
     for (const HostSlot& h : b->hs) {
         if (!h.used || !h.running || h.small || h.d.M != M) continue;
         rows += h.L.D2;
         const int P = M * (M + 1) / 2;
-        if (!h.d.imag)
+        if (!h.real_w)
             MCTDHB_CUDA_TRY(
                 cudaMemsetAsync(h.d.sp.pair_w + P * P, 0, sizeof(double2), b->st));
     }
@@ -820,6 +821,9 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
     h.bytes = L.total;
     h.L = L;
     h.small = small_eligible(job->npar, job->norb, L.D2, kSmallSlotMacs);
+    h.real_w = !h.small &&
+               stays_real(job->imagtime, (const double2*)job->orbitals,
+                          (size_t)job->norb * job->grid_size, (const double2*)job->coef, L.nc);
     const int N = job->npar, M = job->norb, G = job->grid_size;
     const size_t n = (size_t)M * G;
     char* base = b->arena + off;

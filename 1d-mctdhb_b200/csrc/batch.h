@@ -194,8 +194,8 @@ int batch_prepare();
 // energy, the counters and the wanted arrays (n[a] = 0: not wanted) behind one
 // another into pinned host memory, from where the host hands them out.  Six
 // copies to pageable memory, each with its own wait, took 31 us for a small
-// job; this takes 10 us (32 jobs of N=2..10, 4 steps and a fetch each: 2,759 to
-// 2,082 us).  Above kFetchWords the copies stay with the copy engine.
+// job; this takes 10 us (32 jobs of N=10..24 in 3 and 4 orbitals, 4 steps and a
+// fetch each: 2,759 to 2,082 us).  Above kFetchWords the copies stay with the copy engine.
 constexpr int kFetchHead = 2;
 constexpr size_t kFetchWords = 16384;  // 256 KB
 struct BatchFetch {

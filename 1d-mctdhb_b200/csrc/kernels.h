@@ -159,9 +159,9 @@ template <int M>
 int gram_prepare_tmpl();
 
 // Launch variants of the pair contraction (pairhc_tmpl.cuh, PairHcShape):
-// 0 the default tile, 1 half the rows per tile (up to 6 orbitals), 2 the
-// other output-tile grouping per pass (6 orbitals and more; below, it is
-// the default grouping), 3 variant 0's tiles handed over through mbarriers
+// 0 the default tile, 1 half the rows per tile (up to 6 orbitals), 2 two
+// output tiles at a time (6 orbitals and more), 3 chunks of 32 rows from a
+// producer warp to its consumer warps through mbarriers
 __host__ __device__ constexpr bool pair_variant_ok(int M, int V) {
     return V == 0 || V == 3 || (V == 1 && M * (M + 1) / 2 <= 21) ||
            (V == 2 && M * (M + 1) / 2 > 16);

@@ -10,7 +10,7 @@
 //                 b_i / max b < 1e-14;  v_{i+1} = out / b_i;
 //                 out = H v_{i+1} - b_i v_i;  a_{i+1} = <v_{i+1}, out>
 // then the m x m tridiagonal eigenproblem (implicit QL with Wilkinson
-// shifts, the EISPACK tql2 scheme, in place of LAPACK dstev), the
+// shifts, the EISPACK imtql2 scheme, in place of LAPACK dstev), the
 // propagator y = U exp(-i D dt) U^T e1 and C = sum_j y_j v_j.
 // Every scalar (a, b, o, y, the breakdown flag and iteration count) lives
 // in device memory, so a step is a fixed launch sequence with no host

@@ -87,6 +87,18 @@ int split_half_operator(int G, double dx, double a2, double2 a1, int periodic, i
 // g of the half-stepped orbitals into hob / hint, and RK of the nonlinear part
 int orb_split_step(OrbCtx& c, int order, double dt, const double2* rinv, const double2* rho2,
                    double2* y, double2* ynext, double2* hob, double2* hint, cudaStream_t st);
+// whether the pair matrix of a system stays real, for the tuner: imaginary time,
+// real orbitals (n values, host) and real coefficients (nc values, host, as far
+// as the first 65,536 tell)
+inline bool stays_real(int imagtime, const double2* orb, size_t n, const double2* coef,
+                       size_t nc) {
+    if (!imagtime) return false;
+    for (size_t i = 0; i < n; i++)
+        if (orb[i].y != 0.0) return false;
+    for (size_t i = 0; i < nc && i < 65536; i++)
+        if (coef[i].y != 0.0) return false;
+    return true;
+}
 // the half-step operator applied to every orbital of y into out (not y)
 int orb_half_step(const OrbCtx& c, const double2* y, double2* out, cudaStream_t st);
 // S_sl = <f_s|f_l> (Simpson) into c.d_S

@@ -1,12 +1,13 @@
-// orbstep.cu -- the orbital side of a step, one cluster of eight blocks per
-// system (orbstep.cuh).
+// orbstep.cu -- the orbital side of a step, one cluster of blocks per system
+// (orbstep.cuh): eight for one system, 8, 4, 2 or 1 for a slot of the batch
+// (batch.h, cluster_blocks).
 //
 // What bounds it.  The work of a system is small (M=6 on 1024 points: 6 stages
 // of 3.6 M FP64 FMAs) and every stage needs the whole previous one, so the
 // time is latency: barriers, dependent sums, too few threads.  One block per
 // system took 1,980 us at M=6 on 1024 points (RK5 step with Gram-Schmidt and
 // matrices), this kernel takes 170 us; alone, the solver's chain of 30 small
-// launches took 190 us at M=4 on 256 points and takes 75 us.  Eight blocks share the
+// launches took 190 us at M=4 on 256 points and takes 75 us.  The blocks share the
 // points and meet at cluster barriers; every sum over the grid is cut into
 // pieces of 256 points (64 for g_ksql) that one warp adds, and the pieces are
 // added in order, so a value depends on the system alone.  Work taken out: the

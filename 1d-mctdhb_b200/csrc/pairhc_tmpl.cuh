@@ -622,8 +622,8 @@ __device__ __forceinline__ double2 pair_gather_back(const SpaceView& sp,
 // ---------------------------------------------------------------------------
 // single-system kernels
 // ---------------------------------------------------------------------------
-// Y = A W^T for the rows m of the (N-2)-boson space; Y[p * ldy + m] (planes
-// start on 128 bytes: a fragment's 8 rows are one line).  Warp-specialised and
+// Y = A W^T for the rows m of the (N-2)-boson space; Y[p * ldy + m] (planes an
+// odd number of rows apart, pair_ld).  Warp-specialised and
 // double-buffered: while the consumer warps contract rows from one A buffer,
 // the producer warps unrank and gather the next ones into the other.
 template <int M, int V, bool NOWAIT = false>

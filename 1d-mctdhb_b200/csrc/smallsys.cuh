@@ -1,13 +1,15 @@
-// smallsys.cuh -- one cluster of eight blocks per small system (smallsys.h;
-// explicit instantiations in small_m*.cu).
+// smallsys.cuh -- one cluster of blocks per small system (smallsys.h; explicit
+// instantiations in small_m*.cu): eight blocks for one system, 8, 4, 2 or 1 for
+// a slot of the batch (batch.h, cluster_blocks).
 //
 // The general path spends a small space's time in launches: a Lanczos
-// iteration is nine of them, 3 us each, for vectors of a few hundred to a few
-// thousand rows.  Here a thread owns rows, vectors stay where the thread that
-// wrote them reads them again, and a step is a fixed chain of passes over the
-// cluster's 2,048 threads with a cluster barrier between two: the contraction
-// Y = W A (a thread per row of the (N-2)-space and group of output pairs, W in
-// shared memory), the gather-back with the dot product, the dots of the
+// iteration is four of them (nine in the batch), 3 us each, for vectors of a few
+// hundred to a few thousand rows.  Here a thread owns rows; vectors, Krylov
+// vectors and Y are in global memory, where the thread that wrote a row reads it
+// again from its L1, and a step is a fixed chain of passes over 2,048 numbered
+// threads with a cluster barrier between two: the contraction
+// Y = W A (a thread per row of the (N-2)-space and group of output pairs; W, the
+// rank tables and the pieces of sums are in shared memory), the gather-back with the dot product, the dots of the
 // reorthogonalisation, its subtraction with the norm, and the scaling.  A
 // thread's sums over its rows stay in its registers.  Sums:
 // rows of a thread in order, the 32 threads of a warp by a butterfly, the 64
@@ -195,8 +197,9 @@ struct SmallRun : SmallSize<B> {
     }
 
     // The Lanczos recurrence (multiconfig_lanczos.c:12-90), the operations of
-    // lanczos_run, in two passes an iteration that meet in global memory, so
-    // they run as one kernel or as one each with the same bits.
+    // lanczos_run, in two passes an iteration that meet in global memory: the
+    // whole recurrence is one launch for a slot of the batch, each pass one for a
+    // single system.
     // product(i):  v_i = out / beta_{i-1}, out = H v_i - beta_{i-1} v_{i-1},
     //              alpha_i = <v_i, out>
     __device__ __forceinline__ double2 product(int i) {

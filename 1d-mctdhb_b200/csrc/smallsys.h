@@ -1,5 +1,7 @@
-// smallsys.h -- H.C, the short iterative Lanczos step and the densities of a
-// small Fock space in one launch (smallsys.cuh).
+// smallsys.h -- H.C and the short iterative Lanczos step of a small Fock space on
+// one cluster of blocks (smallsys.cuh): H.C in one launch; a step of one system in
+// two an iteration and one for the combination (its densities take the Gram
+// kernels); in the batch the recurrence, the combination and rho2 in one each.
 #pragma once
 #include "batch.h"
 #include "common.cuh"

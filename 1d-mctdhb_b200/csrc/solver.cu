@@ -566,22 +566,22 @@ int mctdhb_solver_set_state(mctdhb_solver s, const void* orb, const void* coef) 
         if (hc_prep(sc.view, s->d_hob, s->d_hint, sc.d_tab, st, false)) return -1;
         // Tune H.C on this state before the graph is captured, unless neither
         // a Lanczos nor a Runge-Kutta step of this space launches the tuned
-        // kernel.  In real time W is complex from the first step on, whatever
-        // the orbitals here, and the variants differ (N=30 M=8, H.C: real W
-        // 2,529 us by variant 0, 2,646 by 3; complex 3,202 and 2,952): there
-        // the real-W flag is off while it tunes.
+        // kernel.  W is complex from the first step on unless time is imaginary
+        // and orbitals and coefficients are real, and the variants differ (N=30
+        // M=8, H.C: real W 2,529 us by variant 0, 2,646 by 3; complex 3,202 and
+        // 2,952): there the real-W flag is off while it tunes.
         const SpaceView& v = sc.view;
         const bool pair = v.pair_y != nullptr && s->M <= kMaxTemplOrb;
         if (!pair || !sil_small(v, s->lanczos_m) ||
             !small_eligible(s->N, s->M, v.dim2, kSmallHcMacs)) {
             const int P = s->M * (s->M + 1) / 2;
-            if (pair && !s->imagtime)
+            const bool turns = pair && !stays_real(s->imagtime, (const double2*)orb, n,
+                                                   (const double2*)coef, nc);
+            if (turns)
                 MCTDHB_CUDA_TRY(cudaMemsetAsync(v.pair_w + P * P, 0, sizeof(double2), st));
             HcEpilogue ep;
             hc_variant(v, s->d_coef, s->sp->lw.out, sc.d_tab, ep, st);
-            if (pair && !s->imagtime &&
-                hc_prep(v, s->d_hob, s->d_hint, sc.d_tab, st, false))
-                return -1;
+            if (turns && hc_prep(v, s->d_hob, s->d_hint, sc.d_tab, st, false)) return -1;
         }
     }
     MCTDHB_CUDA_TRY(cudaStreamSynchronize(st));

@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(256)
     if (e == P * P) W[e] = make_double2(0.0, 0.0);
 }
 
-// Y[p * D2 + m]: ST strips of 16 rows a block (two up to 20 orbitals, where
-// two blocks fit an SM; one beyond, where the A tile of two strips takes over
-// 110 KB and at 29 orbitals no longer fits).  Warps take the output tiles of
+// Y[p * D2 + m]: ST strips of 16 rows a block (two up to 20 orbitals: two blocks
+// fit an SM up to 19; one beyond, where the A tile of two strips takes over
+// 118 KB and at 29 orbitals no longer fits).  Warps take the output tiles of
 // 8 pairs; a tile's W fragments come from L2 and serve every strip, with four
 // real products per complex one (the kernel waits on its gathers and W, not on
 // the tensor cores: the three-product form is no faster here).

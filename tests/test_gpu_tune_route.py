@@ -16,12 +16,14 @@ def dev(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
-def solver(gpu, dim, N, M, imag, G=64):
+def solver(gpu, dim, N, M, imag, G=64, real=False):
     orb, _ = hermite_orbitals(M, G, -8.0, 8.0)
+    c = rand_coef(np.random.default_rng(N), dim(N, M))
+    c = c.real / np.linalg.norm(c.real) + 0j if real else c
     s = gpu.Solver(N, M, G, -8.0, 8.0, 1e-3, imag, rk_order=4, lanczos_iter=5)
     s.set_potential(0.5 * np.linspace(-8, 8, G) ** 2)
     s.set_interaction(0.1)
-    s.set_state(orb, rand_coef(np.random.default_rng(N), dim(N, M)))
+    s.set_state(orb, c)
     return s
 
 
@@ -46,15 +48,24 @@ def test_small_spaces_are_not_tuned(gpu, oracle):
     step.close()
 
 
-def test_real_time_is_tuned_for_a_complex_w(gpu, oracle):
-    """22 bosons in 8 orbitals: variant 3 is 8 % ahead with a complex W, variant 0
-    4 % with a real one"""
-    N, M = 22, 8
-    s = solver(gpu, oracle.dim, N, M, False)
-    assert gpu.tune_get("hcp_y", N, M) == 3
-    # the flag is back: the energy of the state as the oracle has it
+@pytest.mark.parametrize("N,imag", [(22, False), (23, True)])
+def test_tuned_for_the_complex_w_that_comes(gpu, oracle, N, imag):
+    """8 orbitals: variant 3 is 8 % ahead with a complex W, variant 0 4 % with a
+    real one.  Real time, and imaginary time with complex coefficients"""
+    s = solver(gpu, oracle.dim, N, 8, imag)
+    assert gpu.tune_get("hcp_y", N, 8) == 3
     s.step(1)
     assert np.isfinite(s.get()["coef"]).all()
+
+
+def test_all_real_stays_real(gpu, oracle):
+    """imaginary time from real orbitals and coefficients: both stay real, and the
+    contraction is tuned with the real W it runs with"""
+    s = solver(gpu, oracle.dim, 21, 8, True, real=True)
+    assert gpu.tune_get("hcp_y", 21, 8) in (0, 2, 3)
+    s.step(2)
+    got = s.get()
+    assert not got["orb"].imag.any() and not got["coef"].imag.any()
 
 
 def test_batch_in_real_time_keeps_its_bits(gpu, oracle):
