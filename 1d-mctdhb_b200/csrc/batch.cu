@@ -333,7 +333,7 @@ int rebuild_lists(mctdhb_batch_s* b) {
                                             cudaMemcpyHostToDevice, st));
     b->present_mask = mask;
     b->small_mask = small;
-    if (b->orb_waves[0] == 0 && (orb_step_prepare() || orb_step_waves(b->orb_waves))) return -1;
+    if (b->orb_waves[0] == 0 && (orb_step_prepare(true) || orb_step_waves(b->orb_waves))) return -1;
     b->orb_blocks = cluster_blocks(b->orb_waves, list(0)[0]);
     // the small slots of all orbital counts run beside one another
     b->small_blocks = kClusterMax;
@@ -956,7 +956,7 @@ int mctdhb_batch_admit(mctdhb_batch b, const mctdhb_job* job, int* slot) {
         set_error("mctdhb_batch_admit: upload failed");
         return undo();
     }
-    if (prepare_group(M) || orb_step_prepare() ||
+    if (prepare_group(M) || orb_step_prepare(true) ||
         orb_step_launch(b->d_slots, pl + 1, pl, 1, kOrbMatrices, nullptr, kClusterMax, st) ||
         dens_group(M, b->d_slots, b->d_pro_g, dpc, pl + 1, pl, 1, st))
         return undo();
@@ -1219,6 +1219,11 @@ int mctdhb_batch_set_nowait(mctdhb_batch b, int on) {
         return -1;
     }
     std::lock_guard<std::mutex> lk(b->mu);
+    if (on && (batch_prepare_nowait<2>() || batch_prepare_nowait<3>() ||
+               batch_prepare_nowait<4>() || batch_prepare_nowait<5>() ||
+               batch_prepare_nowait<6>() || batch_prepare_nowait<7>() ||
+               batch_prepare_nowait<8>()))
+        return -1;
     b->nowait = on != 0;
     drop_graph(b);  // captured with the old launches
     return 0;

@@ -189,6 +189,8 @@ int gram_batch_launch(const BatchSlot* slots, const BatchTile* g2, const int* cn
                       const int* list, const int* nlist, int nblocks, cudaStream_t st);
 template <int M>
 int batch_prepare();
+template <int M>
+int batch_prepare_nowait();
 
 // A slot's results read to the host (mctdhb_batch_fetch): one launch writes the
 // energy, the counters and the wanted arrays (n[a] = 0: not wanted) behind one

@@ -6,4 +6,5 @@ template int hcp_batch_launch<2>(const BatchSlot*, const BatchTile*, const Batch
 template int gram_batch_launch<2>(const BatchSlot*, const BatchTile*, const int*, const int*,
                                   const int*, int, cudaStream_t);
 template int batch_prepare<2>();
+template int batch_prepare_nowait<2>();
 }  // namespace mctdhb

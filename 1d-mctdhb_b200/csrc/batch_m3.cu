@@ -6,4 +6,5 @@ template int hcp_batch_launch<3>(const BatchSlot*, const BatchTile*, const Batch
 template int gram_batch_launch<3>(const BatchSlot*, const BatchTile*, const int*, const int*,
                                   const int*, int, cudaStream_t);
 template int batch_prepare<3>();
+template int batch_prepare_nowait<3>();
 }  // namespace mctdhb

@@ -6,4 +6,5 @@ template int hcp_batch_launch<8>(const BatchSlot*, const BatchTile*, const Batch
 template int gram_batch_launch<8>(const BatchSlot*, const BatchTile*, const int*, const int*,
                                   const int*, int, cudaStream_t);
 template int batch_prepare<8>();
+template int batch_prepare_nowait<8>();
 }  // namespace mctdhb

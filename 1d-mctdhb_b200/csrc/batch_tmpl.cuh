@@ -312,10 +312,15 @@ int batch_y_attr() {
         MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bhcp_y_kernel<M, V>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)batch_y_smem<M, V>()));
-    if constexpr (PairHcShape<M, V>::PIPE)
-        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bhcp_y_kernel<M, V, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)batch_y_smem<M, V>()));
+    return 0;
+}
+
+// the instance without waits, loaded only where it is asked for
+template <int M>
+int batch_prepare_nowait() {
+    MCTDHB_CUDA_TRY(cudaFuncSetAttribute(bhcp_y_kernel<M, 3, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)batch_y_smem<M, 3>()));
     return 0;
 }
 

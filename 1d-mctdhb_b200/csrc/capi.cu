@@ -125,6 +125,7 @@ int mctdhb_space_set_nowait(mctdhb_space h, int on) {
         set_error("mctdhb_space_set_nowait: null space");
         return -1;
     }
+    if (on && hcp_prepare_nowait(h->sp.M)) return -1;
     h->sp.nowait = on != 0;
     return 0;
 }

@@ -191,6 +191,19 @@ int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, do
     return 0;
 }
 
+int hcp_prepare_nowait(int M) {
+    switch (M) {
+        case 2: return hcp_prepare_nowait_tmpl<2>();
+        case 3: return hcp_prepare_nowait_tmpl<3>();
+        case 4: return hcp_prepare_nowait_tmpl<4>();
+        case 5: return hcp_prepare_nowait_tmpl<5>();
+        case 6: return hcp_prepare_nowait_tmpl<6>();
+        case 7: return hcp_prepare_nowait_tmpl<7>();
+        case 8: return hcp_prepare_nowait_tmpl<8>();
+    }
+    return 0;
+}
+
 static bool hc_templated(int M) { return M >= 2 && M <= kMaxTemplOrb; }
 
 static int hcp_apply_v(const SpaceView& sp, const double2* C, double2* HC, const HcEpilogue& ep,

@@ -7,4 +7,5 @@ template int hc_launch_tmpl<7>(const SpaceView&, const double2*, double2*, const
 template int hcp_apply_tmpl<7>(const SpaceView&, const double2*, double2*, const HcEpilogue&,
                                  int, int, cudaStream_t);
 template int hcp_prepare_tmpl<7>();
+template int hcp_prepare_nowait_tmpl<7>();
 }

@@ -175,6 +175,8 @@ constexpr int kBatchPairVariants = 4;  // batched kernel: 0, 2, 3
 template <int M>
 int hcp_prepare_tmpl();
 template <int M>
+int hcp_prepare_nowait_tmpl();
+template <int M>
 int hcp_apply_tmpl(const SpaceView& sp, const double2* C, double2* HC, const HcEpilogue& ep,
                    int variant, int parts, cudaStream_t st);
 
@@ -197,6 +199,7 @@ int hc_prep(const SpaceView& sp, const double2* d_hob, const double2* d_hint, do
 bool hcp_eligible(int N, int M);
 size_t hcp_scratch_bytes(int N, int M);
 int hcp_prepare(int M);
+int hcp_prepare_nowait(int M);
 int hc_variant(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,
                const HcEpilogue& ep, cudaStream_t st);
 int hc_apply(const SpaceView& sp, const double2* C, double2* HC, const double2* tab,

@@ -636,15 +636,18 @@ __global__ void __launch_bounds__(kOrbThreads)
     }
 }
 
-int orb_step_prepare() {
+template <int B>
+static int orb_step_attributes() {
     static std::atomic<uint64_t> done{0};
     return set_attributes_once(done, []() -> int {
-        for (auto* kernel : {orb_step_kernel<0>, orb_step_kernel<kClusterMax>})
-            MCTDHB_CUDA_TRY(cudaFuncSetAttribute(kernel,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)orb_step_smem()));
+        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(orb_step_kernel<B>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)orb_step_smem()));
         return 0;
     });
+}
+int orb_step_prepare(bool batch) {
+    return batch ? orb_step_attributes<0>() : orb_step_attributes<kClusterMax>();
 }
 
 int orb_step_waves(int (&at)[kClusterSizes]) {

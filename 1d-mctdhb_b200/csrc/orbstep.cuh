@@ -22,8 +22,9 @@ constexpr int kOrbStep = 63;
 // (nullptr: none)
 int orb_step_launch(const BatchSlot* slots, const int* list, const int* nlist, int nslots,
                     int parts, int* mon, int blocks, cudaStream_t st);
-// launch attributes (call before any stream capture)
-int orb_step_prepare();
+// launch attributes (call before any stream capture) of the batch's instance or
+// the single system's (each is seven orbital counts of code to load)
+int orb_step_prepare(bool batch);
 // clusters that run at a time (cluster_blocks)
 int orb_step_waves(int (&at)[kClusterSizes]);
 inline bool orb_step_eligible(int M, int G) {

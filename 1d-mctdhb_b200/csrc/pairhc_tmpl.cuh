@@ -779,10 +779,15 @@ int hcp_set_attr() {
         MCTDHB_CUDA_TRY(cudaFuncSetAttribute(hcp_y_kernel<M, V>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)PairHcShape<M, V>::SMEM));
-    if constexpr (PairHcShape<M, V>::PIPE)
-        MCTDHB_CUDA_TRY(cudaFuncSetAttribute(hcp_y_kernel<M, V, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)PairHcShape<M, V>::SMEM));
+    return 0;
+}
+
+// the instance without waits, loaded only where it is asked for
+template <int M>
+int hcp_prepare_nowait_tmpl() {
+    MCTDHB_CUDA_TRY(cudaFuncSetAttribute(hcp_y_kernel<M, 3, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)PairHcShape<M, 3>::SMEM));
     return 0;
 }
 

@@ -137,7 +137,7 @@ int upload_slots(mctdhb_solver_s* s) {
     MCTDHB_CUDA_TRY(cudaMemcpy(s->d_flags + BF_STATE, &state, sizeof(int), cudaMemcpyHostToDevice));
     MCTDHB_CUDA_TRY(cudaMemcpy(s->d_flags + BF_ROBUST, &o.robust, sizeof(int),
                                cudaMemcpyHostToDevice));
-    return orb_step_prepare();
+    return orb_step_prepare(false);
 }
 
 // one launch of the cluster kernel on view v
