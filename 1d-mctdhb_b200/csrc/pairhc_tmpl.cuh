@@ -547,10 +547,11 @@ template <int M>
 __device__ __forceinline__ void pair_poison(uint32_t c, uint32_t step, uint32_t nchunk, int lane,
                                             const SpaceView& sp, double2* __restrict__ Y) {
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    constexpr int UNROLL = M == 7 ? M * (M + 1) / 2 : 1;  // hcp_y_kernel, IN_LOOP
     for (; c < nchunk; c += step) {
         const uint32_t m = c * 32 + lane;
         if (m >= sp.dim2) continue;
-#pragma unroll 1
+#pragma unroll UNROLL
         for (int p = 0; p < M * (M + 1) / 2; p++)
             Y[(size_t)p * sp.ldy + m] = make_double2(nan, nan);
     }
@@ -697,10 +698,11 @@ __global__ void __launch_bounds__(PairHcShape<M, V>::THREADS, 1)
             return;
         }
         // Where the loss is dealt with changes the code the compiler makes of
-        // the consumers' loop: at 7 orbitals in the loop (N=25 M=7: 166 us of
-        // H.C, 170 us after it), else after it (N=30 M=8: 2,956 us, 3,048 us in
-        // the loop; 2,932 us with no NaN and no vote at all; 3,030 us in a lambda
-        // as above).
+        // the consumers' loop: at 7 orbitals in the loop and unrolled (N=25 M=7:
+        // 165.6 us of H.C, 169 us not unrolled, 170 us after the loop; 165.2 us
+        // with no NaN and no vote at all), else after it (N=30 M=8: 2,952 us,
+        // 3,018 us unrolled, 3,048 us in the loop, 3,030 us in a lambda as
+        // above; 2,936 us with neither).
         constexpr bool IN_LOOP = M == 7;
         int i = 0;
         bool ok = true;
