@@ -334,8 +334,9 @@ int rebuild_lists(mctdhb_batch_s* b) {
     b->present_mask = mask;
     b->small_mask = small;
     if (b->orb_waves[0] == 0 && (orb_step_prepare(true) || orb_step_waves(b->orb_waves))) return -1;
-    b->orb_blocks = cluster_blocks(b->orb_waves, list(0)[0]);
+    b->orb_blocks = cluster_blocks(b->orb_waves, list(0)[0], 0, b->orb_blocks);
     // the small slots of all orbital counts run beside one another
+    const int small_now = b->small_blocks;
     b->small_blocks = kClusterMax;
     for (int M = kBatchMinOrb; M <= kBatchMaxOrb; M++) {
         if (!(small >> M & 1)) continue;
@@ -343,7 +344,7 @@ int rebuild_lists(mctdhb_batch_s* b) {
             return -1;
         b->small_blocks = std::min(
             b->small_blocks,
-            cluster_blocks(b->small_waves[M], list(0)[0] - list(1)[0], small_rows));
+            cluster_blocks(b->small_waves[M], list(0)[0] - list(1)[0], small_rows, small_now));
     }
     b->lists_dirty = false;
     return 0;

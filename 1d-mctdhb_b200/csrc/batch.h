@@ -42,12 +42,20 @@ constexpr int kClusterSizes = 4;
 // rows a block (N=190 M=3, 18,336 rows, 256 jobs: 4,753 us on one block each,
 // 3,904 us on four), so a longer one takes more.
 // at[i]: clusters of 1 << i blocks that run at a time; rows: of a vector, the
-// longest (0: none)
+// longest (0: none); now: the size so far (0: none), which grows only where a
+// quarter more slots would still fit, since a change costs a capture of the step
+// graph and the slots of a served stream come and go
 constexpr uint32_t kClusterRows = 8192;
-inline int cluster_blocks(const int (&at)[kClusterSizes], int n, uint32_t rows = 0) {
-    int i = kClusterSizes - 1;
-    while (i > 0 && at[i] < n && rows <= kClusterRows << (i - 1)) i--;
-    return 1 << i;
+inline int cluster_blocks(const int (&at)[kClusterSizes], int n, uint32_t rows, int now) {
+    auto size = [&](int slots) {
+        int i = kClusterSizes - 1;
+        while (i > 0 && at[i] < slots && rows <= kClusterRows << (i - 1)) i--;
+        return 1 << i;
+    };
+    const int want = size(n);
+    if (now == 0 || want <= now) return want;
+    const int slack = size(n + n / 4 + 1);
+    return slack > now ? slack : now;
 }
 struct ClusterLaunch {
     cudaLaunchConfig_t cfg = {};
