@@ -410,7 +410,10 @@ __device__ inline int sync_rho1_warp(int n, double2* rho1, double2* rinv, double
 // of d and e, lane k rotates row k (k + 32) of z.
 // c and s are quotients: as products by a rounded 1 / r they moved c^2 + s^2
 // off 1 and the error of a Lanczos step against 80-bit arithmetic was 4.9e-16
-// instead of 4.3e-16 (mean of 120 steps of 5,000 to 10,600 configurations).
+// instead of 4.3e-16 (mean of 120 steps of 5,000 to 10,600 configurations).  Even
+// lanes divide f, odd ones g: one division's time for the two, same doubles (a
+// step of 12 bosons in 5 orbitals with 16 vectors 478 -> 462 us, of 8 in 10 with
+// 30 vectors 2,016 -> 1,961 us; both divisions on every lane before).
 __device__ inline int tridiag_ql_warp(int n, double* d, double* e, double* z) {
     const int lane = threadIdx.x & 31;
     for (int k = lane; k < n; k += 32)
@@ -441,8 +444,9 @@ __device__ inline int tridiag_ql_warp(int n, double* d, double* e, double* z) {
                     deflated = true;
                     break;
                 }
-                s = f / r;
-                c = g / r;
+                const double q = (lane & 1 ? g : f) / r;
+                s = __shfl_sync(0xffffffffu, q, 0);
+                c = __shfl_sync(0xffffffffu, q, 1);
                 g = d[i + 1] - p;
                 r = (d[i] - g) * s + 2.0 * c * b;
                 p = s * r;
