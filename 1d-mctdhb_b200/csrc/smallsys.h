@@ -15,10 +15,18 @@ namespace mctdhb {
 //   one product, up to 0.25 M complex multiply-adds of the contraction (rows of
 //     the (N-2)-space times pairs^2): 0.02 M (N=10 M=4)  8.4 us against 12.0;
 //     0.23 M (N=24 M=4) level; 0.45 M (N=30 M=4) 16.7 against 13
-//   a step of one system (5 vectors, with densities), up to 2,048 rows, one a
-//     thread: 1,501 rows (N=1500 M=2) 82 us against 86; 1,716 (N=6 M=8) 145
-//     against 158; 1,891 (N=60 M=3) 92 against 95; 2,380 (N=13 M=5) 137 against
-//     127; 4,845 (N=16 M=5) 185 against 121; 18,336 (N=190 M=3) 230 against 111
+//   a step of one system, up to 2,048 rows, one a thread, and up to 4,096 where
+//     a product has at most 0.21 M.  Captured steps of 5 vectors with densities:
+//     1,501 rows (N=1500 M=2) 82 us against 86; 1,716 (N=6 M=8) 145 against
+//     158; 2,145 (N=64 M=3) 101 against 103; 2,556 (N=70 M=3) 111 against 99;
+//     2,600 (N=23 M=4, 0.20 M) 111 against 119; 4,001 (N=4000 M=2) 95 against
+//     97.  Past the line: 2,380 (N=13 M=5, 0.31 M) 127 against 123; 2,925 (N=24
+//     M=4, 0.23 M) 123 against 119; 4,656 (N=95 M=3) 130 against 109; 5,001
+//     (N=5000 M=2) 109 against 99; 18,336 (N=190 M=3) 230 against 111.  A step
+//     by the reference's C entry, where each launch costs the host time, in the
+//     same order of sizes from 2,145 rows: 212 / 226 / 232 / 216 us against 238
+//     / 241 / 257 / 233, past the line 248 / 241 / 258 / 236 against 259 / 257 /
+//     261 / 241
 //   a slot of the batch, where the general path's iteration has twice the
 //     launches, up to 0.7 M: 0.69 M (N=16 M=5) 2 / 32 / 128 / 256 jobs 281 /
 //     387 / 1,174 / 2,283 us against 392 / 504 / 1,130 / 2,022; 0.43 M (N=6 M=8)
@@ -26,11 +34,13 @@ namespace mctdhb {
 //     follows (N, M) alone, for a job's bits
 constexpr double kSmallHcMacs = 2.5e5, kSmallSlotMacs = 7e5;
 constexpr uint32_t kSmallStepRows = 2048;
+constexpr double kSmallStepMacs = 2.1e5;  // from there to twice the rows
 bool small_eligible(int N, int M, uint32_t D2, double macs);
 // whether a step of one system with m Lanczos vectors runs here
 inline bool sil_small(const SpaceView& sp, int m) {
-    return m <= kBatchMaxLz && sp.pair_y != nullptr && sp.dim <= kSmallStepRows &&
-           small_eligible(sp.N, sp.M, sp.dim2, kSmallSlotMacs);
+    if (m > kBatchMaxLz || sp.pair_y == nullptr || sp.dim > 2 * kSmallStepRows) return false;
+    return small_eligible(sp.N, sp.M, sp.dim2,
+                          sp.dim <= kSmallStepRows ? kSmallSlotMacs : kSmallStepMacs);
 }
 
 // what one system's step works on; every pointer is device memory

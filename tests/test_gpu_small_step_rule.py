@@ -1,6 +1,6 @@
 """Which step of one system runs on one cluster of blocks (csrc/smallsys.h): up
-to 2,048 configurations, one a thread; more take the general path, which is
-faster from there.  The routes differ in their launches, 2 an iteration on the
+to 2,048 configurations, one a thread, and up to twice that where the product
+is small; more take the general path, which is faster from there.  The routes differ in their launches, 2 an iteration on the
 cluster (product, orthogonalisation) and 4 beside it.  Both against the oracle
 at the edge; 1e-10 of the largest element, as for Lanczos steps elsewhere."""
 import numpy as np
@@ -11,9 +11,12 @@ from helpers import phys_hint, rand_coef, rand_hob, rel_err
 pytestmark = pytest.mark.gpu
 
 
-# 2,048 and 2,049; 2,016 and 2,080; 2,002 and 2,380; 1,716 and 3,003 rows
-@pytest.mark.parametrize("N,M,cluster", [(2047, 2, True), (2048, 2, False), (62, 3, True),
-                                         (63, 3, False), (9, 6, True), (13, 5, False),
+# 2,048, 2,049, 4,096 and 4,097; 2,016, 2,080, 4,095 and 4,186; 2,600 (0.20 M
+# multiply-adds a product) and 2,925 (0.23 M); 2,002 and 2,380; 1,716 and 3,003 rows
+@pytest.mark.parametrize("N,M,cluster", [(2047, 2, True), (2048, 2, True), (4095, 2, True),
+                                         (4096, 2, False), (62, 3, True), (63, 3, True),
+                                         (89, 3, True), (90, 3, False), (23, 4, True),
+                                         (24, 4, False), (9, 6, True), (13, 5, False),
                                          (6, 8, True), (8, 7, False)])
 @pytest.mark.parametrize("imag", [False, True])
 def test_step_at_the_edge(gpu, oracle, N, M, cluster, imag):
